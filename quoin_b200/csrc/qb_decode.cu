@@ -1,9 +1,8 @@
 // Block decoder (reference src/decoder.rs:145-190 and the per-codec decode
 // functions).  Two kernels:
-//  * k_walk_frames — one thread per frame: validates the frame's payload
+//  * k_walk_frames — one warp per frame: validates the frame's payload
 //    structure in the reference's check order and records the byte offsets of
-//    its FastLanes sub-blocks (the sub-block sizes are data-dependent, so this
-//    is a short dependent walk; every frame walks concurrently);
+//    its FastLanes sub-blocks and ALP-RD exceptions (qb_walk.cuh);
 //  * k_decode_frames — one CTA per frame, one warp per 1024-value sub-block:
 //    coalesced unpack of the lane-transposed words, delta / RLE prefix sums
 //    across sub-blocks, ALP / FLOAT_MULT reconstruction, exception patching,
@@ -13,6 +12,7 @@
 #include "qb_common.cuh"
 #include "qb_kernels.h"
 #include "qb_layout.h"
+#include "qb_walk.cuh"
 
 namespace qb {
 
@@ -31,74 +31,18 @@ struct FrameAux {
   uint64_t a, b, c, d;  // mode-specific scalars
   uint64_t e0, e1, e2;  // entropy-coded parts: payload positions
   uint32_t t0, t1;      // and their tags
-  uint32_t defer;       // 1: an ALP-RD exception list left to the frame kernel's walk
+  uint32_t sorted;      // 1: an ALP-RD exception list's positions strictly increase
   uint32_t pad_;
   uint64_t dict8[8];    // ALP-RD dictionary
   uint32_t offs[2][kMaxSubs + 1];  // chain 0 / chain 1 sub-block header offsets (payload-relative)
 };
-
-// ---------------------------------------------------------------------------
-// FoR sub-block chain (reference codecs/for_bitpack.rs:108-157), walked over
-// p[pos .. bound): varint(n) then sub-blocks [width u8][min u64][128*width B].
-// ---------------------------------------------------------------------------
-__device__ uint32_t for_walk(const uint8_t* p, uint64_t bound, uint64_t pos, uint64_t n_values, uint32_t* offs) {
-  uint64_t n64;
-  uint32_t e = rd_varint(p, bound, &pos, &n64);
-  if (e) return e;
-  if (n64 != n_values) return E_CORRUPT;
-  uint32_t nsub = (uint32_t)((n_values + kSub - 1) / kSub);
-  for (uint32_t k = 0; k < nsub; k++) {
-    if (pos >= bound) return E_TRUNCATED;
-    uint32_t w = p[pos];
-    if (w > 64) return E_CORRUPT;
-    if (bound - pos - 1 < 8) return E_TRUNCATED;
-    uint64_t need = 128ull * w;
-    if (bound - pos - 9 < need) return E_TRUNCATED;
-    offs[k] = (uint32_t)pos;
-    pos += 9 + need;
-  }
-  offs[nsub] = (uint32_t)pos;
-  return E_OK;
-}
-
-// ALP sub-block chain (reference codecs/alp.rs:168-248).
-__device__ uint32_t alp_walk(const uint8_t* p, uint64_t plen, uint64_t n, uint32_t* offs) {
-  uint64_t pos = 0, n64;
-  uint32_t e = rd_varint(p, plen, &pos, &n64);
-  if (e) return e;
-  if (n64 != n) return E_CORRUPT;
-  uint32_t nsub = (uint32_t)((n + kSub - 1) / kSub);
-  for (uint32_t k = 0; k < nsub; k++) {
-    uint64_t count = qmin(kSub, n - (uint64_t)k * kSub);
-    if (pos >= plen) return E_TRUNCATED;
-    uint32_t ee = p[pos];
-    if (pos + 1 >= plen) return E_TRUNCATED;
-    uint32_t ff = p[pos + 1];
-    if (ee > 18 || ff > ee) return E_CORRUPT;
-    if (plen < pos + 4) return E_TRUNCATED;
-    uint32_t exc = ld_u16(p + pos + 2);
-    if (plen < pos + 12 || pos + 12 >= plen) return E_TRUNCATED;
-    uint32_t w = p[pos + 12];
-    if (w > 32) return E_CORRUPT;
-    offs[k] = (uint32_t)pos;
-    uint64_t q = pos + 13;
-    if (plen - q < 128ull * w) return E_TRUNCATED;
-    q += 128ull * w;
-    for (uint32_t x = 0; x < exc; x++) {
-      if (plen < q + 2 || plen < q + 10) return E_TRUNCATED;
-      if (ld_u16(p + q) >= count) return E_CORRUPT;
-      q += 10;
-    }
-    pos = q;
-  }
-  return E_OK;
-}
 
 // ALP-RD payload after the exception list (alp_rd.rs:208-285): codes tag,
 // varint(codes_len), codes, rights tag, rights.  Bit-packed parts get their
 // FoR sub-block offsets; an entropy-coded part (tag 1) leaves the rest to the
 // frame kernel's entropy path.
 __device__ uint32_t alprd_walk_tail(const uint8_t* p, uint64_t plen, uint64_t n, uint64_t pos, FrameAux& A) {
+  const bool l0 = (threadIdx.x & 31) == 0;
   if (pos >= plen) return E_TRUNCATED;
   uint32_t ctag = p[pos++];
   uint64_t clen;
@@ -109,39 +53,51 @@ __device__ uint32_t alprd_walk_tail(const uint8_t* p, uint64_t plen, uint64_t n,
   pos += clen;
   if (pos >= plen) return E_TRUNCATED;
   uint32_t rtag = p[pos++];
-  A.e0 = cpos;
-  A.e1 = clen;
-  A.e2 = pos;
-  A.t0 = ctag;
-  A.t1 = rtag;
+  if (l0) {
+    A.e0 = cpos;
+    A.e1 = clen;
+    A.e2 = pos;
+    A.t0 = ctag;
+    A.t1 = rtag;
+  }
   if (ctag == 1) {  // codes entropy-coded: the frame kernel decodes the rest in order
-    A.ent = 1;
+    if (l0) A.ent = 1;
     return E_OK;
   }
   if (ctag != 0) return E_CORRUPT;
-  e = for_walk(p, cpos + clen, cpos, n, A.offs[0]);
+  e = warp_for_walk(p, cpos + clen, cpos, n, A.offs[0]);
   if (e) return e;
   if (rtag == 1) {  // rights entropy-coded (bit-packed rights bytes)
-    A.ent = 1;
+    if (l0) A.ent = 1;
     return E_OK;
   }
   if (rtag != 0) return E_CORRUPT;
-  return for_walk(p, plen, pos, n, A.offs[1]);
+  return warp_for_walk(p, plen, pos, n, A.offs[1]);
 }
 
-// One thread per frame.
-__global__ void k_walk_frames(const uint8_t* __restrict__ stream, const FrameDesc* __restrict__ frames, int nf,
-                              int dtype, FrameAux* __restrict__ aux, unsigned long long* __restrict__ err,
-                              BatchView bv) {
-  int f = blockIdx.x * blockDim.x + threadIdx.x;
+// One warp per frame; every lane takes the same path (the payload's scalars
+// are broadcast loads) and lane 0 writes the record.  An ALP-RD frame's
+// exception record offsets (u32, payload-relative) go to its scratch range.
+constexpr int kWalkWarps = 4;
+__global__ void __launch_bounds__(kWalkWarps * 32) k_walk_frames(const uint8_t* __restrict__ stream,
+                                                                 const FrameDesc* __restrict__ frames, int nf,
+                                                                 int dtype, FrameAux* __restrict__ aux,
+                                                                 uint64_t* __restrict__ scratch,
+                                                                 unsigned long long* __restrict__ err, BatchView bv) {
+  int f = blockIdx.x * kWalkWarps + (threadIdx.x >> 5);
   if (f >= nf) return;
+  const int l = threadIdx.x & 31;
   FrameDesc d = frames[f];
-  if (bv.cols) dtype = bv.cols[bv.frame_col[f]].dtype;
+  if (bv.cols) {
+    dtype = bv.cols[bv.frame_col[f]].dtype;
+    scratch = bv.cols[bv.frame_col[f]].scratch;
+  }
   const uint8_t* p = stream + d.payload_off;
   uint64_t plen = d.plen, n = d.n;
   FrameAux& A = aux[f];
-  A.ent = 0;
-  A.defer = 0;
+  uint32_t ent = 0;
+  if (l == 0) A.ent = 0;  // before alprd_walk_tail sets it
+  uint64_t ra = 0, rb = 0, rc = 0, rd = 0;  // A.a .. A.d
   uint32_t e = E_OK;
   switch (d.mode) {
     case M_RAW:
@@ -156,11 +112,11 @@ __global__ void k_walk_frames(const uint8_t* __restrict__ stream, const FrameDes
     case M_XORZ:
       break;  // validated by the parallel decoder
     case M_FOR_BITPACK:
-      e = for_walk(p, plen, 0, n, A.offs[0]);
+      e = warp_for_walk(p, plen, 0, n, A.offs[0]);
       break;
     case M_DELTA_BITPACK:  // delta_bitpack.rs:48-64
       if (plen < 8) { e = E_TRUNCATED; break; }
-      e = for_walk(p, plen, 8, n, A.offs[0]);
+      e = warp_for_walk(p, plen, 8, n, A.offs[0]);
       break;
     case M_BYTE_TRANSPOSE:  // transpose.rs:10-32: the whole payload is entropy-coded
     case M_ORDERED_DELTA:   // linear.rs: entropy-coded residual bytes (decoder.rs:162-171)
@@ -170,24 +126,23 @@ __global__ void k_walk_frames(const uint8_t* __restrict__ stream, const FrameDes
     case M_PRED_RC:
     case M_PRED2:
     case M_LZ:              // lz.rs: entropy-coded LZ tokens (decoder.rs:172-175)
-      A.ent = 1;
+      ent = 1;
       break;
     case M_FLOAT_MULT: {  // float_mult.rs:100-133
       if (plen < 1 || plen < 2) { e = E_TRUNCATED; break; }
       uint32_t tag = p[0], si = p[1];
       if (si >= 7) { e = E_CORRUPT; break; }
+      ra = si;
       if (tag == 1) {  // FM_ENTROPY: rANS over LEB128 zigzag deltas of k
-        A.a = si;
-        A.ent = 1;
+        ent = 1;
         break;
       }
       if (tag != 0) { e = E_CORRUPT; break; }
-      A.a = si;
-      e = for_walk(p, plen, 2, n, A.offs[0]);
+      e = warp_for_walk(p, plen, 2, n, A.offs[0]);
       break;
     }
     case M_ALP:
-      e = alp_walk(p, plen, n, A.offs[0]);
+      e = warp_alp_walk(p, plen, n, A.offs[0]);
       break;
     case M_ALP_RD: {  // alp_rd.rs:208-285
       uint64_t pos = 0;
@@ -197,24 +152,35 @@ __global__ void k_walk_frames(const uint8_t* __restrict__ stream, const FrameDes
       if (pos >= plen) { e = E_TRUNCATED; break; }
       uint32_t dsz = p[pos++];
       if (dsz > 8) { e = E_CORRUPT; break; }
-      for (uint32_t j = 0; j < dsz; j++) {
-        if (plen < pos + 8) { e = E_TRUNCATED; break; }
-        A.dict8[j] = ld_u64(p + pos);
-        pos += 8;
-      }
-      if (e) break;
+      if (plen < pos + 8ull * dsz) { e = E_TRUNCATED; break; }
+      if ((uint32_t)l < dsz) A.dict8[l] = ld_u64(p + pos + 8 * l);
+      pos += 8ull * dsz;
       uint64_t nexc;
       e = rd_varint(p, plen, &pos, &nexc);
       if (e) break;
       if (nexc > n) { e = E_CORRUPT; break; }
-      A.a = lbw;
-      A.b = dsz;
-      A.c = pos;
-      A.d = nexc;
-      if (nexc) {  // the list and the rest of the walk: alprd_list_walk + alprd_walk_tail in the frame kernel
-        A.defer = 1;
-        break;
+      ra = lbw;
+      rb = dsz;
+      rc = pos;
+      rd = nexc;
+      bool inc = true;
+      if (nexc) {
+        if (!scratch) { e = E_UNSUPPORTED; break; }
+        uint32_t* offs = reinterpret_cast<uint32_t*>(scratch + d.value_off);  // nexc <= n of them
+        uint64_t prev = ~0ull;  // the position before the group's first (~0: none)
+        e = warp_exc_walk(p, plen, &pos, nexc, [&](bool act, uint64_t x, uint64_t q, uint64_t v) {
+          if (act) offs[x] = (uint32_t)q;
+          uint64_t before = __shfl_up_sync(0xffffffffu, v, 1);
+          if (l == 0) before = prev;
+          inc = inc && !(act && before != ~0ull && v <= before);
+          uint32_t na = __popc(__ballot_sync(0xffffffffu, act));
+          if (na) prev = __shfl_sync(0xffffffffu, v, na - 1);
+          return v < n;
+        });
+        if (e) break;
       }
+      inc = __all_sync(0xffffffffu, inc);
+      if (l == 0) A.sorted = inc;
       e = alprd_walk_tail(p, plen, n, pos, A);
       break;
     }
@@ -228,19 +194,18 @@ __global__ void k_walk_frames(const uint8_t* __restrict__ stream, const FrameDes
       e = rd_varint(p, plen, &pos, &vlen);
       if (e) break;
       if (vlen > plen - pos) { e = E_TRUNCATED; break; }
-      uint64_t vpos = pos;
+      ra = card;
+      rb = vtag;
+      rc = pos;
+      rd = vlen;
       if (vtag == 0) {
         if (vlen != card * 8) { e = E_CORRUPT; break; }
       } else if (vtag == 1) {
         if (vlen < 8) { e = E_TRUNCATED; break; }
-        e = for_walk(p, vpos + vlen, vpos + 8, card, A.offs[1]);
+        e = warp_for_walk(p, pos + vlen, pos + 8, card, A.offs[1]);
         if (e) break;
       } else if (vtag == 2) {  // TRANSPOSE values: the frame kernel decodes the rest in order
-        A.a = card;
-        A.b = vtag;
-        A.c = vpos;
-        A.d = vlen;
-        A.ent = 1;
+        ent = 1;
         break;
       } else {
         e = E_CORRUPT;
@@ -249,17 +214,13 @@ __global__ void k_walk_frames(const uint8_t* __restrict__ stream, const FrameDes
       pos += vlen;
       if (pos >= plen) { e = E_TRUNCATED; break; }
       uint32_t ctag = p[pos++];
-      A.a = card;
-      A.b = vtag;
-      A.c = vpos;
-      A.d = vlen;
       if (ctag == 1) {  // CODES_ENTROPY byte planes
-        A.e0 = pos;
-        A.ent = 1;
+        if (l == 0) A.e0 = pos;
+        ent = 1;
         break;
       }
       if (ctag != 0) { e = E_CORRUPT; break; }
-      e = for_walk(p, plen, pos, n, A.offs[0]);
+      e = warp_for_walk(p, plen, pos, n, A.offs[0]);
       break;
     }
     case M_RLE: {  // rle.rs:44-75
@@ -270,16 +231,22 @@ __global__ void k_walk_frames(const uint8_t* __restrict__ stream, const FrameDes
       if (plen - pos < nr * 8) { e = E_TRUNCATED; break; }
       uint64_t vpos = pos;
       pos += nr * 8;
-      e = for_walk(p, plen, pos, nr, A.offs[0]);
-      A.a = nr;
-      A.b = vpos;
+      e = warp_for_walk(p, plen, pos, nr, A.offs[0]);
+      ra = nr;
+      rb = vpos;
       break;
     }
     default:
       e = E_UNSUPPORTED;
       break;
   }
+  if (l) return;
   A.err = e;
+  if (ent) A.ent = 1;
+  A.a = ra;
+  A.b = rb;
+  A.c = rc;
+  A.d = rd;
   if (e) atomicMin(err, ((unsigned long long)f << 8) | e);
 }
 
@@ -457,6 +424,19 @@ __device__ uint64_t warp_select(const DecodeOut& O, uint64_t c) {
     }
   }
   return O.n;
+}
+
+// Position of the c-th valid value (c < nvalid) by one thread: the table's
+// stretch of bitmap words, halved by their ranks.
+__device__ inline uint64_t lane_position(const DecodeOut& O, uint64_t c) {
+  if (!O.bm32) return c;
+  uint64_t lo = O.sel[c >> 9] >> 5, hi = (O.n + 31) >> 5;  // the last word with rank <= c lies in [lo, hi)
+  if (((c >> 9) + 1) << 9 < O.nvalid) hi = (O.sel[(c >> 9) + 1] >> 5) + 1;
+  while (hi - lo > 1) {
+    uint64_t mid = (lo + hi) >> 1;
+    if (O.wrank[mid] <= c) lo = mid; else hi = mid;
+  }
+  return (lo << 5) + select_in_word(O.bm32[lo], (uint32_t)(c - O.wrank[lo]));
 }
 
 __device__ __forceinline__ void run_positions(const DecodeOut& O, uint64_t c0, uint64_t c1, uint64_t* p0,
@@ -777,246 +757,25 @@ __device__ uint32_t dec_xorz(DecSmem& S, const uint8_t* p, uint64_t plen, uint64
   return e;
 }
 
-// ---------------------------------------------------------------------------
-// ALP-RD exception lists (alp_rd.rs:208-285): nexc records of (varint
-// position, u64 left part).  Records have variable length, so the start of
-// each depends on the previous one's varint.  The list is staged through
-// shared memory (at most 16 KB, and at most 18 bytes per remaining record, a
-// round) with a bitmap of its varint terminator bytes (high bit clear); the
-// CTA computes, for every staged offset, where a record starting there would
-// end (the first terminator within 10 bytes, then 8 bytes), and one thread
-// follows the chain through that table: one shared load per record.  The
-// records of a round are then decoded, checked and applied by the whole CTA.
-// ---------------------------------------------------------------------------
-constexpr uint32_t kExcStage = 16384;  // staged list bytes per round
-constexpr uint32_t kExcRecs = 2048;    // records per round (a stage holds at most 16384 / 9 + 1)
-constexpr uint32_t kExcWords = (kExcStage + 32) / 32 + 7;  // 520: two words past the last staged byte
-constexpr uint16_t kNxBadVarint = 0xFFFF, kNxShort = 0xFFFE;
-
-struct ExcStage {
-  uint8_t* bytes;   // bytes[j] = the byte at the 16-byte aligned address below the round's position + j
-  uint16_t* nx;     // nx[j]: stage offset after a record starting at j, or kNxBadVarint / kNxShort
-  uint32_t* epos;   // record positions (over nx, once the chain has been followed)
-  uint64_t* left;   // record left parts (likewise)
-  uint32_t* term;   // terminator bitmap over the stage (bit j: byte j staged, high bit clear)
-  uint16_t* start;  // record starts (stage offsets)
-};
-
-// Carves the stage out of the per-warp staging area (64 KB): 16 KB + 32 of
-// bytes, the next-record table (its space reused for positions and left
-// parts), 520 bitmap words and the starts (55 KB).
-__device__ inline ExcStage exc_stage(DecSmem& S) {
-  uint8_t* base = reinterpret_cast<uint8_t*>((reinterpret_cast<uintptr_t>(&S.u.wbuf[0][0]) + 15) & ~(uintptr_t)15);
-  ExcStage X;
-  X.bytes = base;
-  X.nx = reinterpret_cast<uint16_t*>(base + kExcStage + 32);
-  X.left = reinterpret_cast<uint64_t*>(X.nx);
-  X.epos = reinterpret_cast<uint32_t*>(X.left + kExcRecs);
-  X.term = reinterpret_cast<uint32_t*>(X.nx + kExcStage + 32);
-  X.start = reinterpret_cast<uint16_t*>(X.term + kExcWords);
-  return X;
-}
-static_assert(8 * kExcRecs + 4 * kExcRecs <= 2 * (kExcStage + 32), "positions and left parts fit the table");
-static_assert(3 * (kExcStage + 32) + 4 * kExcWords + 2 * kExcRecs + 15 <= sizeof(uint64_t) * kDecWarps * kSub,
-              "exception stage fits the per-warp staging area");
-
-// The 4 bytes at byte offset o of a 4-byte aligned shared buffer (o + 8 within it).
-__device__ inline uint32_t lds_u32(const uint8_t* b, uint32_t o) {
-  const uint32_t* w = reinterpret_cast<const uint32_t*>(b);
-  return __funnelshift_r(w[o >> 2], w[(o >> 2) + 1], (o & 3) * 8);
-}
-
-// Bits of the 10 bytes from stage offset o in the terminator bitmap.
-__device__ inline uint32_t term10(const uint32_t* term, uint32_t o) {
-  uint64_t win = ((uint64_t)term[o >> 5] | ((uint64_t)term[(o >> 5) + 1] << 32)) >> (o & 31);
-  return (uint32_t)win & 0x3FFu;
-}
-
-// Payload bytes [pos, send) into the stage by the whole CTA (16-byte loads for
-// the aligned middle, bytes at the edges; nothing outside the range is read),
-// the terminator bitmap and the next-record table (bounded by plen as the
-// record reads are).  Returns the stage offset of byte pos.
-__device__ uint32_t stage_list(const ExcStage& X, const uint8_t* p, uint64_t pos, uint64_t send, uint64_t plen) {
-  uintptr_t g0 = reinterpret_cast<uintptr_t>(p + pos), g1 = reinterpret_cast<uintptr_t>(p + send);
-  uintptr_t a0 = g0 & ~(uintptr_t)15, c0 = (g0 + 15) & ~(uintptr_t)15, a1 = g1 & ~(uintptr_t)15;
-  uint32_t head = (uint32_t)(g0 - a0), end = head + (uint32_t)(send - pos);
-  for (uintptr_t c = c0 + 16u * threadIdx.x; c < a1; c += 16u * blockDim.x)
-    *reinterpret_cast<uint4*>(X.bytes + (c - a0)) = __ldg(reinterpret_cast<const uint4*>(c));
-  uintptr_t e0 = c0 < g1 ? c0 : g1, t0 = a1 > c0 ? a1 : c0;
-  for (uintptr_t c = g0 + threadIdx.x; c < e0; c += blockDim.x) X.bytes[c - a0] = *reinterpret_cast<const uint8_t*>(c);
-  for (uintptr_t c = t0 + threadIdx.x; c < g1; c += blockDim.x) X.bytes[c - a0] = *reinterpret_cast<const uint8_t*>(c);
-  __syncthreads();
-  for (uint32_t w = threadIdx.x; w < kExcWords; w += blockDim.x) {
-    uint32_t bits = 0;
-    uint32_t j0 = 32 * w;
-    if (j0 < end && j0 + 32 > head) {
-      const uint32_t* q = reinterpret_cast<const uint32_t*>(X.bytes + j0);
-#pragma unroll
-      for (int i = 0; i < 8; i++) {
-        uint32_t m = ~q[i] & 0x80808080u;
-        bits |= (((m >> 7) & 1u) | ((m >> 14) & 2u) | ((m >> 21) & 4u) | ((m >> 28) & 8u)) << (4 * i);
-      }
-      if (head > j0) bits &= ~0u << (head - j0);
-      if (end < j0 + 32) bits &= (1u << (end - j0)) - 1u;
-    }
-    X.term[w] = bits;
+// ALP-RD exceptions (alp_rd.rs:281-283): put(p, (left << rbw) | rights[p]) for
+// each record, in list order.  The walk left the records' offsets in `offs`
+// and validated them.  A list whose positions strictly increase (every list
+// the encoder writes) is applied by the whole CTA; otherwise thread 0 applies
+// it in order, so a repeated position keeps its last record.
+template <class P>
+__device__ void alprd_exceptions(const uint8_t* p, uint64_t plen, const uint32_t* offs, uint64_t nexc, bool sorted,
+                                 const uint8_t* rsrc, const uint32_t* roffs, uint32_t rbw, P put) {
+  auto apply = [&](uint64_t r) {
+    uint64_t q = offs[r], pp = 0;
+    rd_varint(p, plen, &q, &pp);
+    uint64_t left = ld_u64(p + q);
+    put(pp, (left << rbw) | for_value_at(rsrc, roffs[pp / kSub], (uint32_t)(pp % kSub)));
+  };
+  if (sorted) {
+    for (uint64_t r = threadIdx.x; r < nexc; r += kDecThreads) apply(r);
+  } else if (threadIdx.x == 0) {
+    for (uint64_t r = 0; r < nexc; r++) apply(r);
   }
-  __syncthreads();
-  for (uint32_t j = head + threadIdx.x; j < end; j += blockDim.x) {
-    uint32_t m10 = term10(X.term, j);
-    uint16_t v = kNxBadVarint;
-    if (m10) {
-      uint32_t vl = (uint32_t)__ffs(m10);
-      v = plen - (pos + (j - head) + vl) < 8 ? kNxShort : (uint16_t)(j + vl + 8);
-    }
-    X.nx[j] = v;
-  }
-  __syncthreads();
-  return head;
-}
-
-__device__ __forceinline__ uint32_t lds_u16(const uint16_t* p) {
-  uint16_t v;
-  asm volatile("ld.shared.u16 %0, [%1];" : "=h"(v) : "r"((uint32_t)__cvta_generic_to_shared(p)));
-  return v;
-}
-__device__ __forceinline__ void sts_u16(uint16_t* p, uint32_t v) {
-  asm volatile("st.shared.u16 [%0], %1;" ::"r"((uint32_t)__cvta_generic_to_shared(p)), "h"((uint16_t)v));
-}
-
-// Thread 0: the chain of records from stage offset `head` (list position
-// gpos) while records remain (at most kExcRecs) and each is wholly staged (its
-// start + 18 within the stage, or the stage reaching plen).  Fills X.start;
-// stops at the first record whose varint runs past 10 bytes (E_CORRUPT, as
-// rd_varint) or past plen, or whose 8-byte left part does not fit
-// (E_TRUNCATED).  Returns the records found; *err and *next describe the stop.
-__device__ __forceinline__ uint32_t exc_chain(const ExcStage& X, uint32_t head, uint32_t end, uint64_t gpos,
-                                              uint64_t plen, bool staged_to_plen, uint64_t want, uint32_t* err,
-                                              uint64_t* next) {
-  uint32_t k = 0, e = E_OK, o = head;
-  uint32_t lim = (uint32_t)qmin(want, (uint64_t)kExcRecs);
-  uint32_t last = staged_to_plen ? end : (end >= 18 ? end - 18 : 0);  // records may start at o <= last
-  while (k < lim && o <= last) {
-    if (!staged_to_plen || o < end) {
-      uint32_t nxt = lds_u16(X.nx + o);
-      if (nxt < kNxShort) {
-        sts_u16(X.start + k, o);
-        k++;
-        o = nxt;
-        continue;
-      }
-      e = nxt == kNxShort ? E_TRUNCATED : (plen - (gpos + (o - head)) >= 10 ? E_CORRUPT : E_TRUNCATED);
-    } else {
-      e = E_TRUNCATED;  // the list runs past plen
-    }
-    break;
-  }
-  *err = e;
-  *next = gpos + (o - head);
-  return k;
-}
-
-// Record r of the stage: its position and left part (rd_varint's value).
-__device__ inline void exc_decode(const ExcStage& X, uint32_t r, uint64_t* pp, uint64_t* lv) {
-  uint32_t o = X.start[r];
-  uint32_t vl = (uint32_t)__ffs(term10(X.term, o));
-  uint64_t v = 0;
-  for (uint32_t i = 0; i < vl; i++) v |= (uint64_t)(X.bytes[o + i] & 0x7Fu) << (7 * i);
-  *pp = v;
-  *lv = (uint64_t)lds_u32(X.bytes, o + vl) | ((uint64_t)lds_u32(X.bytes, o + vl + 4) << 32);
-}
-
-// The frame walk's pass over an exception list (alp_rd.rs:230-245): in list
-// order, each record's varint (rd_varint's errors), its 8 bytes (E_TRUNCATED),
-// then position < n (E_CORRUPT); the first failing record decides.  All
-// threads call it.  Returns the error and sets *end past the list.
-__device__ uint32_t alprd_list_walk(DecSmem& S, const uint8_t* p, uint64_t plen, uint64_t n, uint64_t pos,
-                                    uint64_t nexc, uint64_t* end) {
-  ExcStage X = exc_stage(S);
-  uint64_t x = 0;
-  uint32_t e = E_OK;
-  while (x < nexc) {
-    uint64_t send = pos + qmin(qmin((uint64_t)kExcStage, plen - pos), 18 * (nexc - x));
-    __syncthreads();  // the previous round's reads are done
-    uint32_t head = stage_list(X, p, pos, send, plen);
-    if (threadIdx.x == 0) {
-      uint32_t ee;
-      uint64_t q;
-      uint32_t k = exc_chain(X, head, head + (uint32_t)(send - pos), pos, plen, send == plen, nexc - x, &ee, &q);
-      S.sc[0] = q;
-      S.sc[1] = k;
-      S.flag = ee;
-    }
-    __syncthreads();
-    uint32_t k = (uint32_t)S.sc[1];
-    bool bad = false;
-    for (uint32_t r = threadIdx.x; r < k; r += blockDim.x) {
-      uint64_t pp, lv;
-      exc_decode(X, r, &pp, &lv);
-      bad |= pp >= n;
-    }
-    if (__syncthreads_or(bad)) {  // a record before any structural stop
-      e = E_CORRUPT;
-      break;
-    }
-    pos = S.sc[0];
-    x += k;
-    e = S.flag;
-    if (e || k == 0) break;  // k == 0 without an error is not reached: a stage holds a record
-  }
-  *end = pos;
-  return e;
-}
-
-// ALP-RD exceptions (alp_rd.rs:281-283): vals[p] = (left << rbw) | rights[p]
-// for each record, in list order.  A round whose positions strictly increase
-// (every list the encoder writes) is applied by the whole CTA, whose random
-// reads of the rights overlap; otherwise thread 0 applies it in order, so a
-// repeated position keeps its last record.  The list was validated by
-// alprd_list_walk (positions < n, no truncation).
-__device__ void alprd_exceptions(DecSmem& S, const uint8_t* p, uint64_t plen, uint64_t pos, uint64_t nexc,
-                                 const uint8_t* rsrc, const uint32_t* roffs, uint32_t rbw, uint64_t* vals) {
-  ExcStage X = exc_stage(S);
-  int t = threadIdx.x;
-  uint64_t x = 0;
-  while (x < nexc) {
-    uint64_t send = pos + qmin(qmin((uint64_t)kExcStage, plen - pos), 18 * (nexc - x));
-    __syncthreads();  // every thread has left the staging area (and read S.flag)
-    uint32_t head = stage_list(X, p, pos, send, plen);
-    if (t == 0) {
-      uint32_t ee;
-      uint64_t q;
-      uint32_t k = exc_chain(X, head, head + (uint32_t)(send - pos), pos, plen, send == plen, nexc - x, &ee, &q);
-      S.sc[0] = q;
-      S.sc[1] = k;
-    }
-    __syncthreads();
-    uint32_t k = (uint32_t)S.sc[1];
-    uint64_t q = S.sc[0];
-    for (uint32_t r = t; r < k; r += blockDim.x) {
-      uint64_t pp, lv;
-      exc_decode(X, r, &pp, &lv);
-      X.epos[r] = (uint32_t)pp;
-      X.left[r] = lv;
-    }
-    __syncthreads();
-    bool dis = false;
-    for (uint32_t r = t + 1; r < k; r += blockDim.x) dis |= X.epos[r] <= X.epos[r - 1];
-    bool inc = !__syncthreads_or(dis);
-    auto apply = [&](uint32_t r) {
-      uint32_t pp = X.epos[r];
-      vals[pp] = (X.left[r] << rbw) | for_value_at(rsrc, roffs[pp / kSub], pp % kSub);
-    };
-    if (inc) {
-      for (uint32_t r = t; r < k; r += blockDim.x) apply(r);
-    } else if (t == 0) {
-      for (uint32_t r = 0; r < k; r++) apply(r);
-    }
-    if (k == 0) break;  // not reached for a walked list
-    x += k;
-    pos = q;
-  }
-  __syncthreads();
 }
 
 // ---------------------------------------------------------------------------
@@ -1486,7 +1245,7 @@ __device__ uint32_t linear_values(uint32_t mode, const uint8_t* r, uint64_t len,
 // 128 KB model) and stored.  Without an
 // area the frame is not decoded (E_NO_ENTROPY_AREA).
 __device__ __noinline__ uint32_t decode_entropy_frame(DecSmem& S, const FrameDesc& d, const FrameAux& A, const uint8_t* p,
-                                         uint8_t* ent, const DecodeOut& O) {
+                                         uint8_t* ent, const uint32_t* exc_offs, const DecodeOut& O) {
   int t = threadIdx.x, l = t & 31, warp = t >> 5;
   uint64_t plen = d.plen, n = d.n, c0 = d.value_off, len = 0;
   uint32_t nsub = (uint32_t)((n + kSub - 1) / kSub);
@@ -1594,12 +1353,12 @@ __device__ __noinline__ uint32_t decode_entropy_frame(DecSmem& S, const FrameDes
       const uint8_t* rsrc = p;
       uint32_t ee = E_OK;
       if (A.t1 == 0) {
-        if (t == 0) ee = for_walk(p, plen, A.e2, n, S.eoffs);
+        if (warp == 0) ee = warp_for_walk(p, plen, A.e2, n, S.eoffs);
       } else if (A.t1 == 1) {
         e = residuals_cta(S, p + A.e2, plen - A.e2, n * 8 + 64, rb, n * 8 + 64, &len);
         if (e) return e;
         rsrc = rb;
-        if (t == 0) ee = for_walk(rb, len, 0, n, S.eoffs);
+        if (warp == 0) ee = warp_for_walk(rb, len, 0, n, S.eoffs);
       } else {
         ee = E_CORRUPT;
       }
@@ -1626,7 +1385,11 @@ __device__ __noinline__ uint32_t decode_entropy_frame(DecSmem& S, const FrameDes
       }
       __syncthreads();
       if (S.flag) return E_CORRUPT;
-      if (A.d) alprd_exceptions(S, p, plen, A.c, A.d, rsrc, S.eoffs, rbw, vals);
+      if (A.d) {
+        alprd_exceptions(p, plen, exc_offs, A.d, A.sorted, rsrc, S.eoffs, rbw,
+                         [&](uint64_t pp, uint64_t v) { vals[pp] = v; });
+        __syncthreads();
+      }
       cta_store_staged(S, O, c0, (uint32_t)n, [&](uint32_t q) { return vals[q]; });
       return E_OK;
     }
@@ -1661,16 +1424,18 @@ __device__ __noinline__ uint32_t decode_entropy_frame(DecSmem& S, const FrameDes
       uint64_t pos = A.e0;
       if (vtag == 2) {
         uint32_t ee = E_OK;
-        if (t == 0) {
+        if (warp == 0) {
           uint64_t q = vpos + vlen;
           if (q >= plen) {
             ee = E_TRUNCATED;
           } else {
             ctag = p[q];
-            S.sc[2] = q + 1;
-            if (ctag == 0) ee = for_walk(p, plen, q + 1, n, S.eoffs);
+            if (ctag == 0) ee = warp_for_walk(p, plen, q + 1, n, S.eoffs);
             else if (ctag != 1) ee = E_CORRUPT;
-            S.sc[1] = ctag;
+            if (l == 0) {
+              S.sc[1] = ctag;
+              S.sc[2] = q + 1;
+            }
           }
         }
         e = cta_bcast(S, ee);
@@ -1756,7 +1521,7 @@ __device__ __noinline__ uint32_t decode_entropy_frame(DecSmem& S, const FrameDes
 // ---------------------------------------------------------------------------
 __global__ void __launch_bounds__(kDecThreads) k_decode_frames(const uint8_t* __restrict__ stream,
                                                               const FrameDesc* __restrict__ frames, int nf,
-                                                              int dtype, FrameAux* aux,
+                                                              int dtype, const FrameAux* __restrict__ aux,
                                                               DecodeOut O, uint64_t* __restrict__ scratch,
                                                               unsigned long long* __restrict__ err,
                                                               const uint32_t* __restrict__ list,
@@ -1771,25 +1536,15 @@ __global__ void __launch_bounds__(kDecThreads) k_decode_frames(const uint8_t* __
     dtype = C.dtype;
     scratch = C.scratch;
   }
-  FrameAux& A = aux[f];  // written here only by thread 0 of a deferred walk, read after a barrier
+  const FrameAux& A = aux[f];
   if (A.err) return;
   FrameDesc d = frames[f];
   const uint8_t* p = stream + d.payload_off;
-  if (A.defer) {  // an ALP-RD frame with exceptions: the rest of the frame walk
-    uint64_t end = 0;
-    uint32_t e = alprd_list_walk(S, p, d.plen, d.n, A.c, A.d, &end);
-    if (!e) e = cta_bcast(S, threadIdx.x == 0 ? alprd_walk_tail(p, d.plen, d.n, end, A) : 0u);
-    if (e) {
-      if (threadIdx.x == 0) {
-        A.err = e;
-        atomicMin(err, ((unsigned long long)f << 8) | e);
-      }
-      return;
-    }
-  }
+  // an ALP-RD frame's exception record offsets, left there by the walk
+  const uint32_t* exc_offs = reinterpret_cast<const uint32_t*>(scratch + d.value_off);
   if (A.ent) {  // entropy-coded parts, in the frame's area (FrameDesc::aux = 1 + offset / 128)
     uint8_t* area = ent && d.aux ? ent + 128ull * (d.aux - 1) : nullptr;
-    uint32_t ee = decode_entropy_frame(S, d, A, p, area, O);
+    uint32_t ee = decode_entropy_frame(S, d, A, p, area, exc_offs, O);
     if (ee && threadIdx.x == 0) atomicMin(err, ((unsigned long long)f << 8) | ee);
     return;
   }
@@ -1898,35 +1653,32 @@ __global__ void __launch_bounds__(kDecThreads) k_decode_frames(const uint8_t* __
       break;
     case M_ALP_RD: {
       uint32_t lbw = (uint32_t)A.a, dsz = (uint32_t)A.b, rbw = 64 - lbw;
-      // With exceptions the values are assembled in the frame's scratch range
-      // first (the exception list is one sequential stream over the frame).
-      uint64_t* fo = A.d ? scratch + d.value_off : nullptr;
-      for (uint32_t k = warp; k < nsub; k += kDecWarps) {
-        uint32_t cnt = (uint32_t)qmin(kSub, n - (uint64_t)k * kSub);
-        warp_unpack(p, A.offs[0][k], cnt, [&](uint32_t i, uint64_t v) { stg[i] = v; });
-        __syncwarp();
-        uint64_t* o = fo ? fo + (size_t)k * kSub : stg;
-        warp_unpack(p, A.offs[1][k], cnt, [&](uint32_t i, uint64_t r) {
-          uint64_t c = stg[i];
-          if (c >= dsz) S.flag = 1;
-          else o[i] = (A.dict8[c] << rbw) | r;
-        });
-        __syncwarp();
-        if (!fo) warp_store(O, c0 + (uint64_t)k * kSub, cnt, [&](uint32_t q) { return stg[q]; });
-        __syncwarp();
+      if (!list) {  // the whole frame; a listed one's values were decoded as items
+        for (uint32_t k = warp; k < nsub; k += kDecWarps) {
+          uint32_t cnt = (uint32_t)qmin(kSub, n - (uint64_t)k * kSub);
+          warp_unpack(p, A.offs[0][k], cnt, [&](uint32_t i, uint64_t v) { stg[i] = v; });
+          __syncwarp();
+          warp_unpack(p, A.offs[1][k], cnt, [&](uint32_t i, uint64_t r) {
+            uint64_t c = stg[i];
+            if (c >= dsz) S.flag = 1;
+            else stg[i] = (A.dict8[c] << rbw) | r;
+          });
+          __syncwarp();
+          warp_store(O, c0 + (uint64_t)k * kSub, cnt, [&](uint32_t q) { return stg[q]; });
+          __syncwarp();
+        }
+        __syncthreads();
+        if (S.flag) {
+          e = E_CORRUPT;
+          break;
+        }
       }
-      __syncthreads();
-      if (S.flag) {
-        e = E_CORRUPT;
-        break;
-      }
-      if (fo) {
-        alprd_exceptions(S, p, plen, A.c, A.d, p, A.offs[1], rbw, fo);
-        cta_store_staged(S, O, c0, (uint32_t)n, [&](uint32_t q) { return fo[q]; });
-      }
+      alprd_exceptions(p, plen, exc_offs, A.d, A.sorted, p, A.offs[1], rbw,
+                       [&](uint64_t pp, uint64_t v) { put_out(O, lane_position(O, c0 + pp), v); });
       break;
     }
     case M_DICT: {
+      if (list) break;  // decoded as items (k_dict_values, k_decode_items)
       uint64_t card = A.a;
       const uint8_t* vb = p + A.c;
       const uint64_t* dict = nullptr;
@@ -2040,6 +1792,37 @@ __global__ void __launch_bounds__(kDecThreads) k_decode_frames(const uint8_t* __
   if (e && t == 0) atomicMin(err, ((unsigned long long)f << 8) | e);
 }
 
+// The dictionaries of the listed bit-packed DICT frames, as u64 in the frame's
+// scratch range (card <= n), for the items' lookups: one CTA per frame.
+__global__ void __launch_bounds__(kDecThreads) k_dict_values(const uint8_t* __restrict__ stream,
+                                                            const FrameDesc* __restrict__ frames,
+                                                            const FrameAux* __restrict__ aux,
+                                                            uint64_t* __restrict__ scratch,
+                                                            const uint32_t* __restrict__ list, BatchView bv) {
+  extern __shared__ __align__(16) uint8_t smem_raw[];
+  DecSmem& S = *reinterpret_cast<DecSmem*>(smem_raw);
+  int f = (int)list[blockIdx.x];
+  FrameDesc d = frames[f];
+  if (d.mode != M_DICT) return;
+  const FrameAux& A = aux[f];
+  if (A.err || A.ent) return;
+  if (bv.cols) scratch = bv.cols[bv.frame_col[f]].scratch;
+  const uint8_t* p = stream + d.payload_off;
+  const uint8_t* vb = p + A.c;
+  uint64_t* dict = scratch + d.value_off;
+  uint64_t card = A.a;
+  if (A.b == 0) {
+    for (uint64_t i = threadIdx.x; i < card; i += kDecThreads) dict[i] = ld_u64(vb + 8 * i);
+    return;
+  }
+  int l = threadIdx.x & 31;
+  chain_prefix(S, p, A.offs[1], card, ld_u64(vb), &S.u.wbuf[0][0], kDecWarps,
+               [](uint64_t v) { return unzigzag64(v); },
+               [&](uint32_t k, const uint64_t* buf, uint32_t cnt) {
+                 for (uint32_t q = l; q < cnt; q += 32) dict[(uint64_t)k * kSub + q] = buf[q];
+               });
+}
+
 // ===========================================================================
 // Warp-item decoder.  The frame table is cut into warp-sized items of at most
 // 512 values (half a FastLanes sub-block) or 2048 XORZ payload bytes (four
@@ -2053,7 +1836,10 @@ __global__ void __launch_bounds__(kDecThreads) k_decode_frames(const uint8_t* __
 //          terminator, over-long flag   -> value base and XOR carry
 // and a per-frame scan (one warp per frame) that also performs the frame-level
 // checks in the sequential decoder's order.  DICT frames and ALP-RD frames
-// with exceptions are decoded by k_decode_frames from a frame list.
+// with exceptions are items as well, and listed beside: k_dict_values writes
+// the dictionaries before the items, k_decode_frames the exceptions after them
+// (32 frames of 32,768 prices, each with about 1,000 exceptions, took 230 us
+// as one CTA each).  Frames with an entropy-coded part are only listed.
 // ===========================================================================
 constexpr int kItemVals = 512;
 constexpr int kItemBytes = 512;          // XORZ payload bytes per round of an item
@@ -2740,7 +2526,39 @@ __global__ void __launch_bounds__(kItemWarps * 32, QB_ITEM_MIN_BLOCKS) k_decode_
       warp_store_item(O, d.value_off + (uint64_t)k * kSub + hb, hc, [&](uint32_t q) { return stg[skew(q)]; });
       break;
     }
-    case M_ALP_RD: {  // frames without exceptions only
+    case M_DICT: {
+      if (A.ent) break;
+      uint32_t k = it.local >> 1, h = it.local & 1;
+      uint32_t cnt = (uint32_t)qmin(kSub, n - (uint64_t)k * kSub);
+      uint32_t hb = h * kItemVals, hc = cnt > hb ? min((uint32_t)kItemVals, cnt - hb) : 0u;
+      const uint64_t card = A.a;
+      const uint64_t* dict = scratch + d.value_off;
+      uint32_t bad = 0;
+      warp_unpack_half_fast(p, A.offs[0][k], h, cnt, [&](uint32_t i, uint64_t c) { stg[skew(i - hb)] = c; });
+      __syncwarp();
+      for (uint32_t q0 = l; q0 < hc; q0 += 32 * 8) {  // eight lookups in flight per lane
+        uint64_t v[8];
+#pragma unroll
+        for (int j = 0; j < 8; j++) {
+          uint32_t q = q0 + 32 * j;
+          uint64_t c = q < hc ? stg[skew(q)] : 0ull;
+          if (q < hc && c >= card) bad = 1;
+          v[j] = c < card ? dict[c] : 0ull;
+        }
+#pragma unroll
+        for (int j = 0; j < 8; j++)
+          if (q0 + 32 * j < hc) stg[skew(q0 + 32 * j)] = v[j];
+      }
+      __syncwarp();
+      if (warp_or_u32(bad)) {
+        e = E_CORRUPT;
+        break;
+      }
+      warp_store_item(O, d.value_off + (uint64_t)k * kSub + hb, hc, [&](uint32_t q) { return stg[skew(q)]; });
+      break;
+    }
+    case M_ALP_RD: {
+      if (A.ent) break;
       uint32_t k = it.local >> 1, h = it.local & 1;
       uint32_t lbw = (uint32_t)A.a, dsz = (uint32_t)A.b, rbw = 64 - lbw;
       uint32_t cnt = (uint32_t)qmin(kSub, n - (uint64_t)k * kSub);
@@ -2974,6 +2792,7 @@ static void set_decode_frames_smem() {
   static std::atomic<unsigned long long> done{0};
   once_per_device(done, [] {
     cudaFuncSetAttribute(k_decode_frames, cudaFuncAttributeMaxDynamicSharedMemorySize, (int)sizeof(DecSmem));
+    cudaFuncSetAttribute(k_dict_values, cudaFuncAttributeMaxDynamicSharedMemorySize, (int)sizeof(DecSmem));
   });
 }
 
@@ -2984,7 +2803,8 @@ void launch_decode_frames(const uint8_t* stream, const FrameDesc* frames, int nf
   const BatchView bv{nullptr, nullptr};
   if (nf <= 0) return;
   FrameAux* A = reinterpret_cast<FrameAux*>(aux);
-  k_walk_frames<<<(nf + 127) / 128, 128, 0, st>>>(stream, frames, nf, dtype, A, err, bv);
+  k_walk_frames<<<(nf + kWalkWarps - 1) / kWalkWarps, kWalkWarps * 32, 0, st>>>(stream, frames, nf, dtype, A, scratch,
+                                                                               err, bv);
   set_decode_frames_smem();
   k_decode_frames<<<nf, kDecThreads, sizeof(DecSmem), st>>>(stream, frames, nf, dtype, A, out, scratch, err, nullptr,
                                                             nullptr, bv);
@@ -2998,8 +2818,14 @@ void launch_decode_items(const uint8_t* stream, const FrameDesc* frames, int nf,
   if (nf <= 0) return;
   FrameAux* A = reinterpret_cast<FrameAux*>(aux);
   PreRec* P = reinterpret_cast<PreRec*>(pre);
-  k_walk_frames<<<(nf + 127) / 128, 128, 0, st>>>(stream, frames, nf, dtype, A, err, bv);
+  k_walk_frames<<<(nf + kWalkWarps - 1) / kWalkWarps, kWalkWarps * 32, 0, st>>>(stream, frames, nf, dtype, A, scratch,
+                                                                               err, bv);
   int launches = 1;
+  if (plan.nlist) {
+    set_decode_frames_smem();
+    k_dict_values<<<plan.nlist, kDecThreads, sizeof(DecSmem), st>>>(stream, frames, A, scratch, plan.list, bv);
+    launches++;
+  }
   if (plan.npre) {
     k_prepass<<<(plan.npre + kItemWarps - 1) / kItemWarps, kItemWarps * 32, 0, st>>>(stream, frames, A,
                                                                                    plan.pre_items, plan.npre, P,
@@ -3017,7 +2843,6 @@ void launch_decode_items(const uint8_t* stream, const FrameDesc* frames, int nf,
     launches++;
   }
   if (plan.nlist) {
-    set_decode_frames_smem();
     k_decode_frames<<<plan.nlist, kDecThreads, sizeof(DecSmem), st>>>(stream, frames, (int)plan.nlist, dtype, A, out,
                                                                        scratch, err, plan.list, plan.ent, bv);
     launches++;

@@ -34,6 +34,7 @@
 #include "qb_kernels.h"
 #include "qb_layout.h"
 #include "qb_scan.cuh"
+#include "qb_walk.cuh"
 
 namespace qb {
 namespace {
@@ -561,16 +562,13 @@ __global__ void __launch_bounds__(kDpThreads) k_dp_cand_compact(const uint8_t* _
 // Chain resolution and item layout (one CTA per lane).
 // ---------------------------------------------------------------------------
 // ALP-RD header up to the rights tag (alp_rd.rs:208-250); false when it does
-// not parse (the frame is then listed and the frame kernel reports it).
+// not parse (the frame is then listed and the walk reports it).  The whole
+// warp calls it, as the functions below.
 __device__ bool dp_alprd_tags(const uint8_t* p, uint64_t plen, uint64_t* nexc, uint32_t* ctag, uint32_t* rtag) {
   if (plen < 2 || p[1] > 8) return false;
   uint64_t pos = 2 + 8ull * p[1], clen = 0;
   if (pos > plen || rd_varint(p, plen, &pos, nexc) != E_OK) return false;
-  for (uint64_t x = 0; x < *nexc; x++) {
-    uint64_t pp;
-    if (rd_varint(p, plen, &pos, &pp) != E_OK || plen - pos < 8) return false;
-    pos += 8;
-  }
+  if (warp_exc_walk(p, plen, &pos, *nexc, [](bool, uint64_t, uint64_t, uint64_t) { return true; })) return false;
   if (pos >= plen) return false;
   *ctag = p[pos++];
   if (rd_varint(p, plen, &pos, &clen) != E_OK || clen > plen - pos) return false;
@@ -648,19 +646,26 @@ __device__ FrameItems dp_frame_items(const uint8_t* p, uint64_t n, uint64_t plen
       uint32_t ct = 1, rt = 1;
       bool ok = dp_alprd_tags(p, plen, &nexc, &ct, &rt);
       r.dict = true;
-      if (ok && nexc == 0 && ct == 0 && rt == 0) {
+      if (ok && ct == 0 && rt == 0) {  // items; listed as well for its exceptions
         r.nmain = nv;
+        r.list = nexc != 0;
       } else {
         r.list = true;
         if (!ok || ct == 1 || rt == 1) r.ent = ent_area_bytes(n, mode, plog2);
       }
       return r;
     }
+    case 19:  // items; listed as well for its dictionary
+      r.dict = true;
+      r.list = true;
+      if (dp_entropy_frame(p, plen, mode)) r.ent = ent_area_bytes(n, mode, plog2);
+      else r.nmain = nv;
+      return r;
     default:
       r.list = true;
       break;
   }
-  r.dict = mode == 19 || mode == 53 || mode == 52;
+  r.dict = mode == 53;
   if (r.list && dp_entropy_frame(p, plen, mode)) r.ent = ent_area_bytes(n, mode, plog2);
   return r;
 }
@@ -773,23 +778,9 @@ __global__ void __launch_bounds__(kChainThreads) k_dp_marks(const DpHead* __rest
   }
 }
 
-// An ALP-RD frame's exception list (records of a varint position and an
-// 8-byte left part) is walked record by record, each read depending on the
-// one before; the warp first pulls the list's cache lines into L1 so that the
-// walk's reads hit there.
-__device__ __forceinline__ void dp_warp_prefetch_alprd(const uint8_t* p, uint64_t plen, uint32_t mode) {
-  if (mode != 52 || plen < 2) return;
-  const int l = threadIdx.x & 31;
-  uint64_t pos = 2 + 8ull * p[1], nexc = 0;
-  if (pos > plen || rd_varint(p, plen, &pos, &nexc) != E_OK) return;
-  uint64_t end = nexc > plen ? plen : qmin(plen, pos + 18 * nexc + 32);
-  for (uint64_t o = pos + 128ull * l; o < end; o += 128ull * 32)
-    asm volatile("prefetch.global.L1 [%0];" ::"l"(p + o));
-}
-
 // The warp items of every marked candidate (dp_frame_items), across the GPU:
 // nodes[j] for the j-th marked candidate, its candidate index in .succ.  One
-// warp per frame: the prefetch above, then lane 0 counts the items.
+// warp per frame.
 __global__ void k_dp_items(const uint8_t* __restrict__ s, const DpHead* __restrict__ H, int lane,
                            const DpCand* __restrict__ cand, const uint32_t* __restrict__ fidx,
                            const uint64_t* __restrict__ ctl, DpNode* __restrict__ nodes) {
@@ -801,9 +792,8 @@ __global__ void k_dp_items(const uint8_t* __restrict__ s, const DpHead* __restri
     uint32_t i = fidx[j];
     DpCand c = cand[i];
     const uint8_t* p = s + c.pos + 9;
-    dp_warp_prefetch_alprd(p, c.plen_mode >> 8, c.plen_mode & 0xFF);
-    if ((threadIdx.x & 31) != 0) continue;
     FrameItems it = dp_frame_items(p, c.n, c.plen_mode >> 8, c.plen_mode & 0xFF, plog2);
+    if ((threadIdx.x & 31) != 0) continue;
     DpNode d;
     d.succ = i;
     d.nmain = it.nmain;
@@ -1321,9 +1311,8 @@ __global__ void k_dpb_items(DpBatch B) {
     const DpBLane& Ln = B.lanes[c];
     uint64_t i = lo + B.flist[j];
     DpCand cd = B.cand[i];
-    dp_warp_prefetch_alprd(Ln.s + cd.pos + 9, cd.plen_mode >> 8, cd.plen_mode & 0xFF);
-    if ((threadIdx.x & 31) != 0) continue;
     FrameItems it = dp_frame_items(Ln.s + cd.pos + 9, cd.n, cd.plen_mode >> 8, cd.plen_mode & 0xFF, Ln.L.plog2);
+    if ((threadIdx.x & 31) != 0) continue;
     DpNode d;
     d.succ = (uint32_t)(i - lo);
     d.nmain = it.nmain;

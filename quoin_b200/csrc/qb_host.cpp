@@ -893,7 +893,8 @@ bool entropy_frame_h(const uint8_t* p, uint64_t plen, uint32_t mode) {
 
 // Warp items of every frame (512 values, or kXorzItemBytes payload bytes for XORZ).
 // Frames the items do not cover, or whose header cannot be read here, go to
-// the frame list; the device walk reports their errors.  Listed frames with
+// the frame list (DICT frames and ALP-RD frames with exceptions are in both);
+// the device walk reports their errors.  Listed frames with
 // an entropy-coded part get a device area (ent_area_bytes: the mode's layout,
 // the range coder's model, a predictor table, the LZ cascade's scratch)
 // (128-byte units, 1 + its offset in FrameDesc::aux; 0 = none).
@@ -949,13 +950,18 @@ void build_items(const uint8_t* src, LaneIdx& L) {
         L.need_scan = true;
         break;
       }
-      case 52: {  // ALP-RD: items only without exceptions and with both parts bit-packed
+      case 52: {  // ALP-RD: items with both parts bit-packed, listed as well for its exceptions
         uint64_t nexc = 1;
         uint32_t ct = 1, rt = 1;
-        if (alprd_tags_h(p, plen, &nexc, &ct, &rt) && nexc == 0 && ct == 0 && rt == 0) add_main(nv);
-        else L.list.push_back(f);
+        const bool packed = alprd_tags_h(p, plen, &nexc, &ct, &rt) && ct == 0 && rt == 0;
+        if (packed) add_main(nv);
+        if (!packed || nexc) L.list.push_back(f);
         break;
       }
+      case 19:  // DICT: items with values and codes not entropy-coded, listed as well for its dictionary
+        if (!entropy_frame_h(p, plen, 19)) add_main(nv);
+        L.list.push_back(f);
+        break;
       default:
         L.list.push_back(f);
         break;
