@@ -1,5 +1,5 @@
 // Block decoder (reference src/decoder.rs:145-190 and the per-codec decode
-// functions).  Two kernels:
+// functions).  The kernels:
 //  * k_walk_frames — one warp per frame: validates the frame's payload
 //    structure in the reference's check order and records the byte offsets of
 //    its FastLanes sub-blocks and ALP-RD exceptions (qb_walk.cuh);
@@ -23,6 +23,8 @@ constexpr int kDictSmem = 2048;
 constexpr int kXorzChunk = kDecThreads * 8;  // payload bytes per XORZ step
 constexpr int kXorzRing = 4096;              // decoded XORZ values awaiting their store
 constexpr uint64_t kSelStep = 512;           // select-table granularity (valid values)
+constexpr uint32_t kRansRing = 4096;         // rANS stream bytes staged at a time (four such pieces held)
+constexpr uint32_t kRansSteps = kRansRing / 8;  // steps of four symbols between stagings (at most 8 bytes a step)
 
 // Per-frame results of the walk (device memory, one per frame).
 struct FrameAux {
@@ -355,8 +357,9 @@ struct DecSmem {
     struct {                         // rANS tables (rans.rs:110-175)
       uint32_t freq[256];
       uint32_t cum[257];
-      uint8_t sym[4096];
       uint64_t sc[4];
+      uint2 slot[4096];              // per slot: frequency | symbol << 16, slot - cumulative frequency
+      uint8_t ring[4 * kRansRing + 128];  // stream bytes around the read position, the first 128 again at the end
     } r;
   } u;
 };
@@ -783,16 +786,22 @@ __device__ void alprd_exceptions(const uint8_t* p, uint64_t plen, const uint32_t
 // rans.rs:110-175 behind the entropy tag of entropy/mod.rs:152-178.
 // ---------------------------------------------------------------------------
 
-// One rANS block decoded by the CTA: thread 0 reads the header and runs the
-// decoder (four states share one byte stream, so it is sequential); all
-// threads build the slot -> symbol table.  Writes the first min(len, cap)
-// symbols to out and the decoded length to *len_out.  Error kinds and their
-// order follow rans.rs.
+// One rANS block decoded by the CTA: thread 0 reads the header, all threads
+// build the slot table, and lanes 0..3 of warp 0 run the four states, which
+// share one byte stream: a step decodes four symbols, and two votes tell each
+// lane how many of its step's bytes the states before it take.  The other
+// warps keep the next bytes staged in shared memory.  A step's dependent chain
+// (slot load, multiply-add, votes, byte selection) bounds it, about 70 ns for
+// four symbols (thread 0 alone took 90 ns a symbol: 76 ms to decode 1,000,003
+// f32 readings and as many f64 prices at Balanced-in-pool, now 10 ms).  A
+// state that needs more than two bytes (only in a damaged stream) makes the
+// steps run state by state.  Writes the first
+// min(len, cap) symbols to out and the decoded length to *len_out.  Error
+// kinds and their order follow rans.rs.
 __device__ __noinline__ uint32_t rans_decode_cta(DecSmem& S, const uint8_t* p, uint64_t plen, uint64_t max_len, uint8_t* out,
                                    uint64_t cap, uint64_t* len_out) {
   int t = threadIdx.x;
   for (int i = t; i < 256; i += blockDim.x) S.u.r.freq[i] = 0;
-  for (int i = t; i < 4096; i += blockDim.x) S.u.r.sym[i] = 0;
   __syncthreads();
   if (t == 0) {
     uint32_t e = E_OK;
@@ -836,37 +845,139 @@ __device__ __noinline__ uint32_t rans_decode_cta(DecSmem& S, const uint8_t* p, u
     __syncthreads();
     return e;
   }
-  for (int sy = t; sy < 256; sy += blockDim.x)
-    for (uint32_t slot = S.u.r.cum[sy]; slot < S.u.r.cum[sy + 1] && slot < 4096; slot++) S.u.r.sym[slot] = (uint8_t)sy;
-  __syncthreads();
-  if (t == 0) {
-    uint64_t pos = S.u.r.sc[1], n64 = S.u.r.sc[2];
-    uint32_t x[4] = {0, 0, 0, 0};
-    uint32_t ee = E_OK;
-    for (int k = 0; k < 4 && !ee; k++) {
-      if (plen < pos + 4) {
-        ee = E_TRUNCATED;
-      } else {
-        x[k] = ld_u32(p + pos);
-        pos += 4;
-      }
+  // every slot's symbol: the last whose cumulative frequency is at or below it
+  // (symbol 0 past the last, when a repeated symbol leaves the table short)
+  for (uint32_t slot = t; slot < 4096; slot += blockDim.x) {
+    uint32_t lo = 0, hi = 256;
+    while (hi - lo > 1) {
+      uint32_t mid = (lo + hi) >> 1;
+      if (S.u.r.cum[mid] <= slot) lo = mid; else hi = mid;
     }
-    for (uint64_t i = 0; i < n64 && !ee; i++) {
-      uint32_t idx = (uint32_t)(i & 3), xi = x[idx], slot = xi & 4095u;
-      uint32_t sy = S.u.r.sym[slot];
-      if (i < cap) out[i] = (uint8_t)sy;
-      uint32_t xn = S.u.r.freq[sy] * (xi >> 12) + slot - S.u.r.cum[sy];
-      while (xn < (1u << 23)) {
-        if (pos >= plen) {
-          ee = E_TRUNCATED;
+    if (slot >= S.u.r.cum[256]) lo = 0;
+    S.u.r.slot[slot] = make_uint2(S.u.r.freq[lo] | lo << 16, slot - S.u.r.cum[lo]);
+  }
+  const int warp = t >> 5, l = t & 31;
+  const uint64_t n64 = S.u.r.sc[2], body = S.u.r.sc[1] + 16;  // stream bytes follow the four states
+  const bool have = plen >= body;
+  // stream bytes are staged in pieces of kRansRing from payload offset `body`
+  const uint64_t sbytes = have ? plen - body : 0, pieces = (sbytes + kRansRing - 1) / kRansRing;
+  auto stage = [&](uint64_t c, int t0, int nt) {
+    if (c >= pieces) return;
+    uint64_t b0 = c * kRansRing;
+    uint32_t cnt = (uint32_t)qmin(kRansRing, sbytes - b0);
+    uint8_t* dst = S.u.r.ring + (c & 3) * kRansRing;
+    const uint8_t* src = p + body + b0;
+    for (uint32_t i = 4 * t0; i < cnt; i += 4 * nt) {
+      uint32_t w = 0;
+      if (i + 4 <= cnt) w = ld_u32(src + i);
+      else for (uint32_t q = i; q < cnt; q++) w |= (uint32_t)src[q] << (8 * (q - i));
+      *reinterpret_cast<uint32_t*>(dst + i) = w;
+      if ((c & 3) == 0 && i < 128) *reinterpret_cast<uint32_t*>(S.u.r.ring + 4 * kRansRing + i) = w;
+    }
+  };
+  stage(0, t, blockDim.x);
+  stage(1, t, blockDim.x);
+  const uint32_t sel = l & 3;
+  uint32_t x = have ? ld_u32(p + body - 16 + 4 * sel) : 0u;
+  uint32_t ee = have ? E_OK : E_TRUNCATED;
+  uint64_t pos = 0, staged = 2;  // read position in the stream; pieces staged
+  __syncthreads();
+  for (uint64_t i0 = 0; i0 < n64 && !ee; i0 += 4 * kRansSteps) {
+    // pieces floor(pos / kRansRing) and the next are staged: enough for kRansSteps steps
+    const bool more = staged < pieces && staged < pos / kRansRing + 3;
+    if (warp) {
+      if (more) stage(staged, t - 32, blockDim.x - 32);
+    } else {
+      const uint64_t i1 = qmin(n64, i0 + 4 * kRansSteps);
+      // Batches of eight whole steps, all of whose symbols are stored, without
+      // a check in the chain: positions are 32-bit offsets in the ring, a
+      // window holds the 8 bytes a step may take, and the votes' nibbles (lanes
+      // 4.. repeat the states of lanes 0..3) give a lane's place in it.  A
+      // batch that met a state below 2^7 (more than two bytes due) or ran past
+      // the stream is undone and left to the checked steps below.
+      uint64_t i = i0;
+      const uint32_t below = ((1u << sel) - 1u) * 0x11u;
+      const uint8_t* ring = S.u.r.ring;
+      auto next8 = [&](uint32_t q, uint32_t* hi) {  // ring[q .. q + 8), the ring continued past its end
+        const uint32_t* r32 = reinterpret_cast<const uint32_t*>(ring) + (q >> 2);
+        const uint32_t w0 = r32[0], w1 = r32[1], w2 = r32[2];
+        *hi = __funnelshift_r(w1, w2, q * 8);
+        return __funnelshift_r(w0, w1, q * 8);
+      };
+      const uint64_t whole = qmin(i1, cap);
+      uint32_t q = (uint32_t)pos & (4 * kRansRing - 1);
+      uint64_t lin = pos - q;  // stream offset of ring offset 0
+      for (; i + 32 <= whole; i += 32) {
+        if (q >= 4 * kRansRing) {
+          q -= 4 * kRansRing;
+          lin += 4 * kRansRing;
+        }
+        static_assert(64 + 12 <= 128, "a batch from the ring's last byte stays in its continuation");
+        const uint32_t x0 = x, q0 = q;
+        uint32_t low = 0xFFFFFFFFu, whi;
+        uint32_t wlo = next8(q, &whi);
+        uint8_t* o = out + i + sel;
+#pragma unroll
+        for (int j = 0; j < 8; j++) {
+          const uint2 sl = S.u.r.slot[x & 4095u];
+          const uint32_t xn = (sl.x & 0xFFFFu) * (x >> 12) + sl.y;
+          const bool b1 = xn < (1u << 23), b2 = xn < (1u << 15);
+          const uint32_t m1 = __ballot_sync(0xffffffffu, b1), m2 = __ballot_sync(0xffffffffu, b2);
+          const uint32_t m = (m1 & 0x0Fu) | (m2 & 0xF0u);
+          low = min(low, xn);
+          if (l < 4) o[4 * j] = (uint8_t)(sl.x >> 16);
+          const uint32_t two = __byte_perm(wlo, whi, __popc(m & below) * 0x11u + 0x10u);
+          q += __popc(m);
+          wlo = next8(q, &whi);
+          const uint32_t xa = __byte_perm(two, xn, 0x6540), xb = __byte_perm(two, xn, 0x5401);
+          x = b2 ? xb : (b1 ? xa : xn);
+        }
+        if (__any_sync(0xffffffffu, low < (1u << 7)) || lin + q > sbytes) {
+          x = x0;
+          q = q0;
           break;
         }
-        xn = (xn << 8) | p[pos++];
       }
-      x[idx] = xn;
+      pos = lin + q;
+      for (uint32_t left = 8; i < i1 && (left || i + 32 > whole); i += 4, left -= left ? 1 : 0) {
+        const bool act = i + sel < n64;
+        const uint2 sl = S.u.r.slot[x & 4095u];
+        uint32_t xn = (sl.x & 0xFFFFu) * (x >> 12) + sl.y;
+        if (l < 4 && act && i + sel < cap) out[i + sel] = (uint8_t)(sl.x >> 16);
+        for (uint32_t k = 0; k < 4 && i + k < n64 && !ee; k++) {  // state by state, bytes from memory
+          uint32_t xk = __shfl_sync(0xffffffffu, xn, k);
+          while (xk < (1u << 23)) {
+            if (pos >= sbytes) {
+              ee = E_TRUNCATED;
+              break;
+            }
+            xk = (xk << 8) | p[body + pos++];
+          }
+          if (sel == k) xn = xk;
+        }
+        if (act) x = xn;
+        if (ee) break;
+      }
+      i0 = i - 4 * kRansSteps;  // the next round starts here
+      if (l == 0) {
+        S.u.r.sc[0] = ee;
+        S.u.r.sc[3] = pos;
+        S.u.r.sc[1] = i0;
+      }
     }
-    S.u.r.sc[0] = ee;
+    __syncthreads();
+    if (more) staged++;
+    ee = (uint32_t)S.u.r.sc[0];
+    pos = S.u.r.sc[3];
+    i0 = S.u.r.sc[1];
+    // a damaged step may have jumped ahead of what is staged
+    while (staged < pos / kRansRing + 2 && staged < pieces) {
+      stage(staged, t, blockDim.x);
+      staged++;
+    }
+    __syncthreads();
   }
+  if (t == 0) S.u.r.sc[0] = ee;
   __syncthreads();
   e = (uint32_t)S.u.r.sc[0];
   *len_out = S.u.r.sc[2];
@@ -1244,6 +1355,74 @@ __device__ uint32_t linear_values(uint32_t mode, const uint8_t* r, uint64_t len,
 // frame's entropy area (24 bytes per value + 128, then the range coder's
 // 128 KB model) and stored.  Without an
 // area the frame is not decoded (E_NO_ENTROPY_AREA).
+// Exclusive prefix sum over the CTA's threads (wrapping); *total = the sum.
+__device__ inline uint64_t cta_excl_sum(DecSmem& S, uint64_t v, uint64_t* total) {
+  int l = threadIdx.x & 31, warp = threadIdx.x >> 5;
+  uint64_t inc = warp_incl_scan(v), before = 0, tot = 0;
+  __syncthreads();  // wxor is free
+  if (l == 31) S.wxor[warp] = inc;
+  __syncthreads();
+  for (int w = 0; w < kDecWarps; w++) {
+    if (w < warp) before += S.wxor[w];
+    tot += S.wxor[w];
+  }
+  *total = tot;
+  return before + inc - v;
+}
+
+// vals[0 .. n) = running sums of the n zigzag LEB128 deltas that r[0 .. len)
+// holds (float_mult.rs:112-125), by the whole CTA: a thread owns a stretch of
+// bytes and the values whose last byte lies in it; a scan numbers them and a
+// scan of their sums gives the values before.  Errors as reading them one by
+// one: the first value longer than 10 bytes (E_CORRUPT) or cut off by the
+// end (E_TRUNCATED), then bytes left over (E_CORRUPT).  (131,072 values took
+// thread 0 9 ms.)
+__device__ uint32_t leb_deltas_cta(DecSmem& S, const uint8_t* r, uint64_t len, uint64_t n, uint64_t* vals) {
+  const uint64_t seg = (len + kDecThreads - 1) / kDecThreads;
+  const uint64_t a0 = qmin(threadIdx.x * seg, len), a1 = qmin(a0 + seg, len);
+  // the start of the value that r[a0] belongs to, no further than 10 bytes back
+  uint64_t s0 = a0;
+  while (s0 > 0 && a0 - s0 < 10 && (r[s0 - 1] & 0x80)) s0--;
+  uint64_t cnt = 0, sum = 0, total, nsum;
+  for (int pass = 0; pass < 2; pass++) {
+    uint64_t i = 0, run = 0;
+    bool bad = false;
+    if (pass) {
+      i = cta_excl_sum(S, cnt, &total);
+      run = cta_excl_sum(S, sum, &nsum);
+    }
+    uint64_t v = 0;
+    uint32_t k = 0;  // bytes of the value so far
+    for (uint64_t q = s0; q < a1; q++) {
+      const uint32_t b = r[q];
+      if (k < 10) v |= (uint64_t)(b & 0x7F) << (7 * k);
+      k++;
+      if (b & 0x80) continue;
+      if (pass) {
+        if (i < n) {
+          if (k > 10) bad = true;
+          run += unzigzag64(v);
+          vals[i] = run;
+          if (i == n - 1 && q != len - 1) bad = true;  // bytes left over
+        }
+        i++;
+      } else {
+        cnt++;
+        sum += unzigzag64(v);
+      }
+      v = 0;
+      k = 0;
+    }
+    if (pass && __syncthreads_or(bad)) return E_CORRUPT;
+  }
+  if (n == 0) return len ? E_CORRUPT : E_OK;
+  if (total >= n) return E_OK;
+  // the value cut off by the end of the bytes
+  uint64_t tail = 0;
+  while (tail < 10 && tail < len && (r[len - 1 - tail] & 0x80)) tail++;
+  return tail >= 10 ? E_CORRUPT : E_TRUNCATED;
+}
+
 __device__ __noinline__ uint32_t decode_entropy_frame(DecSmem& S, const FrameDesc& d, const FrameAux& A, const uint8_t* p,
                                          uint8_t* ent, const uint32_t* exc_offs, const DecodeOut& O) {
   int t = threadIdx.x, l = t & 31, warp = t >> 5;
@@ -1320,20 +1499,7 @@ __device__ __noinline__ uint32_t decode_entropy_frame(DecSmem& S, const FrameDes
       e = residuals_cta(S, p + 2, plen - 2, cap, res, cap, &len);
       if (e) return e;
       uint64_t* vals = reinterpret_cast<uint64_t*>(ent + ((cap + 15) & ~15ull));
-      uint32_t ee = E_OK;
-      if (t == 0) {
-        uint64_t pos = 0;
-        int64_t prev = 0;
-        for (uint64_t i = 0; i < n && !ee; i++) {
-          uint64_t z = 0;
-          ee = rd_varint(res, len, &pos, &z);
-          if (ee) break;
-          prev = (int64_t)((uint64_t)prev + unzigzag64(z));
-          vals[i] = (uint64_t)prev;
-        }
-        if (!ee && pos != len) ee = E_CORRUPT;
-      }
-      e = cta_bcast(S, ee);
+      e = leb_deltas_cta(S, res, len, n, vals);
       if (e) return e;
       double scale = kFmScales[A.a];
       cta_store_staged(S, O, c0, (uint32_t)n,
