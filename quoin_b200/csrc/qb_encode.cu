@@ -18,7 +18,6 @@ constexpr int kSubsMax = kMaxBlock / kSub;  // 128
 constexpr uint32_t kHashCap = 2048;         // smem hash slots (dict / ALP-RD left parts)
 constexpr uint32_t kHashLimit = 1536;       // distinct keys before falling back to scratch
 constexpr uint32_t kLbBits = 1u << 17;      // dict cardinality lower-bound bitset
-constexpr uint32_t kRunsSmem = 4096;
 constexpr uint32_t kNoLb = 0xFFFFFFFFu;
 
 // 17-bit bucket of the dictionary cardinality lower-bound bitset.
@@ -141,7 +140,8 @@ __device__ inline int64_t fm_k(uint64_t x, int s) {
 // Shared memory of the competition and emission kernels
 // ---------------------------------------------------------------------------
 struct RdArea {
-  uint64_t smp[4096];
+  uint32_t smp[2][4096];  // the sample's top 24 bits (two buffers of the sort)
+  uint8_t cp[4096];       // leading bits (of 24) a sorted key shares with the one before
   uint32_t hkey[kHashCap];
   uint32_t hcnt[kHashCap];
 };
@@ -150,13 +150,9 @@ struct DictArea {
   uint32_t hval[kHashCap];
   uint64_t sorted[kHashCap];
 };
-struct RleArea {
-  uint32_t starts[kRunsSmem];
-};
 union BigArea {
   RdArea rd;
   DictArea dict;
-  RleArea rle;
 };
 constexpr uint32_t kRansChunk = 4096;  // bytes staged per step of the rANS encoder
 struct RansArea {
@@ -167,6 +163,26 @@ struct RansArea {
   uint32_t hdr, emitted;
   uint32_t bound;  // a lower bound on the coded bytes (rans_plan)
 };
+
+// What the competition leaves for the emission besides the mode: per sub-block
+// the ALP-RD (or RLE) layout, per block its dictionary of left parts and the DICT
+// dictionary's size (kept in the block's scratch when it is small), so that
+// the emission makes no pass over the block before it packs, and several CTAs
+// can share a block.
+struct RdRec {
+  uint64_t rmin;    // smallest right part (RLE: smallest length of the run chunk)
+  uint32_t eb;      // exception bytes
+  uint16_t ne;      // exceptions
+  uint8_t cw, rw;   // code and right widths (RLE: rw, the chunk's)
+  uint8_t cmin, pad[7];
+};
+static_assert(sizeof(RdRec) == 24, "RdRec layout");
+struct BlkRec {
+  uint64_t dict8[8];
+  uint64_t vlen;    // DICT value bytes
+  uint32_t dl, card, vtag, pad;  // card: DICT's values (0 = not kept), RLE's runs
+};
+static_assert(sizeof(BlkRec) == 88, "BlkRec layout");
 
 struct EncSmem {
   uint8_t w_a[kSubsMax];   // FoR widths (also ALP widths in emit)
@@ -184,12 +200,16 @@ struct EncSmem {
   uint32_t distinct_bits[512];
   uint64_t alp_smp[kEncWarps][32];
   double rd_pv[24];
+  uint32_t rd_top[24][8];  // per cut: the sample's largest left-part groups (size << 12 | first sorted key)
+  uint32_t rd_cand[8], rd_cnt[8], rd_ncand;
+  uint8_t rd_mask[kSubsMax];  // per sub-block: which of rd_cand occur
+  uint32_t rd_ne[kSubsMax], rd_eb[kSubsMax];  // per sub-block: ALP-RD exceptions and their bytes
   uint64_t dict8[8];
   uint64_t red[kEncWarps];
   uint32_t red32[kEncWarps];
   uint64_t sc[8];
   uint32_t exp_lo, exp_hi;
-  BigArea big;
+  alignas(16) BigArea big;
   RansArea ra;
 };
 
@@ -232,21 +252,35 @@ __device__ inline void warp_minmax(uint32_t cnt, bool sgn, V val, uint64_t* mn_o
   }
 }
 
+// The low `k` bytes of v at d (k <= 4).
+__device__ __forceinline__ void put_low(uint8_t* d, uint32_t v, uint32_t k) {
+  for (uint32_t i = 0; i < k; i++) d[i] = (uint8_t)(v >> (8 * i));
+}
+
 // Pack one FoR sub-block (header + FastLanes words) at dst; residual of
 // index i = val(i) - mn for i < cnt, 0 for the padding (reference
-// for_bitpack.rs:47-96, bitpack.rs:48-133).
+// for_bitpack.rs:47-96, bitpack.rs:48-133).  Consecutive lanes' words are
+// consecutive in memory, at any byte address: a lane writes the aligned word
+// that ends its own and starts with the top of its neighbour's (lane 0: of the
+// last lane's word a row earlier), so a row of 32 words is one aligned store
+// and only the stream's first and last bytes are written singly (a byte per
+// store took 55 us for 16,777,216 timestamps' frames, a third of the copy rate).
+// Above 32 bits, 16 lanes hold 64-bit words; the two half warps take rows 0-31
+// and 32-63, whose bits meet at the middle of a word when the width is odd:
+// the second half's first word waits for the first half's end.
 template <class V>
 __device__ inline void warp_for_pack(uint8_t* dst, uint32_t cnt, uint64_t mn, uint32_t w, V val) {
   int lane = threadIdx.x & 31;
-  if (lane == 0) {
-    put_u8(dst, w);
-    put_u64(dst + 1, mn);
-  }
+  if (lane < 8) dst[1 + lane] = (uint8_t)(mn >> (8 * lane));
+  if (lane == 8) put_u8(dst, w);
   if (w == 0) return;
   uint8_t* words = dst + 9;
+  const uint32_t mis = (uint32_t)(reinterpret_cast<uintptr_t>(words) & 3), sh = 8 * mis;
+  uint32_t* al = reinterpret_cast<uint32_t*>(words - mis);  // al[j]: the aligned word that ends word j of the stream
   if (w <= 32) {
     uint64_t acc = 0;
-    uint32_t nb = 0, wd = 0;
+    uint32_t nb = 0, carry = 0, first = 0;
+    uint32_t* o = al + lane;
     for (uint32_t r0 = 0; r0 < 32; r0 += 8) {
      uint32_t rs[8];
 #pragma unroll
@@ -261,60 +295,107 @@ __device__ inline void warp_for_pack(uint8_t* dst, uint32_t cnt, uint64_t mn, ui
       acc |= (uint64_t)res << nb;
       nb += w;
       if (nb >= 32) {
-        put_u32(words + 4u * (wd * 32u + lane), (uint32_t)acc);
-        wd++;
+        const uint32_t x = (uint32_t)acc, rot = __shfl_sync(0xffffffffu, x, (lane + 31) & 31);
+        const uint32_t out = __funnelshift_l(lane ? rot : carry, x, sh);
+        if (o != al || !mis) *o = out;  // the very first word is shared with what precedes the stream
+        else first = x;
+        carry = rot;
+        o += 32;
         acc >>= 32;
         nb -= 32;
       }
      }
     }
-  } else if (lane < 16) {
-    unsigned __int128 acc = 0;
-    uint32_t nb = 0, wd = 0;
-    for (uint32_t r0 = 0; r0 < 64; r0 += 8) {
+    if (lane == 0 && mis) {
+      put_low(words, first, 4 - mis);
+      put_low(reinterpret_cast<uint8_t*>(o), carry >> (32 - sh), mis);
+    }
+  } else {
+    const uint32_t h = (uint32_t)lane >> 4, fl = lane & 15;
+    const uint32_t half = h * 32 * w;  // the half's first bit
+    uint64_t acc = 0, first = 0;
+    uint32_t nb = half & 63, wi = half >> 6, carry = 0;
+    bool wait = h != 0;
+    auto put = [&](uint32_t k, uint64_t x, uint32_t prev) {  // word k of the lane; prev: the 32 bits before it
+      const uint32_t lo = (uint32_t)x, hi = (uint32_t)(x >> 32), j = 2 * (k * 16 + fl);
+      if (mis && j == 0) put_low(words, lo, 4 - mis);
+      else al[j] = __funnelshift_l(prev, lo, sh);
+      al[j + 1] = __funnelshift_l(lo, hi, sh);
+    };
+    for (uint32_t r0 = 0; r0 < 32; r0 += 8) {
      uint64_t rs[8];
 #pragma unroll
      for (int q = 0; q < 8; q++) {
-       uint32_t iq = (r0 + q) * 16 + lane;
+       uint32_t iq = (h * 32 + r0 + q) * 16 + fl;
        rs[q] = iq < cnt ? (val(iq) - mn) : 0ull;
      }
 #pragma unroll
      for (int q = 0; q < 8; q++) {
       uint64_t res = rs[q];
       if (w < 64) res &= (1ull << w) - 1ull;
-      acc |= (unsigned __int128)res << nb;
+      acc |= res << nb;
       nb += w;
-      if (nb >= 64) {
-        put_u64(words + 8u * (wd * 16u + lane), (uint64_t)acc);
-        wd++;
-        acc >>= 64;
+      const uint32_t rot = __shfl_sync(0xffffffffu, (uint32_t)(acc >> 32), (fl + 15) & 15, 16);
+      if (nb >= 64) {  // the same for the lanes of a half
+        if (wait) first = acc;
+        else put(wi, acc, fl ? rot : carry);
+        wait = false;
+        carry = rot;
+        wi++;
         nb -= 64;
+        acc = nb ? res >> (w - nb) : 0ull;
       }
      }
     }
+    // the second half's first word: its low bits (an odd width) and what
+    // precedes lane 0's are the first half's last
+    const uint32_t low = __shfl_sync(0xffffffffu, (uint32_t)acc, fl), before = __shfl_sync(0xffffffffu, carry, 0);
+    if (w & 1) first |= low;
+    const uint32_t rot = __shfl_sync(0xffffffffu, (uint32_t)(first >> 32), (fl + 15) & 15, 16);
+    if (h) put(w >> 1, first, fl ? rot : before);
+    if (lane == 16 && mis) put_low(reinterpret_cast<uint8_t*>(al + 32u * w), carry >> (32 - sh), mis);
   }
+}
+
+// S.subsz[0 .. nsub) (sizes) turned into offsets from `base`, the end in
+// S.subsz[nsub].  All threads call it; the sizes are written before.
+__device__ inline void block_offsets(EncSmem& S, uint32_t nsub, uint32_t base) {
+  __syncthreads();
+  if (threadIdx.x < 32) {
+    uint32_t c[kSubsMax / 32], s = 0;
+#pragma unroll
+    for (int j = 0; j < kSubsMax / 32; j++) {
+      uint32_t k = threadIdx.x * (kSubsMax / 32) + j;
+      c[j] = k < nsub ? S.subsz[k] : 0u;
+      s += c[j];
+    }
+    uint32_t inc = warp_incl_scan(s), off = base + inc - s;
+#pragma unroll
+    for (int j = 0; j < kSubsMax / 32; j++) {
+      uint32_t k = threadIdx.x * (kSubsMax / 32) + j;
+      if (k < nsub) S.subsz[k] = off;
+      off += c[j];
+    }
+    if (threadIdx.x == 31) S.subsz[nsub] = base + inc;
+  }
+  __syncthreads();
 }
 
 // Second half of the FoR stream writer: with S.w_a[k] / S.submin[k] set for
 // every sub-block, lays out varint(M) + sub-blocks and (dst non-null) packs
-// val(0..M).  Returns the byte length (all threads).
+// sub-blocks k0 .. k1 of val(0..M), the varint with the first.  Returns the
+// byte length (all threads).
 template <class V>
-__device__ uint64_t block_for_write(EncSmem& S, uint8_t* dst, uint32_t M, V val) {
+__device__ uint64_t block_for_write(EncSmem& S, uint8_t* dst, uint32_t M, V val, uint32_t k0 = 0,
+                                    uint32_t k1 = kSubsMax) {
   int warp = threadIdx.x >> 5;
   uint32_t nsub = (M + kSub - 1) / kSub;
-  if (threadIdx.x == 0) {
-    uint32_t off = varint_len(M);
-    for (uint32_t k = 0; k < nsub; k++) {
-      S.subsz[k] = off;
-      off += 9 + 128u * S.w_a[k];
-    }
-    S.subsz[nsub] = off;
-    if (dst) put_varint(dst, M);
-  }
-  __syncthreads();
+  for (uint32_t k = threadIdx.x; k < nsub; k += blockDim.x) S.subsz[k] = 9 + 128u * S.w_a[k];
+  block_offsets(S, nsub, varint_len(M));
+  if (threadIdx.x == 0 && dst && k0 == 0) put_varint(dst, M);
   uint64_t total = S.subsz[nsub];
   if (dst) {
-    for (uint32_t k = warp; k < nsub; k += kEncWarps) {
+    for (uint32_t k = k0 + warp; k < min(nsub, k1); k += kEncWarps) {
       uint32_t cnt = min((uint32_t)kSub, M - k * kSub);
       warp_for_pack(dst + S.subsz[k], cnt, S.submin[k], S.w_a[k], [&](uint32_t i) { return val(k * kSub + i); });
     }
@@ -488,56 +569,162 @@ __device__ inline uint32_t rd_code_bits(uint32_t dl) {
   return b ? b : 1;
 }
 
+// Ascending bitonic sort of 512 * K u32 keys, K per thread: a warp holds
+// 32 * K consecutive positions (row r, lane l at 32r + l), so only the
+// exchanges between warps (10 of the 66 steps at 2,048 keys) pass through
+// shared memory and take a barrier.  `buf` holds two buffers; the sorted keys
+// end in the returned one, readable after the barrier inside.
+template <int K>
+__device__ uint32_t* block_sort_u32(uint32_t (&a)[K], uint32_t (*buf)[4096]) {
+  constexpr uint32_t P = kEncThreads * K, W = 32 * K;
+  const uint32_t l = threadIdx.x & 31, base = (threadIdx.x >> 5) * W;
+  int cur = 0;
+  for (uint32_t k = 2; k <= P; k <<= 1) {
+    for (uint32_t j = k >> 1; j > 0; j >>= 1) {
+      if (j >= W) {
+#pragma unroll
+        for (int r = 0; r < K; r++) buf[cur][base + 32 * r + l] = a[r];
+        __syncthreads();
+        const bool keep_min = ((base & j) == 0) == ((base & k) == 0);
+#pragma unroll
+        for (int r = 0; r < K; r++) {
+          uint32_t o = buf[cur][(base ^ j) + 32 * r + l];
+          a[r] = keep_min ? min(a[r], o) : max(a[r], o);
+        }
+        cur ^= 1;  // the next exchange writes the other buffer: one barrier each
+      } else if (j >= 32) {
+#pragma unroll
+        for (int d = 1; d < K; d <<= 1) {
+          if (j != 32u * d) continue;
+#pragma unroll
+          for (int r = 0; r < K; r++) {
+            if (r & d) continue;
+            const bool up = ((base + 32 * r) & k) == 0;
+            uint32_t x = a[r], y = a[r | d];
+            a[r] = up ? min(x, y) : max(x, y);
+            a[r | d] = up ? max(x, y) : min(x, y);
+          }
+        }
+      } else {
+#pragma unroll
+        for (int r = 0; r < K; r++) {
+          uint32_t o = __shfl_xor_sync(0xffffffffu, a[r], j);
+          const bool keep_min = ((l & j) == 0) == (((base + 32 * r + l) & k) == 0);
+          a[r] = keep_min ? min(a[r], o) : max(a[r], o);
+        }
+      }
+    }
+  }
+#pragma unroll
+  for (int r = 0; r < K; r++) buf[cur][base + 32 * r + l] = a[r];
+  __syncthreads();
+  return buf[cur];
+}
+
 // Returns the chosen left bit width, or 0 when ALP-RD does not apply.  The
 // sample is block[0], block[step], ... (step = max(n/2048, 1)); when `pre` is
-// given it holds those values at pre[i * pre_stride].
+// given it holds those values at pre[i * pre_stride].  A cut keeps at most 24
+// left bits, so the keys are the sample's top 24 bits; sorted, a cut's groups
+// are the runs between positions that share fewer leading bits with their
+// predecessor than the cut keeps.  One warp per cut gathers those positions as
+// 32-bit words, a lane's words together cover consecutive positions, and each
+// lane ranks the groups that end in its own.  S.rd_cand gets the largest
+// groups of the chosen cut.  (With 64-bit keys sorted through shared memory
+// and a vote per 32 positions it took 56 us of the 144 us that a 32,768-price
+// block's competition took.)
+template <int K>
+__device__ uint32_t* rd_sort_sample(EncSmem& S, const uint64_t* v, uint32_t sn, uint32_t step, const uint64_t* pre,
+                                    uint32_t pre_stride) {
+  uint32_t a[K];
+  const uint32_t base = (threadIdx.x >> 5) * 32 * K + (threadIdx.x & 31);
+#pragma unroll
+  for (int r = 0; r < K; r++) {
+    uint32_t i = base + 32 * r;
+    a[r] = i < sn ? (uint32_t)((pre ? pre[(uint64_t)i * pre_stride] : v[(uint64_t)i * step]) >> 40) : 0xFFFFFFFFu;
+  }
+  return block_sort_u32<K>(a, S.big.rd.smp);
+}
 __device__ uint32_t rd_choose_cut(EncSmem& S, const uint64_t* v, uint32_t n, const uint64_t* pre, uint32_t pre_stride) {
-  int lane = threadIdx.x & 31, warp = threadIdx.x >> 5;
+  const int lane = threadIdx.x & 31, warp = threadIdx.x >> 5;
   uint32_t step = max(n / 2048u, 1u);
-  uint32_t sn = (n + step - 1) / step;
-  uint32_t P = pow2_at_least(sn);
-  uint64_t* smp = S.big.rd.smp;
-  for (uint32_t i = threadIdx.x; i < P; i += blockDim.x)
-    smp[i] = i < sn ? (pre ? pre[(uint64_t)i * pre_stride] : v[(uint64_t)i * step]) : kEmpty64;
+  uint32_t sn = (n + step - 1) / step;  // at most 4095
+  static_assert(kEncThreads * 8 == 4096, "a sample of 4,095 values, eight a thread");
+  __syncthreads();  // the area is free
+  const uint32_t* key = sn <= kEncThreads * 4 ? rd_sort_sample<4>(S, v, sn, step, pre, pre_stride)
+                                              : rd_sort_sample<8>(S, v, sn, step, pre, pre_stride);
+  for (uint32_t i = threadIdx.x; i < sn; i += blockDim.x) {
+    uint32_t d = i ? key[i] ^ key[i - 1] : 0x800000u;
+    S.big.rd.cp[i] = (uint8_t)(d ? __clz(d) - 8 : 24);
+  }
   __syncthreads();
-  block_bitonic_sort(smp, P);
-  for (uint32_t lbw = warp + 1; lbw <= 24; lbw += blockDim.x / 32) {
+  const uint32_t rows = (sn + 31) / 32, q = (rows + 31) / 32;  // a lane takes q consecutive rows (at most 4)
+  for (uint32_t lbw = warp + 1; lbw <= 24; lbw += kEncWarps) {
     uint32_t rbw = 64 - lbw;
-    uint32_t t[8] = {0, 0, 0, 0, 0, 0, 0, 0};
-    uint32_t last_start = 0, G = 0;
-    for (uint32_t base = 0; base < sn; base += 32) {
-      uint32_t i = base + lane;
-      bool ok = i < sn;
-      bool bnd = ok && (i == 0 || (smp[i] >> rbw) != (smp[i - 1] >> rbw));
-      uint32_t m = __ballot_sync(0xffffffffu, bnd);
-      G += __popc(m);
-      if (bnd && i > 0) {
-        uint32_t below = m & ((1u << lane) - 1u);
-        uint32_t ps = below ? base + (31 - __clz(below)) : last_start;
-        top8_insert(t, i - ps);
+    uint32_t w[4] = {0, 0, 0, 0};
+    for (uint32_t o = 0; o * q < rows; o++) {
+#pragma unroll
+      for (uint32_t u = 0; u < 4; u++) {
+        uint32_t i = (o * q + u) * 32 + lane;
+        uint32_t m = u < q ? __ballot_sync(0xffffffffu, i < sn && S.big.rd.cp[i] < lbw) : 0u;
+        if ((uint32_t)lane == o) w[u] = m;
       }
-      if (m) last_start = base + (31 - __clz(m));
     }
-    if (lane == 0) top8_insert(t, sn - last_start);
-    uint64_t cov = 0;
+    uint32_t G = 0, last = 0;  // last: 1 + the lane's last group start
+#pragma unroll
+    for (uint32_t u = 0; u < 4; u++) {
+      G += __popc(w[u]);
+      if (w[u]) last = (lane * q + u) * 32 + 32 - __clz(w[u]);
+    }
+    G = __reduce_add_sync(0xffffffffu, G);
+    uint32_t before = last;  // the largest over the lanes up to this one, then those before it
+    for (int o = 1; o < 32; o <<= 1) {
+      uint32_t x = __shfl_up_sync(0xffffffffu, before, o);
+      if (lane >= o) before = max(before, x);
+    }
+    const uint32_t end = __shfl_sync(0xffffffffu, before, 31);
+    uint32_t start = __shfl_up_sync(0xffffffffu, before, 1);
+    if (lane == 0) start = 0;
+    uint32_t t[8] = {0, 0, 0, 0, 0, 0, 0, 0};  // size << 12 | first key, descending
+    // Groups of two and more, each at the start that follows it (a start whose
+    // predecessor is none): the many of one key that a deep cut leaves cost
+    // nothing, and only their number matters.
+    uint32_t tail = start && start == lane * q * 32 ? 1u : 0u;  // the position before the lane's words starts a group
+#pragma unroll
+    for (uint32_t u = 0; u < 4; u++) {
+      if (u >= q) break;
+      const uint32_t b0 = (lane * q + u) * 32;
+      uint32_t m = w[u] & ~(w[u] << 1 | tail);
+      tail = w[u] >> 31;
+      while (m) {
+        const uint32_t j = __ffs(m) - 1;
+        m &= m - 1;
+        const uint32_t prev = w[u] & ((1u << j) - 1u);
+        const uint32_t st = prev ? b0 + 32 - __clz(prev) : start;  // 1 + the group's first key
+        if (st) top8_insert(t, (b0 + j - (st - 1)) << 12 | (st - 1));
+      }
+      if (w[u]) start = b0 + 32 - __clz(w[u]);
+    }
+    if (lane == 0 && sn - (end - 1) >= 2) top8_insert(t, (sn - (end - 1)) << 12 | (end - 1));
+    uint32_t cov = 0, have = 0;
     for (int r = 0; r < 8; r++) {
-      uint32_t mx = warp_max(t[0]);
-      if (mx == 0) break;
-      uint32_t who = __ballot_sync(0xffffffffu, t[0] == mx);
-      if (lane == __ffs(who) - 1) {
+      uint32_t mx = __reduce_max_sync(0xffffffffu, t[0]);
+      if (lane == 0) S.rd_top[lbw - 1][r] = mx;
+      if (t[0] == mx && mx) {  // one lane: the packed groups differ
 #pragma unroll
         for (int i = 0; i < 7; i++) t[i] = t[i + 1];
         t[7] = 0;
       }
-      cov += mx;
+      cov += mx >> 12;
+      have += mx ? 1u : 0u;
     }
+    if (have < 8) cov += min(8u - have, G - have);  // groups of one key
     uint32_t dl = min(G, 8u);
     uint64_t num = (uint64_t)sn * (uint64_t)(rbw + rd_code_bits(dl)) + ((uint64_t)sn - cov) * 96ull;
     if (lane == 0) S.rd_pv[lbw - 1] = __ddiv_rn(__ull2double_rn(num), __ull2double_rn((uint64_t)sn));
   }
   __syncthreads();
-  uint32_t best = 0;
   if (threadIdx.x == 0) {
+    uint32_t best = 0;
     double bb = __longlong_as_double(0x7FF0000000000000ll);  // +inf
     for (uint32_t lbw = 1; lbw <= 24; lbw++) {
       if (S.rd_pv[lbw - 1] < bb) {
@@ -547,11 +734,200 @@ __device__ uint32_t rd_choose_cut(EncSmem& S, const uint64_t* v, uint32_t n, con
     }
     if (best == 0 || bb >= 63.0) best = 0;
     S.sc[0] = best;
+    uint32_t nc = 0;
+    for (; best && nc < 8 && S.rd_top[best - 1][nc]; nc++)
+      S.rd_cand[nc] = key[S.rd_top[best - 1][nc] & 4095u] >> (24 - best);
+    S.rd_ncand = nc;
   }
   __syncthreads();
-  best = (uint32_t)S.sc[0];
+  uint32_t best = (uint32_t)S.sc[0];
   __syncthreads();
   return best;
+}
+
+// One value's left part counted in a table of cap slots (a power of two):
+// false when it holds no free slot for it.  `fresh` counts the keys.
+__device__ __forceinline__ void rd_count(uint32_t* hk, uint32_t* hc, uint32_t cap, uint32_t lg, uint32_t key,
+                                         uint32_t add, uint32_t* fresh) {
+  uint32_t h = (uint32_t)(((uint64_t)key * 0x9E3779B97F4A7C15ull) >> (64 - lg));
+  for (uint32_t probe = 0; probe < cap; probe++) {
+    uint32_t cur = hk[h];
+    if (cur == kEmpty32) {
+      uint32_t old = atomicCAS(&hk[h], kEmpty32, key);
+      if (old == kEmpty32) {
+        if (fresh) atomicAdd(fresh, 1u);
+        cur = key;
+      } else {
+        cur = old;
+      }
+    }
+    if (cur == key) {
+      atomicAdd(&hc[h], add);
+      return;
+    }
+    h = (h + 1) & (cap - 1);
+  }
+}
+
+// The block's eight most frequent left parts and everything that the payload
+// needs to know of them: the chosen cut's largest sample groups (S.rd_cand)
+// are counted by comparison; the other left parts (a few in a hundred where
+// ALP-RD is any good) are listed in shared memory and counted in a table
+// afterwards.  If none of those is as frequent as the rarest candidate, the
+// candidates are the dictionary; otherwise the table names the right ones and
+// the pass runs once more with them.  On true S.dict8 holds the dictionary by
+// (count desc, key asc) (alp_rd.rs:47-68), and per sub-block S.w_a the codes'
+// width and S.w_c their smallest code, S.rd_ne the exceptions and S.rd_eb
+// their bytes.  False (more keys than the shared table holds): the general
+// pass decides (rd_top8).  (A vote for equal left parts and an
+// atomic per 32 values, eight searches of the table and a second pass took
+// 75 us for 32,768 values.)
+constexpr uint32_t kRdList = 2 * 4096 / kEncWarps;  // listed left parts a warp (over the sample's sort buffers)
+__device__ bool rd_dict_pass(EncSmem& S, const uint64_t* v, uint32_t n, uint32_t lbw) {
+  const int lane = threadIdx.x & 31, warp = threadIdx.x >> 5;
+  const uint32_t rbw = 64 - lbw, nsub = (n + kSub - 1) / kSub, below = (1u << lane) - 1u;
+  uint32_t* hk = S.big.rd.hkey;
+  uint32_t* hc = S.big.rd.hcnt;
+  uint32_t* list = &S.big.rd.smp[0][0] + warp * kRdList;
+  bool full = false;  // the table has no room for more keys
+  auto count_list = [&](uint32_t m) {
+    __syncwarp();
+    for (uint32_t i = lane; i < m && !full; i += 32) {
+      full = *(volatile uint32_t*)&S.card >= kHashLimit;
+      if (!full) rd_count(hk, hc, kHashCap, 11, list[i], 1, &S.card);
+    }
+    __syncwarp();
+  };
+  for (int round = 0;; round++) {
+    const uint32_t nc = S.rd_ncand;
+    for (uint32_t i = threadIdx.x; i < kHashCap; i += blockDim.x) {
+      hk[i] = kEmpty32;
+      hc[i] = 0;
+    }
+    if (threadIdx.x < 8) S.rd_cnt[threadIdx.x] = 0;
+    if (threadIdx.x == 0) S.card = 0;  // keys in the table
+    uint32_t listed = 0;
+    uint32_t cand[8], cnt[8];
+#pragma unroll
+    for (int j = 0; j < 8; j++) {
+      cand[j] = (uint32_t)j < nc ? S.rd_cand[j] : kEmpty32;  // left parts are below 2^24
+      cnt[j] = 0;
+    }
+    __syncthreads();
+    for (uint32_t k = warp; k < nsub; k += kEncWarps) {
+      const uint32_t base = k * kSub, m = min((uint32_t)kSub, n - base);
+      uint32_t seen = 0, ne = 0, eb = 0;
+      for (uint32_t i0 = 0; i0 < m; i0 += 32 * 8) {
+        uint64_t xs[8];
+#pragma unroll
+        for (int u = 0; u < 8; u++) xs[u] = i0 + 32 * u + lane < m ? v[base + i0 + 32 * u + lane] : 0ull;
+#pragma unroll
+        for (int u = 0; u < 8; u++) {
+          const uint32_t i = i0 + 32 * u + lane;
+          const bool in = i < m;
+          const uint32_t left = in ? (uint32_t)(xs[u] >> rbw) : 0xFFFFFFFEu;
+          uint32_t hit = 0;
+#pragma unroll
+          for (int j = 0; j < 8; j++)
+            if (left == cand[j]) {
+              cnt[j]++;
+              hit = 1u << j;
+            }
+          seen |= hit;
+          const bool other = in && !hit;
+          const uint32_t om = __ballot_sync(0xffffffffu, other);
+          if (!om) continue;
+          if (other) {
+            list[listed + __popc(om & below)] = left;
+            ne++;
+            eb += 9 + (base + i >= (1u << 7) ? 1u : 0u) + (base + i >= (1u << 14) ? 1u : 0u);  // i < 2^17
+          }
+          listed += __popc(om);
+          if (listed > kRdList - 32) {
+            count_list(listed);
+            listed = 0;
+          }
+        }
+      }
+      seen = __reduce_or_sync(0xffffffffu, seen);
+      ne = __reduce_add_sync(0xffffffffu, ne);
+      eb = __reduce_add_sync(0xffffffffu, eb);
+      if (lane == 0) {
+        S.rd_mask[k] = (uint8_t)seen;
+        S.rd_ne[k] = ne;
+        S.rd_eb[k] = eb;
+      }
+    }
+#pragma unroll
+    for (int j = 0; j < 8; j++) {
+      uint32_t c = __reduce_add_sync(0xffffffffu, cnt[j]);
+      if (lane == 0 && c) atomicAdd(&S.rd_cnt[j], c);
+    }
+    count_list(listed);
+    if (__syncthreads_or(full)) return false;
+    // is another left part at least as frequent as the rarest candidate?
+    uint32_t rarest = nc == 8 ? 0xFFFFFFFFu : 0u;
+    for (uint32_t j = 0; j < nc && nc == 8; j++) rarest = min(rarest, S.rd_cnt[j]);
+    uint32_t other = 0;
+    for (uint32_t i = threadIdx.x; i < kHashCap; i += blockDim.x) other = max(other, hc[i]);
+    if (!__syncthreads_or(other && other >= rarest)) break;
+    if (round) return false;  // not reached: the exact eight were counted
+    // the exact eight among the candidates and the table's keys
+    if (threadIdx.x < nc) rd_count(hk, hc, kHashCap, 11, S.rd_cand[threadIdx.x], S.rd_cnt[threadIdx.x], nullptr);
+    __syncthreads();
+    uint64_t top[4];  // the thread's four slots: (count, key) packed, larger first in the dictionary
+#pragma unroll
+    for (int u = 0; u < 4; u++) {
+      uint32_t i = threadIdx.x + kEncThreads * u;
+      top[u] = hc[i] ? (uint64_t)hc[i] << 32 | (0xFFFFFFFFu - hk[i]) : 0ull;
+    }
+    static_assert(kHashCap == 4 * kEncThreads, "four table slots a thread");
+    uint32_t found = 0;
+    for (int r = 0; r < 8; r++) {
+      uint64_t mx = top[0];
+#pragma unroll
+      for (int u = 1; u < 4; u++) mx = u64max(mx, top[u]);
+      mx = warp_max(mx);
+      if (lane == 0) S.red[warp] = mx;
+      __syncthreads();
+      mx = 0;
+      for (int w = 0; w < kEncWarps; w++) mx = u64max(mx, S.red[w]);
+      __syncthreads();
+      if (!mx) break;
+#pragma unroll
+      for (int u = 0; u < 4; u++)
+        if (top[u] == mx) top[u] = 0;
+      if (threadIdx.x == 0) S.rd_cand[r] = 0xFFFFFFFFu - (uint32_t)mx;
+      found++;
+    }
+    if (threadIdx.x == 0) S.rd_ncand = found;
+    __syncthreads();
+  }
+  const uint32_t nc = S.rd_ncand;
+  if (threadIdx.x < nc) {  // ranks by (count desc, key asc)
+    const uint32_t j = threadIdx.x;
+    const uint64_t mine = (uint64_t)S.rd_cnt[j] << 32 | (0xFFFFFFFFu - S.rd_cand[j]);
+    uint32_t rank = 0;
+    for (uint32_t i = 0; i < nc; i++)
+      rank += ((uint64_t)S.rd_cnt[i] << 32 | (0xFFFFFFFFu - S.rd_cand[i])) > mine ? 1u : 0u;
+    S.dict8[rank] = S.rd_cand[j];
+    S.red32[j] = rank;
+  }
+  if (threadIdx.x == 0) S.dl = nc;
+  __syncthreads();
+  for (uint32_t k = threadIdx.x; k < nsub; k += blockDim.x) {
+    uint32_t lo = 8, hi = 0;
+    for (uint32_t j = 0; j < nc; j++)
+      if (S.rd_mask[k] >> j & 1u) {
+        lo = min(lo, S.red32[j]);
+        hi = max(hi, S.red32[j]);
+      }
+    if (S.rd_ne[k]) lo = 0;  // an exception's code is 0
+    S.w_a[k] = (uint8_t)bit_width64((uint64_t)(hi - min(lo, hi)));
+    S.w_c[k] = (uint8_t)min(lo, hi);
+  }
+  __syncthreads();
+  return true;
 }
 
 // Full-block top-8 left parts by (count desc, key asc) (reference
@@ -845,7 +1221,10 @@ __device__ __forceinline__ void dict_insert(DictArea& D, EncSmem& S, uint64_t x)
 
 // lb_pre: the block's 17-bit bucket count when the statistics pass computed it
 // (block == one adaptive window), else kNoLb.
-__device__ DictView dict_prepare(EncSmem& S, const uint64_t* v, uint32_t n, uint8_t* scratch, uint32_t lb_pre) {
+// runs / starts (optional): the block's run starts, whose values are all its
+// distinct ones (in a block of geometric runs of 16 an eighth of the work).
+__device__ DictView dict_prepare(EncSmem& S, const uint64_t* v, uint32_t n, uint8_t* scratch, uint32_t lb_pre,
+                                 const uint32_t* starts = nullptr, uint32_t runs = 0) {
   DictArea& D = S.big.dict;
   uint32_t max_card = n / 2 + 1;
   bool have_lb = lb_pre != kNoLb;
@@ -871,18 +1250,26 @@ __device__ DictView dict_prepare(EncSmem& S, const uint64_t* v, uint32_t n, uint
   __syncthreads();
   // the shared-memory hash until it holds kHashLimit keys; the lower-bound
   // bitset is only built (below) for a block that overflows it
-  for (uint32_t base = 0; base < n; base += blockDim.x * 8) {
-    if (*(volatile uint32_t*)&S.ovf) break;
-    uint64_t xs[8];
+  auto insert_all = [&](uint32_t nv, auto at) {
+    for (uint32_t base = 0; base < nv; base += blockDim.x * 8) {
+      if (*(volatile uint32_t*)&S.ovf) break;
+      uint64_t xs[8];
 #pragma unroll
-    for (int q = 0; q < 8; q++) {
-      uint32_t iq = base + q * blockDim.x + threadIdx.x;
-      xs[q] = iq < n ? v[iq] : 0ull;
+      for (int q = 0; q < 8; q++) {
+        uint32_t iq = base + q * blockDim.x + threadIdx.x;
+        xs[q] = iq < nv ? at(iq) : 0ull;
+      }
+      // the first probes of the eight values together: mostly the key is there
+      uint64_t cur[8];
+#pragma unroll
+      for (int q = 0; q < 8; q++) cur[q] = D.hkey[(uint32_t)((xs[q] * 0x9E3779B97F4A7C15ull) >> 53)];
+#pragma unroll
+      for (int q = 0; q < 8; q++)
+        if (base + q * blockDim.x + threadIdx.x < nv && (cur[q] != xs[q] || xs[q] == kEmpty64)) dict_insert(D, S, xs[q]);
     }
-#pragma unroll
-    for (int q = 0; q < 8; q++)
-      if (base + q * blockDim.x + threadIdx.x < n) dict_insert(D, S, xs[q]);
-  }
+  };
+  if (starts) insert_all(runs, [&](uint32_t i) { return v[starts[i]]; });
+  else insert_all(n, [&](uint32_t i) { return v[i]; });
   __syncthreads();
   DictView dv;
   if (!S.ovf) {
@@ -1115,48 +1502,45 @@ __device__ uint64_t dict_values_len(EncSmem& S, const DictView& dv, uint32_t* ta
 
 // ---------------------------------------------------------------------------
 // RLE run starts (reference rle.rs:10-42).  Requires S.neq_k (transitions per
-// sub-block).  Returns the starts array (smem or scratch).
+// sub-block).  Returns the starts, in the first 16 bytes per value of the
+// block's scratch.
 // ---------------------------------------------------------------------------
-__device__ uint32_t* rle_starts(EncSmem& S, const uint64_t* v, uint32_t n, uint32_t runs, uint8_t* scratch) {
+__device__ uint32_t* rle_starts(EncSmem& S, const uint64_t* v, uint32_t n, uint8_t* scratch) {
   int lane = threadIdx.x & 31, warp = threadIdx.x >> 5;
-  uint32_t* st = runs <= kRunsSmem ? S.big.rle.starts : reinterpret_cast<uint32_t*>(scratch);
+  uint32_t* st = reinterpret_cast<uint32_t*>(scratch);
   uint32_t nsub = (n + kSub - 1) / kSub;
-  if (threadIdx.x == 0) {  // exclusive prefix of transitions per sub-block
-    uint32_t acc = 0;
-    for (uint32_t k = 0; k < nsub; k++) {
-      uint32_t c = S.neq_k[k];
-      S.subsz[k] = acc;
-      acc += c;
+  for (uint32_t k = threadIdx.x; k < nsub; k += blockDim.x) S.subsz[k] = S.neq_k[k];
+  if (threadIdx.x == 0) st[0] = 0;
+  block_offsets(S, nsub, 1);
+  // eight rows in flight while the eight before them are compared
+  uint64_t xs[8], nx[8];
+  auto load = [&](uint32_t k, uint32_t j0, uint64_t (&x)[8]) {
+#pragma unroll
+    for (int q = 0; q < 8; q++) {
+      uint32_t i = k * kSub + (j0 + q) * 32 + lane;
+      x[q] = k < nsub && i < n ? v[i] : 0ull;
     }
-    st[0] = 0;
-  }
-  __syncthreads();
+  };
+  load(warp, 0, nx);
   for (uint32_t k = warp; k < nsub; k += kEncWarps) {
-    uint32_t base = k * kSub, cnt = min((uint32_t)kSub, n - base);
+    uint32_t base = k * kSub, before = S.subsz[k];
     uint64_t carry = base ? v[base - 1] : v[0];
-    uint32_t before = S.subsz[k];
     for (uint32_t j0 = 0; j0 < 32; j0 += 8) {
-     uint64_t xs[8];
 #pragma unroll
-     for (int q = 0; q < 8; q++) {
-       uint32_t lq = (j0 + q) * 32 + lane;
-       xs[q] = lq < cnt ? v[base + lq] : 0ull;
-     }
+      for (int q = 0; q < 8; q++) xs[q] = nx[q];
+      if (j0 < 24) load(k, j0 + 8, nx);
+      else load(k + kEncWarps, 0, nx);
 #pragma unroll
-     for (int q = 0; q < 8; q++) {
-      uint32_t j = j0 + q;
-      uint32_t li = j * 32 + lane;
-      bool ok = li < cnt;
-      uint32_t idx = base + li;
-      uint64_t x = xs[q];
-      uint64_t up = __shfl_up_sync(0xffffffffu, x, 1);
-      uint64_t pv = lane ? up : carry;
-      carry = __shfl_sync(0xffffffffu, x, 31);
-      bool tr = ok && idx && x != pv;
-      uint32_t m = __ballot_sync(0xffffffffu, tr);
-      if (tr) st[1 + before + __popc(m & ((1u << lane) - 1u))] = idx;
-      before += __popc(m);
-     }
+      for (int q = 0; q < 8; q++) {
+        uint32_t idx = base + (j0 + q) * 32 + lane;
+        uint64_t x = xs[q];
+        uint64_t rot = __shfl_sync(0xffffffffu, x, (lane + 31) & 31);
+        bool tr = idx < n && x != (lane ? rot : carry);  // the block's first value equals its carry
+        carry = rot;
+        uint32_t m = __ballot_sync(0xffffffffu, tr);
+        if (tr) st[before + __popc(m & ((1u << lane) - 1u))] = idx;
+        before += __popc(m);
+      }
     }
   }
   __syncthreads();
@@ -1976,13 +2360,14 @@ __device__ __noinline__ int sample_winner(EncSmem& S, const uint64_t* v, uint32_
 // FLOAT_MULT, ALP-RD and DICT and the BYTE_TRANSPOSE candidate; the chosen
 // coded parts go to ent[b] for the emission.
 template <bool ENT, bool SAMPLE>
-__global__ void __launch_bounds__(kEncThreads) k_decide(const uint64_t* __restrict__ lane, FrameDesc* frames,
+__global__ void __launch_bounds__(kEncThreads, 2) k_decide(const uint64_t* __restrict__ lane, FrameDesc* frames,
                                                         const uint32_t* __restrict__ nbp, uint64_t fixed_bs,
                                                         int dtype, int level, const SubStats* __restrict__ ss,
                                                         const FmStat* __restrict__ fms,
                                                         const uint64_t* __restrict__ smp16,
                                                         const uint32_t* __restrict__ winbits,
-                                                        uint8_t* __restrict__ scratch, EntRec* __restrict__ ent) {
+                                                        uint8_t* __restrict__ scratch, EntRec* __restrict__ ent,
+                                                        RdRec* __restrict__ rdr, BlkRec* __restrict__ blk) {
   extern __shared__ __align__(16) uint8_t smem_raw[];
   EncSmem& S = *reinterpret_cast<EncSmem*>(smem_raw);
   uint32_t b = blockIdx.x;
@@ -2022,47 +2407,76 @@ __global__ void __launch_bounds__(kEncThreads) k_decide(const uint64_t* __restri
   }
   __syncthreads();
   uint64_t D = n >= 2 ? v[1] - v[0] : 0;
-  uint64_t my_for = 0, my_delta = 0, my_alp = 0;
-  for (uint32_t k = t; k < nsub; k += blockDim.x) {
-    SubStats R = ss[g0 + k];
-    uint64_t pl = k ? ss[g0 + k - 1].last : 0;
-    uint32_t wf = sgn ? bit_width64((uint64_t)R.smax - (uint64_t)R.smin) : bit_width64(R.umax - R.umin);
-    uint64_t dzf = k ? zigzag64(R.first - pl) : 0;
-    uint64_t dmn = R.cnt > 1 ? u64min(R.dzmin, dzf) : dzf, dmx = R.cnt > 1 ? u64max(R.dzmax, dzf) : dzf;
-    my_for += 9 + 128ull * wf;
-    my_delta += 9 + 128ull * bit_width64(dmx - dmn);
-    uint32_t nq = R.neq + ((k && R.first != pl) ? 1u : 0u);
-    S.neq_k[k] = nq;
-    S.item_min[k] = R.umin;
-    S.item_max[k] = R.umax;
-    atomicAdd(&S.neq, nq);
-    atomicAdd(&S.xor_bytes, (unsigned long long)(R.xb + varint_len(R.first ^ pl)));
-    atomic_min_u64(&S.umin, R.umin);
-    atomic_max_u64(&S.umax, R.umax);
-    bool sok = R.stride_ok && (R.cnt < 2 || R.d == D) && (k == 0 || R.first - pl == D);
-    if (!sok) atomicOr(&S.stride_bad, 1u);
-    if (pre_e) {
-      uint64_t emn = step == 16 ? R.e16min : R.e64min, emx = step == 16 ? R.e16max : R.e64max;
-      uint64_t edz = step == 16 ? R.e16dz : R.e64dz;
+  // One sub-block per thread (at most 128); the lanes' results are reduced by
+  // shuffles, so that a warp updates each shared quantity once (with an atomic
+  // per sub-block, whose 64-bit minima are compare-and-swap loops, this took
+  // 9 us of a 32,768-value block's 13).
+  if (warp * 32 < (int)nsub) {
+    const uint32_t k = t;
+    const bool in = k < nsub;
+    SubStats R;
+    uint64_t pl = 0, fsz = 0, dsz = 0, asz = 0, xbytes = 0;
+    uint64_t emn = kEmpty64, emx = 0, edz = 0, umn = kEmpty64, umx = 0;
+    uint32_t nq = 0, pass = 0x7F;
+    bool sbad = false, abad = false;
+    if (in) {
+      R = ss[g0 + k];
+      if (k) pl = ss[g0 + k - 1].last;
+      uint32_t wf = sgn ? bit_width64((uint64_t)R.smax - (uint64_t)R.smin) : bit_width64(R.umax - R.umin);
+      uint64_t dzf = k ? zigzag64(R.first - pl) : 0;
+      uint64_t dmn = R.cnt > 1 ? u64min(R.dzmin, dzf) : dzf, dmx = R.cnt > 1 ? u64max(R.dzmax, dzf) : dzf;
+      fsz = 9 + 128ull * wf;
+      dsz = 9 + 128ull * bit_width64(dmx - dmn);
+      nq = R.neq + ((k && R.first != pl) ? 1u : 0u);
+      S.neq_k[k] = nq;
+      umn = S.item_min[k] = R.umin;
+      umx = S.item_max[k] = R.umax;
+      xbytes = R.xb + varint_len(R.first ^ pl);
+      sbad = !(R.stride_ok && (R.cnt < 2 || R.d == D) && (k == 0 || R.first - pl == D));
+      emn = step == 16 ? R.e16min : R.e64min;
+      emx = step == 16 ? R.e16max : R.e64max;
+      edz = step == 16 ? R.e16dz : R.e64dz;
       if (k) edz = u64max(edz, dzf);
-      atomic_min_u64(&S.e_vmin, emn);
-      atomic_max_u64(&S.e_vmax, emx);
-      atomic_max_u64(&S.e_dmax, edz);
+      pass = R.fm_pass;
+      abad = !R.alp_ok;
+      asz = 13 + 128ull * R.alp_w + 10ull * R.alp_exc;
+    }
+    // the sizes fit 32 bits (a sub-block's parts stay below 20 KB)
+    const uint32_t sfor = __reduce_add_sync(0xffffffffu, (uint32_t)fsz), sdel = __reduce_add_sync(0xffffffffu, (uint32_t)dsz);
+    const uint32_t sxor = __reduce_add_sync(0xffffffffu, (uint32_t)xbytes), sneq = __reduce_add_sync(0xffffffffu, nq);
+    umn = warp_min(umn);
+    umx = warp_max(umx);
+    const bool any_s = __any_sync(0xffffffffu, sbad);
+    if (lane_id == 0) {
+      atomicAdd((unsigned long long*)&S.sc[1], (unsigned long long)sfor);
+      atomicAdd((unsigned long long*)&S.sc[2], (unsigned long long)sdel);
+      atomicAdd(&S.xor_bytes, (unsigned long long)sxor);
+      atomicAdd(&S.neq, sneq);
+      atomic_min_u64(&S.umin, umn);
+      atomic_max_u64(&S.umax, umx);
+      if (any_s) atomicOr(&S.stride_bad, 1u);
+    }
+    if (pre_e && !fam_float) {  // only the integer early-out reads them
+      emn = warp_min(emn);
+      emx = warp_max(emx);
+      edz = warp_max(edz);
+      if (lane_id == 0) {
+        atomic_min_u64(&S.e_vmin, emn);
+        atomic_max_u64(&S.e_vmax, emx);
+        atomic_max_u64(&S.e_dmax, edz);
+      }
     }
     if (fam_float && !reduced) {
-      atomicAnd(&S.fm_mask, (uint32_t)R.fm_pass);
-      if (!R.alp_ok) atomicOr(&S.alp_fail, 1u);
-      my_alp += 13 + 128ull * R.alp_w + 10ull * R.alp_exc;
+      const uint32_t salp = __reduce_add_sync(0xffffffffu, (uint32_t)asz), am = __reduce_and_sync(0xffffffffu, pass);
+      const bool any_a = __any_sync(0xffffffffu, abad);
+      if (lane_id == 0) {
+        atomicAdd((unsigned long long*)&S.sc[4], (unsigned long long)salp);
+        atomicAnd(&S.fm_mask, am);
+        if (any_a) atomicOr(&S.alp_fail, 1u);
+      }
     }
   }
-  my_for = warp_sum(my_for);
-  my_delta = warp_sum(my_delta);
-  my_alp = warp_sum(my_alp);
-  if (lane_id == 0) {
-    atomicAdd((unsigned long long*)&S.sc[1], (unsigned long long)my_for);
-    atomicAdd((unsigned long long*)&S.sc[2], (unsigned long long)my_delta);
-    atomicAdd((unsigned long long*)&S.sc[4], (unsigned long long)my_alp);
-  }
+  static_assert(kSubsMax <= kEncThreads, "one sub-block per thread");
   __syncthreads();
   uint64_t vl = varint_len(n);
   uint64_t sz_for = vl + S.sc[1], sz_delta = 8 + vl + S.sc[2], sz_alp = vl + S.sc[4];
@@ -2187,32 +2601,34 @@ __global__ void __launch_bounds__(kEncThreads) k_decide(const uint64_t* __restri
     rd_lbw = (SAMPLE && win != M_ALP_RD) ? 0u
                                          : rd_choose_cut(S, v, n, pre_s ? smp16 + fd.value_off / 16 : nullptr,
                                                          step / 16);
-    if (rd_lbw && !SAMPLE && !ENT) {
-      // The rights' FoR size is exact from one cheap pass (each sub-block's
-      // range of x & rmask); with the smallest possible rest of the payload
-      // (a 2-byte header, varint(nexc), the tags and lengths, one 9-byte
-      // header per code sub-block) and ALP-RD's decode penalty, it may
-      // already reach the best score of the candidates sized so far, and
-      // ALP-RD cannot win (strict <): its dictionary and exception passes are
-      // skipped.
-      uint32_t rbw = 64 - rd_lbw;
-      uint64_t rmask = (1ull << rbw) - 1ull;
+    uint64_t rlen = vl;
+    if (rd_lbw) {  // the rights' FoR layout: each sub-block's range of x & rmask
+      uint64_t rmask = (1ull << (64 - rd_lbw)) - 1ull;
       if (t == 0) S.acc64 = 0;
       __syncthreads();
       for (uint32_t k = warp; k < nsub; k += kEncWarps) {
         uint32_t base = k * kSub, cnt = min((uint32_t)kSub, n - base);
-        uint64_t rmn = kEmpty64, rmx = 0;
-        for (uint32_t i = lane_id; i < cnt; i += 32) {
-          uint64_t r = v[base + i] & rmask;
-          rmn = u64min(rmn, r);
-          rmx = u64max(rmx, r);
+        uint64_t mn;
+        uint32_t w;
+        warp_minmax(cnt, false, [&](uint32_t i) { return v[base + i] & rmask; }, &mn, &w);
+        if (lane_id == 0) {
+          S.w_b[k] = (uint8_t)w;
+          S.submin[k] = mn;
+          atomicAdd(&S.acc64, (unsigned long long)(9 + 128ull * w));
         }
-        rmn = warp_min(rmn);
-        rmx = warp_max(rmx);
-        if (lane_id == 0) atomicAdd(&S.acc64, (unsigned long long)(9 + 128ull * bit_width64(rmx - rmn)));
       }
       __syncthreads();
-      uint64_t floor_len = 6 + 2 * vl + 9ull * nsub + S.acc64;
+      rlen += S.acc64;
+      __syncthreads();
+    }
+    if (rd_lbw && !SAMPLE && !ENT) {
+      // With the rights' exact size and the smallest possible rest of the
+      // payload (a 2-byte header, varint(nexc), the tags and lengths, one
+      // 9-byte header per code sub-block) and ALP-RD's decode penalty, it may
+      // already reach the best score of the candidates sized so far, and
+      // ALP-RD cannot win (strict <): its dictionary and exception pass is
+      // skipped.
+      uint64_t floor_len = 6 + vl + 9ull * nsub + rlen;
       uint64_t best = decoded_bytes + ((lambda * decode_weight(M_RAW) * decoded_bytes) >> 8);
       auto sc_of = [&](int m, uint64_t len) { return len + ((lambda * decode_weight(m) * decoded_bytes) >> 8); };
       if (S.umin == S.umax) best = u64min(best, sc_of(M_CONST, 8));
@@ -2226,50 +2642,61 @@ __global__ void __launch_bounds__(kEncThreads) k_decide(const uint64_t* __restri
       __syncthreads();
     }
     if (rd_lbw) {
-      rd_top8(S, v, n, rd_lbw, scr);
       uint32_t rbw = 64 - rd_lbw;
       uint64_t rmask = (1ull << rbw) - 1ull;
+      if (!rd_dict_pass(S, v, n, rd_lbw)) {
+        __syncthreads();
+        rd_top8(S, v, n, rd_lbw, scr);
+        for (uint32_t k = warp; k < nsub; k += kEncWarps) {
+          uint32_t base = k * kSub, cnt = min((uint32_t)kSub, n - base);
+          uint32_t cmx = 0, cmn = 8, eb = 0, ne = 0;
+          for (uint32_t i = lane_id; i < cnt; i += 32) {
+            int c = rd_code(S, v[base + i] >> rbw);
+            uint32_t code = c < 0 ? 0u : (uint32_t)c;
+            if (c < 0) {
+              ne++;
+              eb += varint_len(base + i) + 8;
+            }
+            cmn = min(cmn, code);
+            cmx = max(cmx, code);
+          }
+          cmn = __reduce_min_sync(0xffffffffu, cmn);
+          cmx = __reduce_max_sync(0xffffffffu, cmx);
+          ne = __reduce_add_sync(0xffffffffu, ne);
+          eb = __reduce_add_sync(0xffffffffu, eb);
+          if (lane_id == 0) {
+            S.w_a[k] = (uint8_t)bit_width64((uint64_t)(cmx - cmn));
+            S.w_c[k] = (uint8_t)cmn;
+            S.rd_ne[k] = ne;
+            S.rd_eb[k] = eb;
+          }
+        }
+        __syncthreads();
+      }
+      // sums, and the layout for the emission
       if (t == 0) {
         S.acc64 = 0;
         S.cnt32 = 0;
+        S.sc[5] = 0;
       }
       __syncthreads();
-      for (uint32_t k = warp; k < nsub; k += kEncWarps) {
-        uint32_t base = k * kSub, cnt = min((uint32_t)kSub, n - base);
-        uint64_t cmx = 0, rmn = kEmpty64, rmx = 0, cmn = kEmpty64, eb = 0;
-        uint32_t ne = 0;
-        for (uint32_t i = lane_id; i < cnt; i += 32) {
-          uint64_t x = v[base + i];
-          int c = rd_code(S, x >> rbw);
-          uint64_t code = c < 0 ? 0 : (uint64_t)c;
-          if (c < 0) {
-            ne++;
-            eb += varint_len(base + i) + 8;
-          }
-          cmn = u64min(cmn, code);
-          cmx = u64max(cmx, code);
-          rmn = u64min(rmn, x & rmask);
-          rmx = u64max(rmx, x & rmask);
-        }
-        cmn = warp_min(cmn);
-        cmx = warp_max(cmx);
-        rmn = warp_min(rmn);
-        rmx = warp_max(rmx);
-        ne = warp_sum(ne);
-        eb = warp_sum(eb);
-        if (lane_id == 0) {
-          S.w_a[k] = (uint8_t)bit_width64(cmx - cmn);
-          S.w_b[k] = (uint8_t)bit_width64(rmx - rmn);
-          atomicAdd(&S.cnt32, ne);
-          atomicAdd(&S.acc64, (unsigned long long)eb);
-        }
+      for (uint32_t k = t; k < nsub; k += blockDim.x) {
+        atomicAdd(&S.cnt32, S.rd_ne[k]);
+        atomicAdd(&S.acc64, (unsigned long long)S.rd_eb[k]);
+        atomicAdd((unsigned long long*)&S.sc[5], (unsigned long long)(9 + 128ull * S.w_a[k]));
+        RdRec r;
+        r.rmin = S.submin[k];
+        r.eb = S.rd_eb[k];
+        r.ne = (uint16_t)S.rd_ne[k];
+        r.cw = S.w_a[k];
+        r.rw = S.w_b[k];
+        r.cmin = S.w_c[k];
+        rdr[g0 + k] = r;
       }
+      if (t < 8) blk[b].dict8[t] = S.dict8[t];
+      if (t == 8) blk[b].dl = S.dl;
       __syncthreads();
-      uint64_t nexc = S.cnt32, excb = S.acc64, clen = vl, rlen = vl;
-      for (uint32_t k = 0; k < nsub; k++) {
-        clen += 9 + 128ull * S.w_a[k];
-        rlen += 9 + 128ull * S.w_b[k];
-      }
+      uint64_t nexc = S.cnt32, excb = S.acc64, clen = vl + S.sc[5];
       c_rd.ok = nexc * 4 <= n;
       auto code_at = [&](uint32_t i) {
         int c = rd_code(S, v[i] >> rbw);
@@ -2392,8 +2819,18 @@ __global__ void __launch_bounds__(kEncThreads) k_decide(const uint64_t* __restri
     // that and DICT's decode penalty already reach the best score, it cannot
     // win (strict <) and its passes are skipped.
     if (!SAMPLE && best_score <= 22 + ((lambda * decode_weight(M_DICT) * decoded_bytes) >> 8)) want_dict = false;
+    // RLE's floor: the run values, two varint(runs) and a 9-byte header per
+    // 1,024 run lengths
+    const uint32_t neq = S.neq, runs = neq + 1;
+    const uint64_t rle_floor = 2 * varint_len(runs) + 8ull * runs + 9ull * ((runs + kSub - 1) / kSub) +
+                               ((lambda * decode_weight(M_RLE) * decoded_bytes) >> 8);
+    const bool want_rle = (!SAMPLE || win == M_RLE) && neq <= n / 2 + 1 && (SAMPLE || best_score > rle_floor);
+    uint32_t* st = want_rle ? rle_starts(S, v, n, scr) : nullptr;
     DictView dv;
-    if (want_dict) dv = dict_prepare(S, v, n, scr, lb_pre);
+    if (want_dict) {
+      dv = dict_prepare(S, v, n, scr, lb_pre, st, runs);
+      if (!dv.smem) st = nullptr;  // a large dictionary is built over the run starts
+    }
     if (want_dict && !S.flag) {
       uint32_t vtag;
       uint64_t vlen = dict_values_len(S, dv, &vtag);
@@ -2439,21 +2876,35 @@ __global__ void __launch_bounds__(kEncThreads) k_decide(const uint64_t* __restri
         }
       }
       consider(M_DICT, varint_len(dv.card) + 1 + varint_len(vlen) + vlen + 1 + clen);
+      // a small dictionary is kept for the emission, in the half of the block's
+      // scratch that the run starts below do not use
+      if (dv.smem && best_mode == M_DICT) {
+        uint64_t* keep = reinterpret_cast<uint64_t*>(scr + 16ull * n);
+        for (uint32_t i = t; i < dv.card; i += blockDim.x) keep[i] = dv.sorted[i];
+        if (t == 0) {
+          blk[b].card = dv.card;
+          blk[b].vtag = vtag;
+          blk[b].vlen = vlen;
+        }
+      } else if (t == 0) {
+        blk[b].card = 0;
+      }
     }
     __syncthreads();
     // RLE (rle.rs:10-42)
-    uint32_t neq = S.neq;
-    // likewise RLE's floor: the run values and two varint(runs) plus a 9-byte
-    // header per 1,024 run lengths
-    const uint64_t rle_floor = 2 * varint_len(neq + 1) + 8ull * (neq + 1) + 9ull * ((neq + 1 + kSub - 1) / kSub) +
-                               ((lambda * decode_weight(M_RLE) * decoded_bytes) >> 8);
-    if ((!SAMPLE || win == M_RLE) && neq <= n / 2 + 1 && (SAMPLE || best_score > rle_floor)) {
-      uint32_t runs = neq + 1;
-      uint32_t* st = rle_starts(S, v, n, runs, scr);
+    if (want_rle && (SAMPLE || best_score > rle_floor)) {
+      if (!st) st = rle_starts(S, v, n, scr);
       uint64_t lens = block_for(S, nullptr, runs, false, [&](uint32_t r) {
         return (uint64_t)((r + 1 < runs ? st[r + 1] : n) - st[r]);
       });
       consider(M_RLE, varint_len(runs) + 8ull * runs + lens);
+      if (best_mode == M_RLE) {  // for the emission: the starts stay in the block's scratch
+        if (t == 0) blk[b].card = runs;
+        for (uint32_t k = t; k < (runs + kSub - 1) / kSub; k += blockDim.x) {
+          rdr[g0 + k].rmin = S.submin[k];
+          rdr[g0 + k].rw = S.w_a[k];
+        }
+      }
     }
   }
   if (t == 0) {
@@ -2466,12 +2917,20 @@ __global__ void __launch_bounds__(kEncThreads) k_decide(const uint64_t* __restri
 }
 
 // ---------------------------------------------------------------------------
-// Emission kernel: writes the frame header and the winner's payload.
+// Emission kernel: writes the frame header and the winner's payload.  A CTA
+// takes sub-blocks [k0, k1) of a block: a window's (32), or half of them when
+// a column has fewer windows than the GPU has places for CTAs, so a column of
+// a few blocks is spread over more SMs and a grown block over four CTAs.  Where
+// every sub-block goes follows from the statistics' and the competition's
+// records.  The CTA with the block's first sub-block (`lead`) writes what is
+// not a sub-block's; it alone emits the modes whose parts depend on a pass
+// over the block (a large dictionary, entropy-coded parts).
 // ---------------------------------------------------------------------------
-__device__ void emit_raw(const uint64_t* v, uint32_t n, int dtype, uint8_t* out) {
+__device__ void emit_raw(const uint64_t* v, uint32_t n, int dtype, uint8_t* out, uint32_t k0, uint32_t k1) {
+  const uint32_t i1 = min(n, k1 * kSub);
   uint32_t lb = lane_bytes(dtype);
 #pragma unroll 8
-  for (uint32_t i = threadIdx.x; i < n; i += blockDim.x) {
+  for (uint32_t i = k0 * kSub + threadIdx.x; i < i1; i += blockDim.x) {
     uint64_t x = v[i];
     if (dtype == DT_F32) put_u32(out + 4ull * i, f64bits_to_f32bits(x));
     else if (lb == 4) put_u32(out + 4ull * i, (uint32_t)x);
@@ -2479,22 +2938,12 @@ __device__ void emit_raw(const uint64_t* v, uint32_t n, int dtype, uint8_t* out)
   }
 }
 
-// S.subsz[k] holds each sub-block's LEB128 byte count on entry.
-__device__ void emit_xorz(EncSmem& S, const uint64_t* v, uint32_t n, uint8_t* out) {
+// S.subsz[k] holds each sub-block's LEB128 byte offset on entry.
+__device__ void emit_xorz(EncSmem& S, const uint64_t* v, uint32_t n, uint8_t* out, uint32_t k0, uint32_t k1) {
   int lane = threadIdx.x & 31, warp = threadIdx.x >> 5;
-  uint32_t nsub = (n + kSub - 1) / kSub;
-  if (threadIdx.x == 0) {
-    uint32_t acc = 0;
-    for (uint32_t k = 0; k < nsub; k++) {
-      uint32_t c = S.subsz[k];
-      S.subsz[k] = acc;
-      acc += c;
-    }
-  }
-  __syncthreads();
-  for (uint32_t k = warp; k < nsub; k += kEncWarps) {
+  for (uint32_t k = k0 + warp; k < k1; k += kEncWarps) {
     uint32_t base = k * kSub, cnt = min((uint32_t)kSub, n - base);
-    uint32_t off = S.subsz[k];
+    uint8_t* dst = out + S.subsz[k];
     uint64_t carry = base ? v[base - 1] : 0ull;
     for (uint32_t j0 = 0; j0 < 32; j0 += 8) {
       uint64_t xs[8];
@@ -2507,19 +2956,20 @@ __device__ void emit_xorz(EncSmem& S, const uint64_t* v, uint32_t n, uint8_t* ou
       for (int q = 0; q < 8; q++) {
         uint32_t li = (j0 + q) * 32 + lane;
         bool ok = li < cnt;
-        uint64_t up = __shfl_up_sync(0xffffffffu, xs[q], 1);
-        uint64_t x = ok ? xs[q] ^ (lane ? up : carry) : 0ull;
-        carry = __shfl_sync(0xffffffffu, xs[q], 31);
+        uint64_t rot = __shfl_sync(0xffffffffu, xs[q], (lane + 31) & 31);
+        uint64_t x = ok ? xs[q] ^ (lane ? rot : carry) : 0ull;
+        carry = rot;
         uint32_t sz = ok ? varint_len(x) : 0u;
         uint32_t inc = warp_incl_scan(sz);
-        if (ok) put_varint(out + off + inc - sz, x);
-        off += __shfl_sync(0xffffffffu, inc, 31);
+        if (ok) put_varint(dst + inc - sz, x);
+        dst += __shfl_sync(0xffffffffu, inc, 31);
       }
     }
   }
 }
 
-__device__ void emit_alp(EncSmem& S, const uint64_t* v, uint32_t n, const SubStats* ss, uint8_t* out) {
+__device__ __noinline__ void emit_alp(EncSmem& S, const uint64_t* v, uint32_t n, const SubStats* ss, uint8_t* out, uint32_t k0,
+                         uint32_t k1) {
   int lane = threadIdx.x & 31, warp = threadIdx.x >> 5;
   uint32_t nsub = (n + kSub - 1) / kSub;
   __shared__ int64_t s_fill[kSubsMax];
@@ -2529,11 +2979,18 @@ __device__ void emit_alp(EncSmem& S, const uint64_t* v, uint32_t n, const SubSta
     s_pfrac[threadIdx.x] = kFrac10[threadIdx.x];
   }
   __syncthreads();
-  for (uint32_t k = warp; k < nsub; k += kEncWarps) {
+  // the statistics' (e, f), width and exception count of every sub-block, or
+  // (Sample at Fastest) all of them searched again by the lead CTA
+  const bool known = ss && (ss[0].pad16 & kAlpEfKnown);
+  if (!known) {
+    if (k0) return;
+    k1 = nsub;
+  }
+  for (uint32_t k = k0 + warp; k < k1; k += kEncWarps) {
     uint32_t cnt = min((uint32_t)kSub, n - k * kSub);
     AlpSub a;
-    uint16_t ef = ss ? ss[k].pad16 : 0;  // the statistics' (e, f), or search again (Sample at Fastest)
-    if (ef & kAlpEfKnown) {
+    if (known) {
+      const uint16_t ef = ss[k].pad16;
       a.e = ef & 0xFF;
       a.f = (ef >> 8) & 0x7F;
       alp_subblock_ef(v + (uint64_t)k * kSub, cnt, a.e, a.f, s_pexp, s_pfrac, &a);
@@ -2547,23 +3004,28 @@ __device__ void emit_alp(EncSmem& S, const uint64_t* v, uint32_t n, const SubSta
       S.alp_exc[k] = (uint16_t)a.exc;
       S.submin[k] = (uint64_t)a.mn;
       s_fill[k] = a.filler;
+      if (!known) S.subsz[k] = 13 + 128u * a.w + 10u * a.exc;
     }
   }
-  __syncthreads();
-  if (threadIdx.x == 0) {
-    uint32_t off = put_varint(out, n);
-    for (uint32_t k = 0; k < nsub; k++) {
-      S.subsz[k] = off;
-      off += 13 + 128u * S.w_c[k] + 10u * S.alp_exc[k];
-    }
-  }
-  __syncthreads();
-  for (uint32_t k = warp; k < nsub; k += kEncWarps) {
+  if (known)
+    for (uint32_t k = threadIdx.x; k < nsub; k += blockDim.x) S.subsz[k] = 13 + 128u * ss[k].alp_w + 10u * ss[k].alp_exc;
+  block_offsets(S, nsub, varint_len(n));
+  if (threadIdx.x == 0 && k0 == 0) put_varint(out, n);
+  for (uint32_t k = k0 + warp; k < k1; k += kEncWarps) {
     uint32_t base = k * kSub, cnt = min((uint32_t)kSub, n - base);
     uint8_t* d = out + S.subsz[k];
     int e = S.alp_ef[k][0], f = S.alp_ef[k][1];
     uint32_t w = S.w_c[k];
     int64_t mn = (int64_t)S.submin[k], fill = s_fill[k];
+    const uint64_t* sv = v + base;
+    // Digits (exceptions and padding take the filler digit), FastLanes packed:
+    // a FoR sub-block at d + 4 whose width byte and minimum the ALP header
+    // holds the other way round.
+    warp_for_pack(d + 4, (uint32_t)kSub, (uint64_t)mn, w, [&](uint32_t i) {
+      int64_t dd;
+      return (uint64_t)(i < cnt && alp_roundtrips(sv[i], e, f, &dd) ? dd : fill);
+    });
+    __syncwarp();
     if (lane == 0) {
       put_u8(d, e);
       put_u8(d + 1, f);
@@ -2571,34 +3033,10 @@ __device__ void emit_alp(EncSmem& S, const uint64_t* v, uint32_t n, const SubSta
       put_u64(d + 4, (uint64_t)mn);
       put_u8(d + 12, w);
     }
-    const uint64_t* sv = v + base;
-    // Digits (exceptions and padding take the filler digit), FastLanes packed.
-    if (w > 0) {
-      uint64_t acc = 0;
-      uint32_t nb = 0, wd = 0;
-      for (uint32_t r = 0; r < 32; r++) {
-        uint32_t i = r * 32 + lane;
-        int64_t dg = fill;
-        if (i < cnt) {
-          int64_t dd;
-          if (alp_roundtrips(sv[i], e, f, &dd)) dg = dd;
-        }
-        uint32_t res = (uint32_t)((uint64_t)dg - (uint64_t)mn);
-        if (w < 32) res &= (1u << w) - 1u;
-        acc |= (uint64_t)res << nb;
-        nb += w;
-        if (nb >= 32) {
-          put_u32(d + 13 + 4u * (wd * 32u + lane), (uint32_t)acc);
-          wd++;
-          acc >>= 32;
-          nb -= 32;
-        }
-      }
-    }
     // Exceptions in position order.
     uint8_t* xp = d + 13 + 128u * w;
     uint32_t before = 0;
-    for (uint32_t j = 0; j < 32; j++) {
+    for (uint32_t j = 0; S.alp_exc[k] && j < 32; j++) {
       uint32_t li = j * 32 + lane;
       bool ok = li < cnt;
       int64_t dd;
@@ -2614,132 +3052,167 @@ __device__ void emit_alp(EncSmem& S, const uint64_t* v, uint32_t n, const SubSta
   }
 }
 
-__device__ void emit_alprd(EncSmem& S, const uint64_t* v, uint32_t n, uint32_t lbw, uint8_t* scr, uint8_t* out,
-                           const EntRec* er) {
-  int lane = threadIdx.x & 31, warp = threadIdx.x >> 5;
-  uint32_t nsub = (n + kSub - 1) / kSub;
-  rd_top8(S, v, n, lbw, scr);
-  uint32_t rbw = 64 - lbw;
-  uint64_t rmask = (1ull << rbw) - 1ull;
-  // exception bytes per sub-block
-  for (uint32_t k = warp; k < nsub; k += kEncWarps) {
-    uint32_t base = k * kSub, cnt = min((uint32_t)kSub, n - base);
-    uint32_t eb = 0, ne = 0;
-    for (uint32_t i = lane; i < cnt; i += 32) {
-      if (rd_code(S, v[base + i] >> rbw) < 0) {
-        eb += varint_len(base + i) + 8;
-        ne++;
-      }
-    }
-    eb = warp_sum(eb);
-    ne = warp_sum(ne);
-    if (lane == 0) {
-      S.subsz[k] = eb;
-      S.neq_k[k] = ne;
-    }
+// ALP-RD from the competition's records: every part's place is known, so a
+// warp writes its sub-block's exceptions, codes and rights one after another
+// while the values are in L1.  (Counting the left parts again, then a pass for
+// each part's sizes and each part's bytes, took 238 us for 1,048,576 prices.)
+__device__ __noinline__ void emit_alprd(EncSmem& S, const uint64_t* v, uint32_t n, uint32_t lbw, const RdRec* rec,
+                           const BlkRec& B, uint8_t* scr, uint8_t* out, const EntRec* er, uint32_t k0, uint32_t k1) {
+  const int lane = threadIdx.x & 31, warp = threadIdx.x >> 5;
+  const uint32_t nsub = (n + kSub - 1) / kSub;
+  const uint32_t rbw = 64 - lbw;
+  const uint64_t rmask = (1ull << rbw) - 1ull;
+  if (threadIdx.x < 8) S.dict8[threadIdx.x] = B.dict8[threadIdx.x];
+  if (threadIdx.x == 0) {
+    S.dl = B.dl;
+    S.cnt32 = 0;
   }
   __syncthreads();
-  if (threadIdx.x == 0) {
+  // offsets of the exceptions (relative), the codes' and the rights' sub-blocks
+  uint32_t ne = 0;
+  for (uint32_t k = threadIdx.x; k < nsub; k += blockDim.x) {
+    S.subsz[k] = rec[k].eb;
+    ne += rec[k].ne;
+  }
+  ne = __reduce_add_sync(0xffffffffu, ne);
+  if (lane == 0 && ne) atomicAdd(&S.cnt32, ne);
+  __syncthreads();
+  const uint32_t nexc = S.cnt32, vl = varint_len(n);
+  const uint32_t head = 2 + 8 * S.dl + varint_len(nexc);
+  block_offsets(S, nsub, head);
+  const uint32_t cpos = S.subsz[nsub];  // the codes' tag
+  for (uint32_t k = threadIdx.x; k < nsub; k += blockDim.x) S.rd_eb[k] = S.subsz[k];
+  __syncthreads();
+  for (uint32_t k = threadIdx.x; k < nsub; k += blockDim.x) S.subsz[k] = 9 + 128u * rec[k].cw;
+  block_offsets(S, nsub, vl);
+  uint32_t clen = S.subsz[nsub];
+  for (uint32_t k = threadIdx.x; k < nsub; k += blockDim.x) S.rd_ne[k] = S.subsz[k];  // within the codes
+  __syncthreads();
+  for (uint32_t k = threadIdx.x; k < nsub; k += blockDim.x) S.subsz[k] = 9 + 128u * rec[k].rw;
+  block_offsets(S, nsub, vl);
+  const bool ccoded = er && (er->flags & kEntRdCodes), rcoded = er && (er->flags & kEntRdRights);
+  if (ccoded) clen = er->rdc;
+  const uint32_t c0 = cpos + 1 + varint_len(clen), rpos = c0 + clen;  // the codes; the rights' tag
+  if (threadIdx.x == 0 && k0 == 0) {
     uint32_t pos = 0;
     put_u8(out + pos++, lbw);
     put_u8(out + pos++, S.dl);
     for (uint32_t j = 0; j < S.dl; j++, pos += 8) put_u64(out + pos, S.dict8[j]);
-    uint64_t nexc = 0;
-    for (uint32_t k = 0; k < nsub; k++) nexc += S.neq_k[k];
-    pos += put_varint(out + pos, nexc);
-    for (uint32_t k = 0; k < nsub; k++) {
-      uint32_t c = S.subsz[k];
-      S.subsz[k] = pos;
-      pos += c;
-    }
-    S.sc[6] = pos;  // codes tag position
+    put_varint(out + pos, nexc);
+    put_u8(out + cpos, ccoded ? 1 : 0);
+    put_varint(out + cpos + 1, clen);
+    if (!ccoded) put_varint(out + c0, n);
+    put_u8(out + rpos, rcoded ? 1 : 0);
+    if (!rcoded) put_varint(out + rpos + 1, n);
   }
-  __syncthreads();
-  for (uint32_t k = warp; k < nsub; k += kEncWarps) {
-    uint32_t base = k * kSub, cnt = min((uint32_t)kSub, n - base);
-    uint32_t off = S.subsz[k];
-    for (uint32_t j = 0; j < 32; j++) {
-      uint32_t li = j * 32 + lane;
-      bool ok = li < cnt;
-      uint64_t x = ok ? v[base + li] : 0;
-      bool ex = ok && rd_code(S, x >> rbw) < 0;
-      uint32_t sz = ex ? varint_len(base + li) + 8 : 0u;
-      uint32_t inc = warp_incl_scan(sz);
-      if (ex) {
-        uint8_t* q = out + off + inc - sz;
-        uint32_t vlb = put_varint(q, base + li);
-        put_u64(q + vlb, x >> rbw);
-      }
-      off += __shfl_sync(0xffffffffu, inc, 31);
-    }
-  }
-  __syncthreads();
-  uint64_t pos = S.sc[6];
-  auto code_of = [&](uint32_t i) -> uint64_t {
+  auto code_at = [&](uint32_t i) -> uint64_t {
     int c = rd_code(S, v[i] >> rbw);
     return c < 0 ? 0ull : (uint64_t)c;
   };
-  uint64_t rpos;
-  if (er && (er->flags & kEntRdCodes)) {
-    uint32_t clen = er->rdc, cvl = varint_len(clen);
-    if (threadIdx.x == 0) {
-      put_u8(out + pos, 1);
-      put_varint(out + pos + 1, clen);
+  for (uint32_t k = k0 + warp; k < k1; k += kEncWarps) {
+    const uint32_t base = k * kSub, cnt = min((uint32_t)kSub, n - base);
+    const RdRec r = rec[k];
+    if (!ccoded) warp_for_pack(out + c0 + S.rd_ne[k], cnt, r.cmin, r.cw, [&](uint32_t i) { return code_at(base + i); });
+    if (!rcoded)
+      warp_for_pack(out + rpos + 1 + S.subsz[k], cnt, r.rmin, r.rw, [&](uint32_t i) { return v[base + i] & rmask; });
+    uint32_t off = S.rd_eb[k];
+    for (uint32_t j0 = 0; r.ne && j0 < 32; j0 += 8) {
+      uint64_t xs[8];
+#pragma unroll
+      for (int q = 0; q < 8; q++) {
+        uint32_t li = (j0 + q) * 32 + lane;
+        xs[q] = li < cnt ? v[base + li] : 0ull;
+      }
+#pragma unroll
+      for (int q = 0; q < 8; q++) {
+        uint32_t li = (j0 + q) * 32 + lane;
+        bool ex = li < cnt && rd_code(S, xs[q] >> rbw) < 0;
+        if (!__any_sync(0xffffffffu, ex)) continue;
+        uint32_t sz = ex ? varint_len(base + li) + 8 : 0u;
+        uint32_t inc = warp_incl_scan(sz);
+        if (ex) {
+          uint8_t* d = out + off + inc - sz;
+          uint32_t vlb = put_varint(d, base + li);
+          put_u64(d + vlb, xs[q] >> rbw);
+        }
+        off += __shfl_sync(0xffffffffu, inc, 31);
+      }
     }
-    coded_write(S.ra, n, [&](uint32_t i) { return (uint32_t)code_of(i); }, out + pos + 1 + cvl, clen);
-    rpos = pos + 1 + cvl + clen;
-  } else {
-    uint64_t clen = block_for(S, nullptr, n, false, code_of);
-    uint32_t cvl = varint_len(clen);
-    if (threadIdx.x == 0) {
-      put_u8(out + pos, 0);
-      put_varint(out + pos + 1, clen);
-    }
-    block_for(S, out + pos + 1 + cvl, n, false, code_of);
-    rpos = pos + 1 + cvl + clen;
   }
-  auto right_of = [&](uint32_t i) { return v[i] & rmask; };
-  if (er && (er->flags & kEntRdRights)) {  // the bit-packed rights, coded
+  if (ccoded) coded_write(S.ra, n, [&](uint32_t i) { return (uint32_t)code_at(i); }, out + c0, clen);
+  if (rcoded) {  // the bit-packed rights, coded
+    auto right_of = [&](uint32_t i) { return v[i] & rmask; };
     uint8_t* rdst = stage_dst(S, scr, n, block_for(S, nullptr, n, false, right_of));
     uint32_t rb = (uint32_t)block_for(S, rdst, n, false, right_of);
-    if (threadIdx.x == 0) put_u8(out + rpos, 1);
     coded_write(S.ra, rb, [&](uint32_t i) { return (uint32_t)rdst[i]; }, out + rpos + 1, er->rdr);
-  } else {
-    if (threadIdx.x == 0) put_u8(out + rpos, 0);
-    block_for(S, out + rpos + 1, n, false, right_of);
   }
 }
 
-__device__ void emit_dict(EncSmem& S, const uint64_t* v, uint32_t n, const SubStats* ss, uint8_t* scr, uint8_t* out,
-                          const EntRec* er) {
-  DictView dv = dict_prepare(S, v, n, scr, kNoLb);
+// The small dictionary that the competition kept (ascending), as the shared
+// hash table of dict_prepare.
+__device__ DictView dict_restore(EncSmem& S, const uint64_t* keep, uint32_t card) {
+  DictArea& D = S.big.dict;
+  for (uint32_t i = threadIdx.x; i < kHashCap; i += blockDim.x) D.hkey[i] = kEmpty64;
+  __syncthreads();
+  for (uint32_t r = threadIdx.x; r < card; r += blockDim.x) {
+    const uint64_t x = keep[r];
+    D.sorted[r] = x;
+    if (x == kEmpty64) {
+      S.max_rank = r;
+      continue;
+    }
+    uint32_t h = (uint32_t)((x * 0x9E3779B97F4A7C15ull) >> 53);
+    while (atomicCAS((unsigned long long*)&D.hkey[h], kEmpty64, x) != kEmpty64) h = (h + 1) & (kHashCap - 1);
+    D.hval[h] = r;
+  }
+  __syncthreads();
+  DictView dv;
+  dv.smem = true;
+  dv.sorted = D.sorted;
+  dv.card = card;
+  return dv;
+}
+
+__device__ __noinline__ void emit_dict(EncSmem& S, const uint64_t* v, uint32_t n, const SubStats* ss, const BlkRec& B, uint8_t* scr,
+                          uint8_t* out, const EntRec* er, uint32_t k0, uint32_t k1) {
+  const bool kept = B.card != 0;
+  if (!kept && k0) return;
+  DictView dv;
   uint32_t vtag;
-  uint64_t vlen = dict_values_len(S, dv, &vtag);
+  uint64_t vlen;
+  if (kept) {
+    dv = dict_restore(S, reinterpret_cast<const uint64_t*>(scr + 16ull * n), B.card);
+    vtag = B.vtag;
+    vlen = B.vlen;
+  } else {
+    dv = dict_prepare(S, v, n, scr, kNoLb);
+    vlen = dict_values_len(S, dv, &vtag);
+    k1 = (n + kSub - 1) / kSub;
+  }
   if (er && (er->flags & kEntDictVals)) {
     vtag = 2;
     vlen = er->dv;
   }
-  uint64_t pos = 0;
-  if (threadIdx.x == 0) {
-    pos = put_varint(out, dv.card);
-    put_u8(out + pos++, vtag);
-    pos += put_varint(out + pos, vlen);
-    S.sc[6] = pos;
-  }
-  __syncthreads();
-  pos = S.sc[6];
+  const uint32_t card = dv.card;
+  uint64_t pos = varint_len(card) + 1 + varint_len(vlen);
   const uint64_t* s = dv.sorted;
-  uint32_t card = dv.card;
-  if (vtag == 0) {
-    for (uint32_t i = threadIdx.x; i < card; i += blockDim.x) put_u64(out + pos + 8ull * i, s[i]);
-  } else if (vtag == 1) {
-    if (threadIdx.x == 0) put_u64(out + pos, s[0]);
-    block_for(S, out + pos + 8, card, false, [&](uint32_t i) { return zigzag64(s[i] - (i ? s[i - 1] : s[0])); });
-  } else {
-    coded_write(S.ra, 8 * card, [&](uint32_t i) {
-      uint32_t pl = i / card;
-      return (uint32_t)(s[i - pl * card] >> (8 * pl)) & 255u;
-    }, out + pos, (uint32_t)vlen);
+  if (k0 == 0) {
+    if (threadIdx.x == 0) {
+      uint32_t q = put_varint(out, card);
+      put_u8(out + q, vtag);
+      put_varint(out + q + 1, vlen);
+    }
+    if (vtag == 0) {
+      for (uint32_t i = threadIdx.x; i < card; i += blockDim.x) put_u64(out + pos + 8ull * i, s[i]);
+    } else if (vtag == 1) {
+      if (threadIdx.x == 0) put_u64(out + pos, s[0]);
+      block_for(S, out + pos + 8, card, false, [&](uint32_t i) { return zigzag64(s[i] - (i ? s[i - 1] : s[0])); });
+    } else {
+      coded_write(S.ra, 8 * card, [&](uint32_t i) {
+        uint32_t pl = i / card;
+        return (uint32_t)(s[i - pl * card] >> (8 * pl)) & 255u;
+      }, out + pos, (uint32_t)vlen);
+    }
   }
   __syncthreads();
   pos += vlen;
@@ -2759,7 +3232,7 @@ __device__ void emit_dict(EncSmem& S, const uint64_t* v, uint32_t n, const SubSt
     }
     return;
   }
-  if (threadIdx.x == 0) put_u8(out + pos, 0);
+  if (threadIdx.x == 0 && k0 == 0) put_u8(out + pos, 0);
   // The dictionary is sorted, so a sub-block's codes run from the rank of its
   // smallest value to the rank of its largest (the statistics' unsigned
   // min / max): the FoR widths and bases without a pass over the codes.
@@ -2770,55 +3243,74 @@ __device__ void emit_dict(EncSmem& S, const uint64_t* v, uint32_t n, const SubSt
     S.submin[k] = r0;
   }
   __syncthreads();
-  block_for_write(S, out + pos + 1, n, [&](uint32_t i) { return (uint64_t)dict_rank(S, dv, v[i]); });
+  block_for_write(S, out + pos + 1, n, [&](uint32_t i) { return (uint64_t)dict_rank(S, dv, v[i]); }, k0, k1);
 }
 
-// The block's run starts from its transitions per sub-block, which the
-// statistics pass counted: the sub-block's own plus its first value against
-// the previous sub-block's last (as the competition counts them).
-__device__ void emit_rle(EncSmem& S, const uint64_t* v, uint32_t n, const SubStats* ss, uint8_t* scr,
-                         uint8_t* out) {
-  uint32_t nsub = (n + kSub - 1) / kSub;
-  for (uint32_t k = threadIdx.x; k < nsub; k += blockDim.x) {
-    const SubStats& R = ss[k];
-    S.neq_k[k] = R.neq + ((k && R.first != ss[k - 1].last) ? 1u : 0u);
+// RLE from the competition's run starts: the CTA's share of the run values and
+// of the 1,024-run chunks of the lengths, whose layout is in the block's
+// records.
+__device__ __noinline__ void emit_rle(EncSmem& S, const uint64_t* v, uint32_t n, const RdRec* rec, const BlkRec& B,
+                                      const uint8_t* scr, uint8_t* out, uint32_t part, uint32_t parts) {
+  const uint32_t* st = reinterpret_cast<const uint32_t*>(scr);
+  const uint32_t runs = B.card, vl = varint_len(runs), nch = (runs + kSub - 1) / kSub;
+  auto len_at = [&](uint32_t r) { return (uint64_t)((r + 1 < runs ? st[r + 1] : n) - st[r]); };
+  if (threadIdx.x == 0 && part == 0) put_varint(out, runs);
+  const uint32_t per = (runs + parts - 1) / parts, r0 = min(part * per, runs), r1 = min(r0 + per, runs);
+  for (uint32_t r = r0 + threadIdx.x; r < r1; r += blockDim.x) put_u64(out + vl + 8ull * r, v[st[r]]);
+  for (uint32_t k = threadIdx.x; k < nch; k += blockDim.x) {
+    S.w_a[k] = rec[k].rw;
+    S.submin[k] = rec[k].rmin;
   }
   __syncthreads();
-  if (threadIdx.x == 0) {
-    uint32_t t = 0;
-    for (uint32_t k = 0; k < nsub; k++) t += S.neq_k[k];
-    S.cnt32 = t + 1;
-  }
-  __syncthreads();
-  uint32_t runs = S.cnt32;
-  uint32_t* st = rle_starts(S, v, n, runs, scr);
-  uint32_t vl = varint_len(runs);
-  if (threadIdx.x == 0) put_varint(out, runs);
-  for (uint32_t r = threadIdx.x; r < runs; r += blockDim.x) put_u64(out + vl + 8ull * r, v[st[r]]);
-  block_for(S, out + vl + 8ull * runs, runs, false,
-            [&](uint32_t r) { return (uint64_t)((r + 1 < runs ? st[r + 1] : n) - st[r]); });
+  const uint32_t cper = (nch + parts - 1) / parts, c0 = min(part * cper, nch);
+  block_for_write(S, out + vl + 8ull * runs, runs, len_at, c0, min(c0 + cper, nch));
 }
 
+// w2b: the block of each window (adaptive plan); split: CTAs per window.
+constexpr uint32_t kWinSubs = kBaseQuantum / kSub;
 template <bool ENT>
-__global__ void __launch_bounds__(kEncThreads) k_emit(const uint64_t* __restrict__ lane,
+__global__ void __launch_bounds__(kEncThreads, 2) k_emit(const uint64_t* __restrict__ lane,
                                                       const FrameDesc* __restrict__ frames,
-                                                      const uint32_t* __restrict__ nbp, uint64_t fixed_bs, int dtype,
+                                                      const uint32_t* __restrict__ nbp,
+                                                      const uint32_t* __restrict__ w2b, uint32_t split,
+                                                      uint64_t fixed_bs, int dtype,
                                                       const SubStats* __restrict__ ss,
                                                       const FmStat* __restrict__ fms,
+                                                      const RdRec* __restrict__ rdr, const BlkRec* __restrict__ blk,
                                                       uint8_t* __restrict__ scratch, uint8_t* __restrict__ outbuf,
                                                       uint64_t out_cap, const EntRec* __restrict__ ent) {
   extern __shared__ __align__(16) uint8_t smem_raw[];
   EncSmem& S = *reinterpret_cast<EncSmem*>(smem_raw);
-  uint32_t b = blockIdx.x;
+  const uint32_t unit = blockIdx.x / split, part = blockIdx.x % split;
+  uint32_t b, win;  // the block, and the unit's window within it
+  if (fixed_bs) {
+    const uint32_t per = (uint32_t)((fixed_bs + kBaseQuantum - 1) / kBaseQuantum);
+    b = unit / per;
+    win = unit % per;
+  } else {
+    b = w2b[unit];
+    win = 0;
+  }
   if (b >= *nbp) return;
   FrameDesc fd = frames[b];
+  if (!fixed_bs) win = unit - (uint32_t)(fd.value_off / kBaseQuantum);
   if (fd.payload_off + fd.plen > out_cap) return;  // the caller sees the total and reports the shortfall
   const uint64_t* v = lane + fd.value_off;
   uint32_t n = fd.n;
+  const uint32_t nsub = (n + kSub - 1) / kSub, cut = kWinSubs / split;
+  uint32_t k0 = win * kWinSubs + part * cut, k1 = min(k0 + cut, nsub);
+  const int m = (int)fd.mode;
+  const uint32_t parts = (nsub + cut - 1) / cut;
+  if (ENT || m == M_CONST || m == M_STRIDE) {  // whole blocks
+    if (k0) return;
+    k1 = nsub;
+  }
+  if (k0 >= k1) return;
+  const bool lead = k0 == 0;
   uint8_t* scr = scratch + fd.value_off * kEncScratchPerValue;
   uint8_t* hdr = outbuf + fd.payload_off - 9;
   uint8_t* out = outbuf + fd.payload_off;
-  if (threadIdx.x == 0) {
+  if (threadIdx.x == 0 && lead) {
     put_u8(hdr, fd.mode);
     put_u32(hdr + 1, n);
     put_u32(hdr + 5, fd.plen);
@@ -2826,9 +3318,7 @@ __global__ void __launch_bounds__(kEncThreads) k_emit(const uint64_t* __restrict
   bool sgn = dtype_signed(dtype);
   // FoR / DELTA / FLOAT_MULT / XORZ sub-block layouts come from the statistics
   // pass (the same numbers the competition sized the frame with).
-  uint32_t nsub = (n + kSub - 1) / kSub;
   uint64_t g0 = fixed_bs ? (uint64_t)b * ((fixed_bs + kSub - 1) / kSub) : fd.value_off / kSub;
-  int m = (int)fd.mode;
   EntRec er = {0, 0, 0, 0, 0, 0, {0, 0}};
   if (ENT) er = ent[b];
   const EntRec* erp = ENT ? &er : nullptr;
@@ -2856,10 +3346,11 @@ __global__ void __launch_bounds__(kEncThreads) k_emit(const uint64_t* __restrict
       S.w_a[k] = (uint8_t)w;
       S.submin[k] = mn;
     }
+    if (m == M_XORZ) block_offsets(S, nsub, 0);
     __syncthreads();
   }
   switch (fd.mode) {
-    case M_RAW: emit_raw(v, n, dtype, out); break;
+    case M_RAW: emit_raw(v, n, dtype, out, k0, k1); break;
     case M_CONST:
       if (threadIdx.x == 0) put_u64(out, v[0]);
       break;
@@ -2869,16 +3360,16 @@ __global__ void __launch_bounds__(kEncThreads) k_emit(const uint64_t* __restrict
         put_u64(out + 8, v[1] - v[0]);
       }
       break;
-    case M_XORZ: emit_xorz(S, v, n, out); break;
-    case M_FOR_BITPACK: block_for_write(S, out, n, [&](uint32_t i) { return v[i]; }); break;
+    case M_XORZ: emit_xorz(S, v, n, out, k0, k1); break;
+    case M_FOR_BITPACK: block_for_write(S, out, n, [&](uint32_t i) { return v[i]; }, k0, k1); break;
     case M_DELTA_BITPACK:
-      if (threadIdx.x == 0) put_u64(out, v[0]);
-      block_for_write(S, out + 8, n, [&](uint32_t i) { return zigzag64(v[i] - (i ? v[i - 1] : v[0])); });
+      if (threadIdx.x == 0 && lead) put_u64(out, v[0]);
+      block_for_write(S, out + 8, n, [&](uint32_t i) { return zigzag64(v[i] - (i ? v[i - 1] : v[0])); }, k0, k1);
       break;
     case M_FLOAT_MULT: {
       int s = (int)fd.aux;
       bool coded = ENT && (er.flags & kEntFm);
-      if (threadIdx.x == 0) {
+      if (threadIdx.x == 0 && lead) {
         put_u8(out, coded ? 1 : 0);
         put_u8(out + 1, s);
       }
@@ -2886,7 +3377,7 @@ __global__ void __launch_bounds__(kEncThreads) k_emit(const uint64_t* __restrict
         uint32_t mb = fm_delta_bytes(S, v, n, s, scr);
         coded_write(S.ra, mb, [&](uint32_t i) { return (uint32_t)scr[i]; }, out + 2, er.fm);
       } else {
-        block_for_write(S, out + 2, n, [&](uint32_t i) { return (uint64_t)fm_k(v[i], s); });
+        block_for_write(S, out + 2, n, [&](uint32_t i) { return (uint64_t)fm_k(v[i], s); }, k0, k1);
       }
       break;
     }
@@ -2897,10 +3388,10 @@ __global__ void __launch_bounds__(kEncThreads) k_emit(const uint64_t* __restrict
           return (uint32_t)(v[i - pl * n] >> (8 * pl)) & 255u;
         }, out, fd.plen);
       break;
-    case M_ALP: emit_alp(S, v, n, ss ? ss + g0 : nullptr, out); break;
-    case M_ALP_RD: emit_alprd(S, v, n, fd.aux, scr, out, erp); break;
-    case M_DICT: emit_dict(S, v, n, ss + g0, scr, out, erp); break;
-    case M_RLE: emit_rle(S, v, n, ss + g0, scr, out); break;
+    case M_ALP: emit_alp(S, v, n, ss ? ss + g0 : nullptr, out, k0, k1); break;
+    case M_ALP_RD: emit_alprd(S, v, n, fd.aux, rdr + g0, blk[b], scr, out, erp, k0, k1); break;
+    case M_DICT: emit_dict(S, v, n, ss + g0, blk[b], scr, out, erp, k0, k1); break;
+    case M_RLE: emit_rle(S, v, n, rdr + g0, blk[b], scr, out, ENT ? 0 : k0 / cut, ENT ? 1 : parts); break;
     default: break;
   }
 }
@@ -2909,10 +3400,12 @@ __global__ void __launch_bounds__(kEncThreads) k_emit(const uint64_t* __restrict
 // Window probe, block planning and frame offsets.
 // ---------------------------------------------------------------------------
 
-// Block plan (reference encoder.rs:154-178): fills frames[].value_off / .n.
+// Block plan (reference encoder.rs:154-178): fills frames[].value_off / .n and
+// (adaptive) each window's block.
 constexpr int kPlanThreads = 1024;
 __global__ void __launch_bounds__(kPlanThreads)
-    k_plan(const uint8_t* __restrict__ grow, uint64_t n, uint64_t fixed_bs, FrameDesc* frames, uint32_t* nb) {
+    k_plan(const uint8_t* __restrict__ grow, uint64_t n, uint64_t fixed_bs, FrameDesc* frames, uint32_t* nb,
+           uint32_t* __restrict__ w2b) {
   if (fixed_bs) {
     uint64_t nblk = (n + fixed_bs - 1) / fixed_bs;
     for (uint64_t i = (uint64_t)blockIdx.x * blockDim.x + threadIdx.x; i < nblk; i += (uint64_t)gridDim.x * blockDim.x) {
@@ -2994,6 +3487,7 @@ __global__ void __launch_bounds__(kPlanThreads)
     base += ci - c;
 #pragma unroll
     for (int q = 0; q < kPer; q++) {
+      if (wb + q < nwin) w2b[wb + q] = base + __popc(starts >> q & 1u) - 1;
       if (!(starts >> q & 1u)) continue;
       uint64_t s0 = (wb + q) * (uint64_t)kBaseQuantum;
       uint64_t end = g[q] ? qmin(s0 + kMaxBlock, n) : qmin(s0 + kBaseQuantum, n);
@@ -3037,12 +3531,12 @@ __global__ void k_frame_apply(FrameDesc* frames, const uint32_t* __restrict__ nb
 // ---------------------------------------------------------------------------
 static size_t enc_smem_bytes() { return sizeof(EncSmem); }
 
-void launch_plan(const uint8_t* grow, uint64_t n, uint64_t fixed_bs, FrameDesc* frames, uint32_t* nb,
+void launch_plan(const uint8_t* grow, uint64_t n, uint64_t fixed_bs, FrameDesc* frames, uint32_t* nb, uint32_t* w2b,
                  cudaStream_t st) {
   unsigned g = 1;
   if (fixed_bs) g = (unsigned)qmin(((n + fixed_bs - 1) / fixed_bs + kPlanThreads - 1) / kPlanThreads, 4096);
   if (g == 0) g = 1;
-  k_plan<<<g, kPlanThreads, 0, st>>>(grow, n, fixed_bs, frames, nb);
+  k_plan<<<g, kPlanThreads, 0, st>>>(grow, n, fixed_bs, frames, nb, w2b);
   count_launches(1);
 }
 
@@ -3074,7 +3568,8 @@ void launch_sub_stats(const uint64_t* lane, uint64_t n, uint64_t fixed_bs, int d
 
 void launch_decide(const uint64_t* lane, FrameDesc* frames, const uint32_t* nb, uint32_t max_blocks, uint64_t fixed_bs,
                    int dtype, int level, const void* ss, const void* fms, const uint64_t* smp16,
-                   const uint32_t* winbits, uint8_t* scratch, void* ent, bool sample, cudaStream_t st) {
+                   const uint32_t* winbits, uint8_t* scratch, void* ent, void* rdr, void* blk, bool sample,
+                   cudaStream_t st) {
   int sm = (int)enc_smem_bytes();
   static std::atomic<unsigned long long> smem_set{0};
   once_per_device(smem_set, [sm] {
@@ -3088,35 +3583,46 @@ void launch_decide(const uint64_t* lane, FrameDesc* frames, const uint32_t* nb, 
     if (ent)
       k_decide<true, false><<<max_blocks, kEncThreads, sm, st>>>(lane, frames, nb, fixed_bs, dtype, level,
                                                           (const SubStats*)ss, (const FmStat*)fms, smp16, winbits,
-                                                          scratch, (EntRec*)ent);
+                                                          scratch, (EntRec*)ent, (RdRec*)rdr, (BlkRec*)blk);
     else if (sample)
       k_decide<false, true><<<max_blocks, kEncThreads, sm, st>>>(lane, frames, nb, fixed_bs, dtype, level,
                                                                  (const SubStats*)ss, (const FmStat*)fms, smp16,
-                                                                 winbits, scratch, nullptr);
+                                                                 winbits, scratch, nullptr, (RdRec*)rdr, (BlkRec*)blk);
     else
       k_decide<false, false><<<max_blocks, kEncThreads, sm, st>>>(lane, frames, nb, fixed_bs, dtype, level,
                                                                   (const SubStats*)ss, (const FmStat*)fms, smp16,
-                                                                  winbits, scratch, nullptr);
+                                                                  winbits, scratch, nullptr, (RdRec*)rdr, (BlkRec*)blk);
   }
   count_launches(max_blocks ? 1 : 0);
 }
 
+// Two CTAs per window while the windows alone leave places free (two CTAs of
+// an SM's registers): 1,048,576 prices' 32 windows emit on 64 SMs.
 void launch_emit(const uint64_t* lane, const FrameDesc* frames, const uint32_t* nb, uint32_t max_blocks,
-                 uint64_t fixed_bs, int dtype, const void* ss, const void* fms, uint8_t* scratch, uint8_t* out,
-                 uint64_t out_cap, const void* ent, cudaStream_t st) {
+                 const uint32_t* w2b, uint64_t n, uint64_t fixed_bs, int dtype, const void* ss, const void* fms,
+                 const void* rdr, const void* blk, uint8_t* scratch, uint8_t* out, uint64_t out_cap, const void* ent,
+                 cudaStream_t st) {
   if (max_blocks) {
+    const uint64_t units = fixed_bs ? max_blocks * ((fixed_bs + kBaseQuantum - 1) / kBaseQuantum)
+                                    : (n + kBaseQuantum - 1) / kBaseQuantum;
+    const uint32_t split = units < 2 * 148 && !ent ? 2 : 1;
+    const unsigned g = (unsigned)(units * split);
     if (ent)
-      k_emit<true><<<max_blocks, kEncThreads, enc_smem_bytes(), st>>>(lane, frames, nb, fixed_bs, dtype,
-                                                                      (const SubStats*)ss, (const FmStat*)fms,
-                                                                      scratch, out, out_cap, (const EntRec*)ent);
+      k_emit<true><<<g, kEncThreads, enc_smem_bytes(), st>>>(lane, frames, nb, w2b, split, fixed_bs, dtype,
+                                                             (const SubStats*)ss, (const FmStat*)fms, (const RdRec*)rdr,
+                                                             (const BlkRec*)blk, scratch, out, out_cap,
+                                                             (const EntRec*)ent);
     else
-      k_emit<false><<<max_blocks, kEncThreads, enc_smem_bytes(), st>>>(lane, frames, nb, fixed_bs, dtype,
-                                                                       (const SubStats*)ss, (const FmStat*)fms,
-                                                                       scratch, out, out_cap, nullptr);
+      k_emit<false><<<g, kEncThreads, enc_smem_bytes(), st>>>(lane, frames, nb, w2b, split, fixed_bs, dtype,
+                                                              (const SubStats*)ss, (const FmStat*)fms,
+                                                              (const RdRec*)rdr, (const BlkRec*)blk, scratch, out,
+                                                              out_cap, nullptr);
   }
   count_launches(max_blocks ? 1 : 0);
 }
 
+uint64_t rd_rec_bytes() { return sizeof(RdRec); }
+uint64_t blk_rec_bytes() { return sizeof(BlkRec); }
 uint64_t ent_rec_bytes() { return sizeof(EntRec); }
 
 unsigned long long* device_win_counters() {

@@ -197,7 +197,8 @@ inline int plain_code(int ext) {
 enum Slot {
   S_IN, S_BM, S_RANK, S_LANE, S_GROW, S_FRAMES, S_NB, S_SIZES, S_TILE, S_SCRATCH, S_OUT, S_VTMP, S_VBLOB,
   S_MISC, S_LIMBS, S_LIMBOUT, S_SRC, S_DSCR, S_ERR, S_OUTVALS, S_DFRAMES, S_DBM, S_DRANK, S_DAUX, S_SUBST, S_FMST,
-  S_SMP16, S_WINBITS, S_DSEL, S_DITEMS, S_PRE, S_ENT, S_ENTREC, S_DPMISC, S_DPCAND, S_DPJ, S_DPRUNS, S_BATCH, S_BSCR, S_BHOST, S_COUNT
+  S_SMP16, S_WINBITS, S_DSEL, S_DITEMS, S_PRE, S_ENT, S_ENTREC, S_DPMISC, S_DPCAND, S_DPJ, S_DPRUNS, S_BATCH, S_BSCR, S_BHOST, S_W2B,
+  S_RDREC, S_BLKREC, S_COUNT
 };
 
 struct QuoinCtx {
@@ -396,6 +397,9 @@ int encode_lane(QuoinCtx* c, cudaStream_t st, const LaneJob& j, uint8_t* d_dst, 
   CK(c->ensure(S_GROW, nwin + 16));
   CK(c->ensure(S_SUBST, (items + 1) * sub_stats_bytes()));
   CK(c->ensure(S_WINBITS, (nwin + 1) * kWinWords * 4));
+  CK(c->ensure(S_W2B, nwin * 4 + 16));
+  CK(c->ensure(S_BLKREC, maxb * blk_rec_bytes()));
+  CK(c->ensure(S_RDREC, (items + 1) * rd_rec_bytes()));
   if (fl) {
     CK(c->ensure(S_FMST, (items + 1) * fm_stats_bytes()));
     CK(c->ensure(S_SMP16, (n / 16 + 2) * 8));
@@ -411,13 +415,14 @@ int encode_lane(QuoinCtx* c, cudaStream_t st, const LaneJob& j, uint8_t* d_dst, 
     TimedRegion tr(T_PLAN, st);
     launch_sub_stats(j.lane, n, bs, j.dtype, level, c->p<void>(S_SUBST), fl ? c->p<void>(S_FMST) : nullptr,
                      fl ? c->p<uint64_t>(S_SMP16) : nullptr, c->p<uint8_t>(S_GROW), c->p<uint32_t>(S_WINBITS), st);
-    launch_plan(c->p<uint8_t>(S_GROW), n, bs, fr, nb, st);
+    launch_plan(c->p<uint8_t>(S_GROW), n, bs, fr, nb, c->p<uint32_t>(S_W2B), st);
   }
   {
     TimedRegion tr(T_COMPETE, st);
     launch_decide(j.lane, fr, nb, (uint32_t)maxb, bs, j.dtype, level, c->p<void>(S_SUBST),
                   fl ? c->p<void>(S_FMST) : nullptr, fl ? c->p<uint64_t>(S_SMP16) : nullptr,
-                  c->p<uint32_t>(S_WINBITS), c->p<uint8_t>(S_SCRATCH), ent, sample, st);
+                  c->p<uint32_t>(S_WINBITS), c->p<uint8_t>(S_SCRATCH), ent, c->p<void>(S_RDREC),
+                  c->p<void>(S_BLKREC), sample, st);
   }
   {
     TimedRegion tr(T_OTHER, st);
@@ -426,7 +431,8 @@ int encode_lane(QuoinCtx* c, cudaStream_t st, const LaneJob& j, uint8_t* d_dst, 
   }
   {  // frames past dst_cap are skipped on the device; the total decides afterwards
     TimedRegion tr(T_EMIT, st);
-    launch_emit(j.lane, fr, nb, (uint32_t)maxb, bs, j.dtype, c->p<void>(S_SUBST), fl ? c->p<void>(S_FMST) : nullptr,
+    launch_emit(j.lane, fr, nb, (uint32_t)maxb, c->p<uint32_t>(S_W2B), n, bs, j.dtype, c->p<void>(S_SUBST),
+                fl ? c->p<void>(S_FMST) : nullptr, c->p<void>(S_RDREC), c->p<void>(S_BLKREC),
                 c->p<uint8_t>(S_SCRATCH), d_dst, dst_cap, ent, st);
   }
   uint64_t hm[2] = {0, 0};

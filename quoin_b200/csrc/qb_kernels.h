@@ -259,7 +259,8 @@ uint64_t sub_stats_bytes();
 uint64_t fm_stats_bytes();
 void launch_sub_stats(const uint64_t* lane, uint64_t n, uint64_t fixed_bs, int dtype, int level, void* ss, void* fms,
                       uint64_t* smp16, uint8_t* grow, uint32_t* winbits, cudaStream_t st);
-void launch_plan(const uint8_t* grow, uint64_t n, uint64_t fixed_bs, FrameDesc* frames, uint32_t* nb,
+// w2b (adaptive): the block of each window.
+void launch_plan(const uint8_t* grow, uint64_t n, uint64_t fixed_bs, FrameDesc* frames, uint32_t* nb, uint32_t* w2b,
                  cudaStream_t st);
 // Competition part 2: one CTA per planned block; writes mode / plen / aux.
 // With `ent` (max_blocks records of ent_rec_bytes()) the Balanced in-pool
@@ -268,17 +269,24 @@ void launch_plan(const uint8_t* grow, uint64_t n, uint64_t fixed_bs, FrameDesc* 
 // Fastest and Fast; not with `ent`).
 void launch_decide(const uint64_t* lane, FrameDesc* frames, const uint32_t* nb, uint32_t max_blocks, uint64_t fixed_bs,
                    int dtype, int level, const void* ss, const void* fms, const uint64_t* smp16,
-                   const uint32_t* winbits, uint8_t* scratch, void* ent, bool sample, cudaStream_t st);
+                   const uint32_t* winbits, uint8_t* scratch, void* ent, void* rdr, void* blk, bool sample,
+                   cudaStream_t st);
 uint64_t ent_rec_bytes();
+// The records that the competition leaves for the emission: rdr per statistics
+// item, blk per block.
+uint64_t rd_rec_bytes();
+uint64_t blk_rec_bytes();
 // `base` (device) holds the byte offset at which the first frame starts.
 void launch_frame_offsets(FrameDesc* frames, const uint32_t* nb, uint32_t max_blocks, const uint64_t* base,
                           uint64_t* sizes_tmp, uint64_t* tile_tmp, uint64_t* total, cudaStream_t st);
-// Emission: one CTA per frame; FoR / DELTA / FLOAT_MULT / XORZ layouts are read
-// from the statistics records of launch_sub_stats.  Frames that would end past
+// Emission: one or two CTAs per 32,768-value window of a frame; FoR / DELTA /
+// FLOAT_MULT / XORZ layouts are read from the statistics records of
+// launch_sub_stats, ALP-RD's and small dictionaries from rdr and blk.  Frames that would end past
 // out_cap bytes are not written.
 void launch_emit(const uint64_t* lane, const FrameDesc* frames, const uint32_t* nb, uint32_t max_blocks,
-                 uint64_t fixed_bs, int dtype, const void* ss, const void* fms, uint8_t* scratch, uint8_t* out,
-                 uint64_t out_cap, const void* ent, cudaStream_t st);
+                 const uint32_t* w2b, uint64_t n, uint64_t fixed_bs, int dtype, const void* ss, const void* fms,
+                 const void* rdr, const void* blk, uint8_t* scratch, uint8_t* out, uint64_t out_cap, const void* ent,
+                 cudaStream_t st);
 
 // ---- lowering / validity (qb_lower.cu) ----
 // Lower n native values (dtype width) to the u64 lane, keeping only positions
