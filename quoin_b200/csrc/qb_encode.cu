@@ -3636,14 +3636,34 @@ unsigned long long* device_win_counters() {
 #include "qb_scan.cuh"
 
 namespace qb {
+// A nested lane's varint(length) and header at *nest.pos, for frames of
+// `total` bytes; returns the offset of the first frame.
+__device__ inline uint64_t nest_base(const NestedLane& nest, uint64_t pos, uint64_t total) {
+  return pos + varint_len(16 + total) + 16;
+}
+__device__ inline void nest_write(const NestedLane& nest, uint64_t pos, uint64_t total) {
+  const uint64_t at = nest_base(nest, pos, total);
+  if (at <= nest.cap) {
+    put_varint(nest.out + pos, 16 + total);
+    for (int i = 0; i < 16; i++) nest.out[at - 16 + i] = nest.hdr.b[i];
+  }
+  *nest.pos = at + total;
+}
+__global__ void k_nest_base(NestedLane nest, const uint64_t* __restrict__ total, uint64_t* __restrict__ base) {
+  if (threadIdx.x || blockIdx.x) return;
+  const uint64_t pos = *nest.pos;
+  *base = nest_base(nest, pos, *total);
+  nest_write(nest, pos, *total);
+}
+
 // At most kSmallWords frames in one CTA of 1,024 threads: k_frame_sizes, the
 // exclusive scan and k_frame_apply in one launch.
 __global__ void __launch_bounds__(1024) k_frame_offsets_small(FrameDesc* frames, const uint32_t* __restrict__ nbp,
-                                                              const uint64_t* __restrict__ base_p,
-                                                              uint64_t* __restrict__ total) {
+                                                              uint64_t* __restrict__ base_p,
+                                                              uint64_t* __restrict__ total, NestedLane nest) {
   __shared__ uint64_t wsum[32];
   uint32_t nb = *nbp, t = threadIdx.x, l = t & 31, warp = t >> 5;
-  uint64_t base = *base_p;
+  uint64_t base = nest.pos ? *nest.pos : *base_p;
   uint64_t v[kSmallPer], s = 0;
 #pragma unroll
   for (uint32_t k = 0; k < kSmallPer; k++) {
@@ -3668,6 +3688,11 @@ __global__ void __launch_bounds__(1024) k_frame_offsets_small(FrameDesc* frames,
     if (l == 31) *total = x;
   }
   __syncthreads();
+  if (nest.pos) {
+    const uint64_t pos = base;
+    base = nest_base(nest, pos, wsum[31]);
+    if (t == 0) nest_write(nest, pos, wsum[31]);
+  }
   uint64_t run = (warp ? wsum[warp - 1] : 0ull) + inc - s;
 #pragma unroll
   for (uint32_t k = 0; k < kSmallPer; k++) {
@@ -3677,18 +3702,26 @@ __global__ void __launch_bounds__(1024) k_frame_offsets_small(FrameDesc* frames,
   }
 }
 
-void launch_frame_offsets(FrameDesc* frames, const uint32_t* nb, uint32_t max_blocks, const uint64_t* base,
-                          uint64_t* sizes_tmp, uint64_t* tile_tmp, uint64_t* total, cudaStream_t st) {
+void launch_frame_offsets(FrameDesc* frames, const uint32_t* nb, uint32_t max_blocks, uint64_t* base,
+                          uint64_t* sizes_tmp, uint64_t* tile_tmp, uint64_t* total, const NestedLane& nest,
+                          cudaStream_t st) {
+  if (max_blocks == 0) {  // a lane without values: its header alone
+    if (!nest.pos) return;
+    cudaMemsetAsync(total, 0, 8, st);
+    k_nest_base<<<1, 32, 0, st>>>(nest, total, base);
+    count_launches(1);
+    return;
+  }
   if (max_blocks <= kSmallWords) {
-    k_frame_offsets_small<<<1, 1024, 0, st>>>(frames, nb, base, total);
+    k_frame_offsets_small<<<1, 1024, 0, st>>>(frames, nb, base, total, nest);
     count_launches(1);
     return;
   }
   unsigned g = (unsigned)qmin((max_blocks + 255) / 256, 1024);
-  if (g == 0) g = 1;
   k_frame_sizes<<<g, 256, 0, st>>>(frames, nb, max_blocks, sizes_tmp);
-  scan_exclusive_u64(sizes_tmp, sizes_tmp, max_blocks ? max_blocks : 1, tile_tmp, total, st);
+  scan_exclusive_u64(sizes_tmp, sizes_tmp, max_blocks, tile_tmp, total, st);
+  if (nest.pos) k_nest_base<<<1, 32, 0, st>>>(nest, total, base);
   k_frame_apply<<<g, 256, 0, st>>>(frames, nb, sizes_tmp, base);
-  count_launches(5);
+  count_launches(nest.pos ? 6 : 5);
 }
 }  // namespace qb

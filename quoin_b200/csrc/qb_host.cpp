@@ -119,13 +119,6 @@ inline uint32_t varint_len_h(uint64_t v) {
   while (v >= 0x80) { v >>= 7; n++; }
   return n;
 }
-inline void put_varint_h(std::vector<uint8_t>& o, uint64_t v) {
-  for (;;) {
-    uint8_t b = (uint8_t)(v & 0x7f);
-    v >>= 7;
-    if (v) o.push_back(b | 0x80); else { o.push_back(b); return; }
-  }
-}
 inline uint64_t rd64(const uint8_t* p) {
   uint64_t v = 0;
   for (int i = 7; i >= 0; i--) v = (v << 8) | p[i];
@@ -196,7 +189,7 @@ inline int plain_code(int ext) {
 // ---------------------------------------------------------------------------
 enum Slot {
   S_IN, S_BM, S_RANK, S_LANE, S_GROW, S_FRAMES, S_NB, S_SIZES, S_TILE, S_SCRATCH, S_OUT, S_VTMP, S_VBLOB,
-  S_MISC, S_LIMBS, S_LIMBOUT, S_SRC, S_DSCR, S_ERR, S_OUTVALS, S_DFRAMES, S_DBM, S_DRANK, S_DAUX, S_SUBST, S_FMST,
+  S_MISC, S_LIMBS, S_SRC, S_DSCR, S_ERR, S_OUTVALS, S_DFRAMES, S_DBM, S_DRANK, S_DAUX, S_SUBST, S_FMST,
   S_SMP16, S_WINBITS, S_DSEL, S_DITEMS, S_PRE, S_ENT, S_ENTREC, S_DPMISC, S_DPCAND, S_DPJ, S_DPRUNS, S_BATCH, S_BSCR, S_BHOST, S_W2B,
   S_RDREC, S_BLKREC, S_COUNT
 };
@@ -320,6 +313,7 @@ struct LaneJob {
   uint64_t block_size;  // 0 = adaptive, else clamped to [1, 131072]
   uint8_t plog2;
   bool vb_raw = false;  // the bitmap's transition count proves the RAW validity blob
+  uint64_t* d_nest = nullptr;  // a decimal's limb lane: its place in the container (device; moves past the stream)
 };
 
 uint64_t max_blocks_for(uint64_t n, uint64_t bs) {
@@ -337,7 +331,8 @@ uint64_t lane_bound(uint64_t n_valid, uint64_t logical_n, int dtype, bool validi
 }
 
 // Runs the GPU competition and emission for one lane (reference
-// encoder.rs:184-214).  Writes the stream at d_dst and its length to *out_len.
+// encoder.rs:184-214).  Writes the stream at d_dst and its length to *out_len;
+// a nested lane goes to d_dst + *j.d_nest and nothing is waited for.
 // LaneJob::level carries Selection::Sample as kSelectSample beside the level.
 constexpr int kSelectSample = 0x100;
 
@@ -353,14 +348,21 @@ int encode_lane(QuoinCtx* c, cudaStream_t st, const LaneJob& j, uint8_t* d_dst, 
     *out_len = lane_bound(n, j.logical_n, j.dtype, j.d_bm != nullptr, bs);
     return QUOIN_ERR_BUFFER_TOO_SMALL;
   }
-  Bytes16 h;
+  NestedLane nest;
+  Bytes16& h = nest.hdr;
   memcpy(h.b, "FCR1", 4);
   h.b[4] = 2;
   h.b[5] = j.d_bm ? 1 : 0;
   h.b[6] = j.plog2;
   h.b[7] = (uint8_t)j.dtype;
   for (int i = 0; i < 8; i++) h.b[8 + i] = (uint8_t)(j.logical_n >> (8 * i));
-  launch_put_header(d_dst, h, d_misc, st);
+  if (j.d_nest) {
+    nest.pos = j.d_nest;
+    nest.out = d_dst;
+    nest.cap = dst_cap;
+  } else {
+    launch_put_header(d_dst, h, d_misc, st);
+  }
   if (j.d_bm) {
     uint64_t ln = j.logical_n, nw = (ln + 31) / 32;
     uint64_t blob_cap = 1 + (ln + 7) / 8 + 16;
@@ -379,6 +381,10 @@ int encode_lane(QuoinCtx* c, cudaStream_t st, const LaneJob& j, uint8_t* d_dst, 
       launch_validity_blob(j.d_bm, ln, vtmp, vtile, c->p<uint8_t>(S_VBLOB), d_misc + 2, st);
       launch_put_validity(d_dst + 16, 16, c->p<uint8_t>(S_VBLOB), d_misc + 2, d_misc, st);
     }
+  }
+  if (maxb == 0 && j.d_nest) {
+    launch_frame_offsets(nullptr, nullptr, 0, d_misc, nullptr, nullptr, d_misc + 1, nest, st);
+    return QUOIN_OK;
   }
   if (maxb == 0) {
     uint64_t base = 0;
@@ -427,7 +433,7 @@ int encode_lane(QuoinCtx* c, cudaStream_t st, const LaneJob& j, uint8_t* d_dst, 
   {
     TimedRegion tr(T_OTHER, st);
     launch_frame_offsets(fr, nb, (uint32_t)maxb, d_misc, c->p<uint64_t>(S_SIZES), c->p<uint64_t>(S_TILE),
-                         d_misc + 1, st);
+                         d_misc + 1, nest, st);
   }
   {  // frames past dst_cap are skipped on the device; the total decides afterwards
     TimedRegion tr(T_EMIT, st);
@@ -435,6 +441,7 @@ int encode_lane(QuoinCtx* c, cudaStream_t st, const LaneJob& j, uint8_t* d_dst, 
                 fl ? c->p<void>(S_FMST) : nullptr, c->p<void>(S_RDREC), c->p<void>(S_BLKREC),
                 c->p<uint8_t>(S_SCRATCH), d_dst, dst_cap, ent, st);
   }
+  if (j.d_nest) return QUOIN_OK;
   uint64_t hm[2] = {0, 0};
   CK(read_small(c, st, hm, d_misc, 16));
   resolve_timing();
@@ -515,75 +522,76 @@ int compress_decimal_device(QuoinCtx* c, cudaStream_t st, int wire, uint64_t n, 
     if (rc) return rc;
     if (n_valid < n) d_bm = d_validity;
   }
-  CK(c->ensure(S_VTMP, (148 * 4 * 5 + 64) * 8));
+  CK(c->ensure(S_VTMP, decimal_vmin_tmp_words() * 8));
   CK(c->ensure(S_MISC, 64 * 8));
   uint64_t* d_vmin = c->p<uint64_t>(S_MISC) + 16;
-  launch_decimal_vmin(d_values, nl, d_bm, n, c->p<uint64_t>(S_VTMP), d_vmin, st);
-  CK(c->ensure(S_LIMBS, (uint64_t)nl * n_valid * 8 + 64));
-  uint64_t* limbs = c->p<uint64_t>(S_LIMBS);
-  launch_decimal_split(d_values, nl, d_bm, d_bm ? c->p<uint64_t>(S_RANK) : nullptr, n, d_vmin, limbs, n_valid, st);
-  uint64_t vmin[4] = {0, 0, 0, 0};
-  CK(read_small(c, st, vmin, d_vmin, 32));
-  std::vector<uint8_t> hdr;
-  const char* magic = "FCR1";
-  hdr.insert(hdr.end(), magic, magic + 4);
-  hdr.push_back(2);
-  hdr.push_back((uint8_t)(2 | (d_bm ? 1 : 0)));
-  hdr.push_back(0);
-  hdr.push_back((uint8_t)wire);
-  for (int i = 0; i < 8; i++) hdr.push_back((uint8_t)(n >> (8 * i)));
-  hdr.push_back((uint8_t)scale);
-  hdr.push_back(precision);
-  hdr.push_back((uint8_t)nl);
-  for (int k = 0; k < nl; k++)
-    for (int i = 0; i < 8; i++) hdr.push_back((uint8_t)(vmin[k] >> (8 * i)));
+  uint64_t* d_pos = c->p<uint64_t>(S_MISC) + 40;  // the container's length so far
   uint64_t need_bound = column_bound(wire, n, d_bm != nullptr, bs);
-  if (dst_cap < hdr.size()) {
+  const uint64_t head = 19 + 8ull * nl;
+  if (dst_cap < head) {
     *out_len = need_bound;
     return QUOIN_ERR_BUFFER_TOO_SMALL;
   }
-  CK(cudaMemcpyAsync(d_dst, hdr.data(), hdr.size(), cudaMemcpyHostToDevice, st));
-  uint64_t pos = hdr.size();
+  // The limbs are streams of their own behind their lengths, written in place
+  // one after another: where the second starts is only known on the device,
+  // so the container's position stays there until the end (one wait a call).
+  {
+    TimedRegion tr(T_LOWER, st);
+    launch_decimal_vmin(d_values, nl, d_bm, n, n_valid != 0, c->p<uint64_t>(S_VTMP), d_vmin, st);
+    CK(c->ensure(S_LIMBS, (uint64_t)nl * n_valid * 8 + 64));
+    launch_decimal_split(d_values, nl, d_bm, d_bm ? c->p<uint64_t>(S_RANK) : nullptr, n, d_vmin,
+                         c->p<uint64_t>(S_LIMBS), n_valid, st);
+  }
+  uint64_t* limbs = c->p<uint64_t>(S_LIMBS);
+  Bytes19 h;
+  memcpy(h.b, "FCR1", 4);
+  h.b[4] = 2;
+  h.b[5] = (uint8_t)(2 | (d_bm ? 1 : 0));
+  h.b[6] = 0;
+  h.b[7] = (uint8_t)wire;
+  for (int i = 0; i < 8; i++) h.b[8 + i] = (uint8_t)(n >> (8 * i));
+  h.b[16] = (uint8_t)scale;
+  h.b[17] = precision;
+  h.b[18] = (uint8_t)nl;
+  launch_put_decimal_header(d_dst, h, nl, d_vmin, d_pos, st);
   if (d_bm) {
     uint64_t nw = (n + 31) / 32;
     uint64_t blob_cap = 1 + (n + 7) / 8 + 16;
-    if (dst_cap < pos + 10 + blob_cap) {
+    if (dst_cap < head + 10 + blob_cap) {
+      CK(cudaStreamSynchronize(st));
       *out_len = need_bound;
       return QUOIN_ERR_BUFFER_TOO_SMALL;
     }
     uint64_t* d_misc = c->p<uint64_t>(S_MISC);
     if (vb_raw) {
-      launch_put_validity_raw(d_dst + pos, pos, d_bm, n, d_misc + 3, st);
+      launch_put_validity_raw(d_dst + head, head, d_bm, n, d_pos, st);
     } else {
       CK(c->ensure(S_VTMP, (validity_tmp_words(n) + scan_tile_count(nw) + 16) * 8));
       CK(c->ensure(S_VBLOB, blob_cap));
       uint64_t* vtmp = c->p<uint64_t>(S_VTMP);
       launch_validity_blob(d_bm, n, vtmp, vtmp + validity_tmp_words(n), c->p<uint8_t>(S_VBLOB), d_misc + 2, st);
-      launch_put_validity(d_dst + pos, pos, c->p<uint8_t>(S_VBLOB), d_misc + 2, d_misc + 3, st);
+      launch_put_validity(d_dst + head, head, c->p<uint8_t>(S_VBLOB), d_misc + 2, d_pos, st);
     }
-    uint64_t np = 0;
-    CK(read_small(c, st, &np, d_misc + 3, 8));
-    pos = np;
   }
-  uint64_t sub_cap = lane_bound(n_valid, n_valid, WT_U64, false, bs);
-  CK(c->ensure(S_LIMBOUT, sub_cap));
   for (int k = 0; k < nl; k++) {
     LaneJob j{limbs + (uint64_t)k * n_valid, n_valid, WT_U64, n_valid, nullptr, level, bs, plog2};
+    j.d_nest = d_pos;
     size_t sl = 0;
-    int rc = encode_lane(c, st, j, c->p<uint8_t>(S_LIMBOUT), sub_cap, &sl);
-    if (rc) return rc;
-    std::vector<uint8_t> vl;
-    put_varint_h(vl, sl);
-    if (pos + vl.size() + sl > dst_cap) {
+    int rc = encode_lane(c, st, j, d_dst, dst_cap, &sl);
+    if (rc) {
+      cudaStreamSynchronize(st);
       *out_len = need_bound;
-      return QUOIN_ERR_BUFFER_TOO_SMALL;
+      return rc;
     }
-    CK(cudaMemcpyAsync(d_dst + pos, vl.data(), vl.size(), cudaMemcpyHostToDevice, st));
-    CK(cudaMemcpyAsync(d_dst + pos + vl.size(), c->p<uint8_t>(S_LIMBOUT), sl, cudaMemcpyDeviceToDevice, st));
-    CK(cudaStreamSynchronize(st));
-    pos += vl.size() + sl;
   }
-  *out_len = pos;
+  uint64_t total = 0;
+  CK(read_small(c, st, &total, d_pos, 8));
+  resolve_timing();
+  if (total > dst_cap) {
+    *out_len = need_bound;
+    return QUOIN_ERR_BUFFER_TOO_SMALL;
+  }
+  *out_len = total;
   return QUOIN_OK;
 }
 

@@ -276,9 +276,22 @@ uint64_t ent_rec_bytes();
 // item, blk per block.
 uint64_t rd_rec_bytes();
 uint64_t blk_rec_bytes();
-// `base` (device) holds the byte offset at which the first frame starts.
-void launch_frame_offsets(FrameDesc* frames, const uint32_t* nb, uint32_t max_blocks, const uint64_t* base,
-                          uint64_t* sizes_tmp, uint64_t* tile_tmp, uint64_t* total, cudaStream_t st);
+struct Bytes16 {
+  uint8_t b[16];
+};
+// A lane stream inside a container (a decimal's limb): varint(length) and the
+// 16-byte header go to out at *pos (device), which moves past the stream.
+struct NestedLane {
+  uint64_t* pos = nullptr;
+  uint8_t* out = nullptr;
+  uint64_t cap = 0;
+  Bytes16 hdr;
+};
+// `base` (device) holds the byte offset at which the first frame starts (for a
+// nested lane it is written: the offset follows from the frames' sizes).
+void launch_frame_offsets(FrameDesc* frames, const uint32_t* nb, uint32_t max_blocks, uint64_t* base,
+                          uint64_t* sizes_tmp, uint64_t* tile_tmp, uint64_t* total, const NestedLane& nest,
+                          cudaStream_t st);
 // Emission: one or two CTAs per 32,768-value window of a frame; FoR / DELTA /
 // FLOAT_MULT / XORZ layouts are read from the statistics records of
 // launch_sub_stats, ALP-RD's and small dictionaries from rdr and blk.  Frames that would end past
@@ -294,8 +307,15 @@ void launch_emit(const uint64_t* lane, const FrameDesc* frames, const uint32_t* 
 void launch_lower(const void* values, int dtype, const uint8_t* bm, const uint64_t* word_rank, uint64_t n,
                   uint64_t* lane, cudaStream_t st);
 // Decimal: compacted limbs of (v - vmin).  `vmin` is computed on device.
-void launch_decimal_vmin(const uint8_t* values, int nlimbs, const uint8_t* bm, uint64_t n, uint64_t* vmin_tmp,
-                         uint64_t* vmin, cudaStream_t st);
+// (0 when no value is valid: any = false); vmin_tmp holds decimal_vmin_tmp_words().
+uint64_t decimal_vmin_tmp_words();
+void launch_decimal_vmin(const uint8_t* values, int nlimbs, const uint8_t* bm, uint64_t n, bool any,
+                         uint64_t* vmin_tmp, uint64_t* vmin, cudaStream_t st);
+struct Bytes19 {
+  uint8_t b[19];
+};
+void launch_put_decimal_header(uint8_t* dst, const Bytes19& head, int nl, const uint64_t* vmin, uint64_t* d_pos,
+                               cudaStream_t st);
 void launch_decimal_split(const uint8_t* values, int nlimbs, const uint8_t* bm, const uint64_t* word_rank,
                           uint64_t n, const uint64_t* vmin, uint64_t* limbs, uint64_t limb_stride, cudaStream_t st);
 // Validity run-length blob (reference validity.rs:40-70): the blob is written
@@ -327,9 +347,6 @@ void launch_write_bytes(uint8_t* dst, const uint8_t* src_dev, uint64_t len, cuda
 unsigned long long* device_win_counters();
 
 // Small writers used by the stream assembly.
-struct Bytes16 {
-  uint8_t b[16];
-};
 void launch_put_header(uint8_t* dst, Bytes16 hdr, uint64_t* d_base, cudaStream_t st);
 // Writes varint(*blob_len) ++ blob at dst and sets *d_base = dst_off + varint + blob.
 void launch_put_validity(uint8_t* dst, uint64_t dst_off, const uint8_t* blob, const uint64_t* blob_len,
