@@ -210,6 +210,21 @@ __device__ inline T warp_sum(T v) {
   for (int o = 16; o; o >>= 1) v += __shfl_xor_sync(0xffffffffu, v, o);
   return v;
 }
+// 64-bit minima and maxima by the warp's 32-bit reductions: the high words,
+// then the low words of the lanes that hold the extreme one.
+__device__ __forceinline__ uint64_t warp_min_u64(uint64_t v) {
+  const uint32_t hi = (uint32_t)(v >> 32), m = __reduce_min_sync(0xffffffffu, hi);
+  return (uint64_t)m << 32 | __reduce_min_sync(0xffffffffu, hi == m ? (uint32_t)v : 0xFFFFFFFFu);
+}
+__device__ __forceinline__ uint64_t warp_max_u64(uint64_t v) {
+  const uint32_t hi = (uint32_t)(v >> 32), m = __reduce_max_sync(0xffffffffu, hi);
+  return (uint64_t)m << 32 | __reduce_max_sync(0xffffffffu, hi == m ? (uint32_t)v : 0u);
+}
+constexpr uint64_t kSignBit = 0x8000000000000000ull;  // signed order as unsigned order
+template <>
+__device__ inline uint64_t warp_min<uint64_t>(uint64_t v) { return warp_min_u64(v); }
+template <>
+__device__ inline uint64_t warp_max<uint64_t>(uint64_t v) { return warp_max_u64(v); }
 __device__ inline uint32_t warp_and(uint32_t v) {
   for (int o = 16; o; o >>= 1) v &= __shfl_xor_sync(0xffffffffu, v, o);
   return v;

@@ -6,6 +6,8 @@
 // distinct/run counts, ALP (e,f) search, ALP-RD cut search), the argmin of
 // `len + penalty` is taken in the reference's candidate order with a strict
 // `<`, and only the winner is written by k_emit.
+#include <cooperative_groups.h>
+
 #include "qb_common.cuh"
 #include "qb_layout.h"
 #include "qb_kernels.h"
@@ -22,7 +24,7 @@ constexpr uint32_t kNoLb = 0xFFFFFFFFu;
 
 // 17-bit bucket of the dictionary cardinality lower-bound bitset.
 __device__ __forceinline__ uint32_t dict_lb_bucket(uint64_t x) {
-  return (uint32_t)((x * 0xD6E8FEB86659FD93ull) >> (64 - 17));
+  return ((uint32_t)x * 0x9E3779B1u + (uint32_t)(x >> 32) * 0x85EBCA77u) >> (32 - 17);
 }
 constexpr uint64_t kEmpty64 = ~0ull;
 constexpr uint32_t kEmpty32 = 0xFFFFFFFFu;
@@ -76,14 +78,8 @@ __device__ inline uint64_t warp_or64(uint64_t v) {
   for (int o = 16; o; o >>= 1) v |= __shfl_xor_sync(0xffffffffu, v, o);
   return v;
 }
-__device__ inline int64_t warp_min_i64(int64_t v) {
-  for (int o = 16; o; o >>= 1) { int64_t u = __shfl_xor_sync(0xffffffffu, v, o); v = u < v ? u : v; }
-  return v;
-}
-__device__ inline int64_t warp_max_i64(int64_t v) {
-  for (int o = 16; o; o >>= 1) { int64_t u = __shfl_xor_sync(0xffffffffu, v, o); v = u > v ? u : v; }
-  return v;
-}
+__device__ inline int64_t warp_min_i64(int64_t v) { return (int64_t)(warp_min_u64((uint64_t)v ^ kSignBit) ^ kSignBit); }
+__device__ inline int64_t warp_max_i64(int64_t v) { return (int64_t)(warp_max_u64((uint64_t)v ^ kSignBit) ^ kSignBit); }
 __device__ inline uint32_t pow2_at_least(uint32_t x) {
   uint32_t p = 1;
   while (p < x) p <<= 1;
@@ -117,21 +113,6 @@ __device__ inline void alp_combo(uint32_t c, int* e, int* f) {
   *f = (int)(c - (uint32_t)(ee * (ee + 1) / 2));
 }
 
-// FLOAT_MULT scale test (reference codecs/float_mult.rs:45-64): bit s set in
-// the result when value x does NOT round-trip exactly through scale s.
-__device__ inline uint32_t fm_fail_bits(uint64_t x, uint32_t alive) {
-  uint32_t fail = 0;
-  double xd = as_f64(x);
-  while (alive) {
-    int s = __ffs(alive) - 1;
-    alive &= alive - 1;
-    double sc = kFmScales[s];
-    double k = round_half_away(__dmul_rn(xd, sc));
-    bool ok = is_finite_f64(k) && fabs(k) < 9.0e18 && f64_bits(__ddiv_rn(k, sc)) == x;
-    if (!ok) fail |= 1u << s;
-  }
-  return fail;
-}
 __device__ inline int64_t fm_k(uint64_t x, int s) {
   return __double2ll_rz(round_half_away(__dmul_rn(as_f64(x), kFmScales[s])));
 }
@@ -1884,7 +1865,10 @@ struct FmStat {  // signed min / max of k = round(x * scale) per FLOAT_MULT scal
   int64_t kmin[7], kmax[7];
 };
 
-constexpr int kStatsWarps = 32;  // one CTA per 32768-value window in adaptive mode
+// Adaptive mode: a cluster of four CTAs of eight warps per 32,768-value window,
+// so that a column of few windows runs on four times as many SMs.
+constexpr int kStatsWarps = 8, kStatsCluster = 4;
+static_assert(kStatsWarps * kStatsCluster * kSub == kBaseQuantum, "a cluster covers a window");
 
 // Start and length of statistics item `item` (one 1024-value sub-block): with
 // a fixed block size the sub-blocks restart at every block boundary.
@@ -1932,23 +1916,186 @@ __global__ void __launch_bounds__(kAlpWarps * 32) k_alp_stats(const uint64_t* __
   }
 }
 
+// A lane's share of a sub-block's statistics.
+struct StatAcc {
+  uint64_t umn = kEmpty64, umx = 0, dzmn = kEmpty64, dzmx = 0;
+  int64_t smn = INT64_MAX, smx = INT64_MIN;
+  uint32_t nq = 0, xb = 0, fmfail = 0;
+  int64_t kmn[7], kmx[7];
+};
+// FLOAT_MULT's scales still alive on value x: the failing ones' bits set, the
+// others' digit ranges widened (float_mult.rs:45-64).
+__device__ __forceinline__ void fm_value(uint64_t x, uint32_t alive, StatAcc& A) {
+  double xd = as_f64(x);
+  while (alive) {
+    int q = __ffs(alive) - 1;
+    alive &= alive - 1;
+    double sc = kFmScales[q];
+    double k = round_half_away(__dmul_rn(xd, sc));
+    bool good = is_finite_f64(k) && fabs(k) < 9.0e18 && f64_bits(__ddiv_rn(k, sc)) == x;
+    if (!good) {
+      A.fmfail |= 1u << q;
+    } else {
+      int64_t ki = __double2ll_rz(k);
+#pragma unroll
+      for (int j = 0; j < 7; j++)
+        if (j == q) {
+          A.kmn[j] = ki < A.kmn[j] ? ki : A.kmn[j];
+          A.kmx[j] = ki > A.kmx[j] ? ki : A.kmx[j];
+        }
+    }
+  }
+}
+// LEB128 bytes of v, with one leading-zero count.
+__device__ __forceinline__ uint32_t leb_len(uint32_t lo, uint32_t hi) {
+  const uint32_t h = hi ? hi : lo | 1u;
+  const uint32_t bits = (hi ? 64u : 32u) - __clz(h);
+  return (bits + 6) * 37 >> 8;  // (bits + 6) / 7 for bits <= 64
+}
+
+// A whole sub-block's rows.  KIND: 0 u64 lane, 1 i64, 2 i32, 3 u32, 4 floats.
+// Issue slots bound this pass (59 % busy, the integer pipe 52 %; 122 a row of
+// 32 values and 350 us for 60,000,000 values before, now 96 and 267 us), so it
+// carries no per-value test: value 0's predecessor is chosen to
+// repeat the first delta (its XOR bytes and transition are taken off at the
+// end), the signed kinds derive the unsigned range unless a sub-block mixes
+// signs (then a second pass over its values, in L1), 4-byte columns compare
+// 32-bit words.
+template <int KIND, bool LB>
+__device__ __forceinline__ void stats_rows(const uint64_t* __restrict__ sv, uint32_t* lbits, uint32_t alive,
+                                           StatAcc& A) {
+  const int lane = threadIdx.x & 31;
+  constexpr bool W32 = KIND == 2 || KIND == 3;
+  const uint64_t x0 = sv[0], d0 = sv[1] - x0;
+  uint64_t carry = x0 - d0;
+  uint32_t umn32 = 0xFFFFFFFFu, umx32 = 0;
+  int32_t smn32 = INT32_MAX, smx32 = INT32_MIN;
+  for (uint32_t r0 = 0; r0 < 32; r0 += 8) {
+    uint64_t xs[8];  // eight independent loads in flight per lane
+#pragma unroll
+    for (int q = 0; q < 8; q++) xs[q] = sv[(r0 + q) * 32 + lane];
+#pragma unroll
+    for (int q = 0; q < 8; q++) {
+      const uint64_t x = xs[q];
+      uint64_t pv;
+      if (W32) {
+        const uint32_t rot = __shfl_sync(0xffffffffu, (uint32_t)x, (lane + 31) & 31);
+        const uint64_t r64 = KIND == 2 ? (uint64_t)(int64_t)(int32_t)rot : (uint64_t)rot;
+        pv = lane ? r64 : carry;
+        carry = r64;
+      } else {
+        const uint64_t rot = __shfl_sync(0xffffffffu, x, (lane + 31) & 31);
+        pv = lane ? rot : carry;
+        carry = rot;
+      }
+      if (W32) {
+        umn32 = min(umn32, (uint32_t)x);
+        umx32 = max(umx32, (uint32_t)x);
+        if (KIND == 2) {
+          smn32 = min(smn32, (int32_t)(uint32_t)x);
+          smx32 = max(smx32, (int32_t)(uint32_t)x);
+        }
+      } else if (KIND == 1) {
+        A.smn = (int64_t)x < A.smn ? (int64_t)x : A.smn;
+        A.smx = (int64_t)x > A.smx ? (int64_t)x : A.smx;
+      } else {
+        A.umn = u64min(A.umn, x);
+        A.umx = u64max(A.umx, x);
+      }
+      const uint64_t dz = zigzag64(x - pv), xo = x ^ pv;
+      A.dzmn = u64min(A.dzmn, dz);
+      A.dzmx = u64max(A.dzmx, dz);
+      A.xb += leb_len((uint32_t)xo, (uint32_t)(xo >> 32));
+      if (xo) {
+        A.nq++;
+        if (LB) {  // a repeat's bucket is already set
+          const uint32_t b = dict_lb_bucket(x);
+          atomicOr(&lbits[b >> 5], 1u << (b & 31));
+        }
+      }
+      if (KIND == 4 && alive) {
+        fm_value(x, alive, A);
+        alive &= ~__reduce_or_sync(0xffffffffu, A.fmfail);  // a scale that failed anywhere in the sub-block is out
+      }
+    }
+  }
+  if (lane == 0) {
+    const uint64_t xo = x0 ^ (x0 - d0);
+    A.xb -= leb_len((uint32_t)xo, (uint32_t)(xo >> 32));
+    if (xo) A.nq--;
+    if (LB) {
+      const uint32_t b = dict_lb_bucket(x0);
+      atomicOr(&lbits[b >> 5], 1u << (b & 31));
+    }
+  }
+  if (KIND == 2) {
+    A.smn = smn32;
+    A.smx = smx32;
+    A.umn = (uint64_t)(int64_t)(int32_t)umn32;  // sign extension keeps the unsigned order
+    A.umx = (uint64_t)(int64_t)(int32_t)umx32;
+  } else if (KIND == 3) {
+    A.umn = umn32;
+    A.umx = umx32;
+  } else if (KIND == 1) {
+    if (__any_sync(0xffffffffu, A.smn < 0) && __any_sync(0xffffffffu, A.smx >= 0)) {
+      for (uint32_t r = 0; r < 32; r++) {
+        const uint64_t x = sv[r * 32 + lane];
+        A.umn = u64min(A.umn, x);
+        A.umx = u64max(A.umx, x);
+      }
+    } else {
+      A.umn = (uint64_t)A.smn;
+      A.umx = (uint64_t)A.smx;
+    }
+  }
+}
+// The rows of a sub-block of fewer than 1,024 values.
+__device__ __noinline__ void stats_partial(const uint64_t* __restrict__ sv, uint32_t cnt, bool lb, uint32_t* lbits,
+                                           uint32_t alive, StatAcc& A) {
+  const int lane = threadIdx.x & 31;
+  for (uint32_t j0 = 0; j0 < cnt; j0 += 32) {
+    const uint32_t j = j0 + lane;
+    if (j < cnt) {
+      const uint64_t x = sv[j], pv = j ? sv[j - 1] : x;
+      A.umn = u64min(A.umn, x);
+      A.umx = u64max(A.umx, x);
+      A.smn = (int64_t)x < A.smn ? (int64_t)x : A.smn;
+      A.smx = (int64_t)x > A.smx ? (int64_t)x : A.smx;
+      if (j > 0) {
+        const uint64_t dz = zigzag64(x - pv);
+        A.dzmn = u64min(A.dzmn, dz);
+        A.dzmx = u64max(A.dzmx, dz);
+        A.xb += varint_len(x ^ pv);
+        A.nq += x != pv ? 1u : 0u;
+      }
+      if (lb) {
+        const uint32_t b = dict_lb_bucket(x);
+        atomicOr(&lbits[b >> 5], 1u << (b & 31));
+      }
+      if (alive) fm_value(x, alive, A);
+    }
+    if (alive) alive &= ~__reduce_or_sync(0xffffffffu, A.fmfail);
+  }
+}
+
 template <bool FLOATS>
-__global__ void __launch_bounds__(kStatsWarps * 32) k_sub_stats(
-    const uint64_t* __restrict__ v, uint64_t n, uint64_t fixed_bs, int dtype, int level,
+__global__ void __cluster_dims__(kStatsCluster, 1, 1) __launch_bounds__(kStatsWarps * 32, FLOATS ? 3 : 5) k_sub_stats(
+    const uint64_t* __restrict__ v, uint64_t n, uint64_t fixed_bs, uint64_t items, int dtype, int level,
     SubStats* __restrict__ ss, FmStat* __restrict__ fms, uint64_t* __restrict__ smp16, uint8_t* __restrict__ grow,
     uint32_t* __restrict__ winbits) {
   __shared__ uint32_t bitsA[512], bitsB[512];
-  __shared__ uint32_t lbits[kLbBits / 32];  // dictionary cardinality lower bound (window)
-  __shared__ uint32_t s_lbc;
+  __shared__ uint32_t lbits[kLbBits / 32];  // dictionary cardinality lower bound (the CTA's share of the window)
+  __shared__ uint32_t s_lbc, s_dc;
   __shared__ uint64_t s_first[kStatsWarps], s_last[kStatsWarps];
   __shared__ uint32_t s_neq[kStatsWarps], s_cnt[kStatsWarps];
   int lane = threadIdx.x & 31, warp = threadIdx.x >> 5;
   const bool do_float = FLOATS && level >= 1;
   uint64_t item = (uint64_t)blockIdx.x * kStatsWarps + warp;
-  uint64_t s;
-  uint32_t cnt = sub_range(item, n, fixed_bs, &s);
+  const uint64_t win = blockIdx.x / kStatsCluster;
+  uint64_t s = 0;
+  uint32_t cnt = item < items ? sub_range(item, n, fixed_bs, &s) : 0u;
   // window probe sampling (adaptive): window-relative stride max(len/4096, 1)
-  uint64_t wstart = (uint64_t)blockIdx.x * kBaseQuantum;
+  uint64_t wstart = win * kBaseQuantum;
   uint32_t wlen = fixed_bs ? 0u : (uint32_t)(wstart < n ? qmin(kBaseQuantum, n - wstart) : 0);
   uint32_t wstride = max(wlen / 4096u, 1u);
   const bool sgn = dtype_signed(dtype);
@@ -1958,99 +2105,56 @@ __global__ void __launch_bounds__(kStatsWarps * 32) k_sub_stats(
       bitsB[i] = 0;
     }
     for (int i = threadIdx.x; i < (int)(kLbBits / 32); i += blockDim.x) lbits[i] = 0;
-    if (threadIdx.x == 0) s_lbc = 0;
+    if (threadIdx.x == 0) s_lbc = s_dc = 0;
     __syncthreads();
   }
   SubStats R;
-  uint64_t umn = kEmpty64, umx = 0, dzmn = kEmpty64, dzmx = 0;
-  int64_t smn = INT64_MAX, smx = INT64_MIN;
-  uint64_t a16mn = kEmpty64, a16mx = 0, a16dz = 0, a64mn = kEmpty64, a64mx = 0, a64dz = 0;
-  uint32_t nq = 0, xb = 0, fmfail = 0;
-  int64_t kmn[7], kmx[7];
+  StatAcc A;
 #pragma unroll
   for (int q = 0; q < 7; q++) {
-    kmn[q] = INT64_MAX;
-    kmx[q] = INT64_MIN;
+    A.kmn[q] = INT64_MAX;
+    A.kmx[q] = INT64_MIN;
   }
   const uint64_t* sv = v + s;
   uint64_t d = cnt >= 2 ? sv[1] - sv[0] : 0;
-  uint32_t alive = do_float ? 0x7Fu : 0u;
-  uint64_t carry = 0;
-  for (uint32_t r0 = 0; r0 < 32; r0 += 8) {
-    uint64_t xs[8];  // eight independent loads in flight per lane
-#pragma unroll
-    for (int q = 0; q < 8; q++) {
-      uint32_t jq = (r0 + q) * 32 + lane;
-      xs[q] = jq < cnt ? sv[jq] : 0ull;
-    }
-#pragma unroll
-    for (int q = 0; q < 8; q++) {
-    uint32_t r = r0 + q;
-    uint32_t j = r * 32 + lane;
-    bool ok = j < cnt;
-    uint64_t x = xs[q];
-    // one rotation gives every lane its predecessor; lane 0's is the previous
-    // row's last value, which the rotation hands it for the next row
-    uint64_t rot = __shfl_sync(0xffffffffu, x, (lane + 31) & 31);
-    uint64_t pv = lane ? rot : carry;
-    carry = rot;
-    if (ok) {
-      umn = u64min(umn, x);
-      umx = u64max(umx, x);
-      if (sgn) {
-        int64_t sx = (int64_t)x;
-        smn = sx < smn ? sx : smn;
-        smx = sx > smx ? sx : smx;
-      }
-      if (j > 0) {
-        uint64_t dz = zigzag64(x - pv);
-        dzmn = u64min(dzmn, dz);
-        dzmx = u64max(dzmx, dz);
-        xb += varint_len(x ^ pv);
-        nq += x != pv ? 1u : 0u;
-      }
-      if (!fixed_bs) {
-        if (j == 0 || x != pv) {  // a repeat's bucket is already set
-          uint32_t lb17 = dict_lb_bucket(x);
-          atomicOr(&lbits[lb17 >> 5], 1u << (lb17 & 31));
-        }
-      }
-      if (FLOATS && alive) {
-        double xd = as_f64(x);
-        uint32_t a2 = alive;
-        while (a2) {
-          int q = __ffs(a2) - 1;
-          a2 &= a2 - 1;
-          double sc = kFmScales[q];
-          double k = round_half_away(__dmul_rn(xd, sc));
-          bool good = is_finite_f64(k) && fabs(k) < 9.0e18 && f64_bits(__ddiv_rn(k, sc)) == x;
-          if (!good) {
-            fmfail |= 1u << q;
-          } else {
-            int64_t ki = __double2ll_rz(k);
-            kmn[q] = ki < kmn[q] ? ki : kmn[q];
-            kmx[q] = ki > kmx[q] ? ki : kmx[q];
-          }
-        }
-      }
-    }
-    // a scale that failed anywhere in the sub-block is out: stop trying it
-    if (FLOATS && alive) alive &= ~warp_or(fmfail);
-    }
+  const uint32_t alive = do_float ? 0x7Fu : 0u;
+  if (cnt < (uint32_t)kSub) {
+    stats_partial(sv, cnt, !fixed_bs, lbits, alive, A);
+  } else if (FLOATS) {
+    if (fixed_bs) stats_rows<4, false>(sv, lbits, alive, A);
+    else stats_rows<4, true>(sv, lbits, alive, A);
+  } else if (dtype == DT_I64) {
+    if (fixed_bs) stats_rows<1, false>(sv, lbits, 0, A);
+    else stats_rows<1, true>(sv, lbits, 0, A);
+  } else if (dtype == DT_I32) {
+    if (fixed_bs) stats_rows<2, false>(sv, lbits, 0, A);
+    else stats_rows<2, true>(sv, lbits, 0, A);
+  } else if (dtype == DT_U32) {
+    if (fixed_bs) stats_rows<3, false>(sv, lbits, 0, A);
+    else stats_rows<3, true>(sv, lbits, 0, A);
+  } else {
+    if (fixed_bs) stats_rows<0, false>(sv, lbits, 0, A);
+    else stats_rows<0, true>(sv, lbits, 0, A);
   }
   // Sampled statistics, kept out of the per-value loop (only a few lanes of a
-  // row would take them): early-out samples at j % 16 / j % 64 == 0 and the
-  // window probe samples (stride wstride, and stride 32).
-  for (uint32_t j = 16u * lane; j < cnt; j += 512) {
-    uint64_t x = sv[j], pv = j ? sv[j - 1] : 0ull;
-    a16mn = u64min(a16mn, x);
-    a16mx = u64max(a16mx, x);
-    if (j > 0) a16dz = u64max(a16dz, zigzag64(x - pv));
-    if (smp16 && !fixed_bs) smp16[(s + j) >> 4] = x;
-    if ((j & 63) == 0) {
-      a64mn = u64min(a64mn, x);
-      a64mx = u64max(a64mx, x);
-      if (j > 0) a64dz = u64max(a64dz, zigzag64(x - pv));
+  // row would take them): early-out samples at j % 16 / j % 64 == 0 (integer
+  // lanes), the ALP-RD sample (float lanes) and the window probe samples
+  // (stride wstride, and stride 32).
+  uint64_t a16mn = kEmpty64, a16mx = 0, a16dz = 0, a64mn = kEmpty64, a64mx = 0, a64dz = 0;
+  if (FLOATS) {
+    if (smp16 && !fixed_bs)
+      for (uint32_t j = 16u * lane; j < cnt; j += 512) smp16[(s + j) >> 4] = sv[j];
+  } else {
+    for (uint32_t j = 16u * lane; j < cnt; j += 512) {
+      uint64_t x = sv[j], pv = j ? sv[j - 1] : 0ull;
+      a16mn = u64min(a16mn, x);
+      a16mx = u64max(a16mx, x);
+      if (j > 0) a16dz = u64max(a16dz, zigzag64(x - pv));
+      if ((j & 63) == 0) {
+        a64mn = u64min(a64mn, x);
+        a64mx = u64max(a64mx, x);
+        if (j > 0) a64dz = u64max(a64dz, zigzag64(x - pv));
+      }
     }
   }
   if (!fixed_bs && cnt) {
@@ -2065,36 +2169,40 @@ __global__ void __launch_bounds__(kStatsWarps * 32) k_sub_stats(
       atomicOr(&bitsB[bk >> 5], 1u << (bk & 31));
     }
   }
-  R.umin = warp_min(umn);
-  R.umax = warp_max(umx);
-  R.smin = warp_min_i64(smn);
-  R.smax = warp_max_i64(smx);
-  R.dzmin = warp_min(dzmn);
-  R.dzmax = warp_max(dzmx);
-  R.e16min = warp_min(a16mn);
-  R.e16max = warp_max(a16mx);
-  R.e16dz = warp_max(a16dz);
-  R.e64min = warp_min(a64mn);
-  R.e64max = warp_max(a64mx);
-  R.e64dz = warp_max(a64dz);
-  R.xb = warp_sum(xb);
-  R.neq = warp_sum(nq);
+  R.umin = warp_min(A.umn);
+  R.umax = warp_max(A.umx);
+  R.smin = sgn ? warp_min_i64(A.smn) : 0;
+  R.smax = sgn ? warp_max_i64(A.smx) : 0;
+  R.dzmin = warp_min(A.dzmn);
+  R.dzmax = warp_max(A.dzmx);
+  R.e16min = R.e16max = R.e16dz = R.e64min = R.e64max = R.e64dz = 0;
+  if (!FLOATS) {
+    R.e16min = warp_min(a16mn);
+    R.e16max = warp_max(a16mx);
+    R.e16dz = warp_max(a16dz);
+    R.e64min = warp_min(a64mn);
+    R.e64max = warp_max(a64mx);
+    R.e64dz = warp_max(a64dz);
+  }
+  R.xb = __reduce_add_sync(0xffffffffu, A.xb);
+  R.neq = __reduce_add_sync(0xffffffffu, A.nq);
   // every internal delta equals d exactly when the zigzag deltas are all zigzag(d)
   R.stride_ok = (cnt < 2 || (R.dzmin == R.dzmax && R.dzmax == zigzag64(d))) ? 1 : 0;
   R.cnt = cnt;
   R.first = cnt ? sv[0] : 0;
   R.last = cnt ? sv[cnt - 1] : 0;
   R.d = d;
-  R.fm_pass = do_float ? (uint8_t)(0x7Fu & ~warp_or(fmfail)) : 0;
+  R.fm_pass = do_float ? (uint8_t)(0x7Fu & ~__reduce_or_sync(0xffffffffu, A.fmfail)) : 0;
   R.alp_ok = 0;
   R.alp_w = 0;
   R.alp_exc = 0;
   R.pad16 = 0;
   R.pad32 = 0;
-  if (FLOATS && do_float) {
+  if (FLOATS && do_float && item < items) {
 #pragma unroll
     for (int q = 0; q < 7; q++) {
-      int64_t a = warp_min_i64(kmn[q]), b = warp_max_i64(kmx[q]);
+      if (!(R.fm_pass >> q & 1)) continue;  // only a passing scale's range is read
+      int64_t a = warp_min_i64(A.kmn[q]), b = warp_max_i64(A.kmx[q]);
       if (lane == 0) {
         fms[item].kmin[q] = a;
         fms[item].kmax[q] = b;
@@ -2102,7 +2210,7 @@ __global__ void __launch_bounds__(kStatsWarps * 32) k_sub_stats(
     }
   }
   if (lane == 0) {
-    ss[item] = R;
+    if (item < items) ss[item] = R;
     s_first[warp] = R.first;
     s_last[warp] = R.last;
     s_neq[warp] = R.neq;
@@ -2112,33 +2220,54 @@ __global__ void __launch_bounds__(kStatsWarps * 32) k_sub_stats(
   // Window probe (reference encoder.rs:166-176, 705-750): grow the block at
   // this window when the sampled distinct count is low or most consecutive
   // values repeat.  consec_eq = len - transitions (the first element counts
-  // against itself).
-  __syncthreads();
+  // against itself).  Each CTA of the cluster joins a quarter of the bitsets;
+  // the first takes the counts.
+  namespace cg = cooperative_groups;
+  cg::cluster_group cl = cg::this_cluster();
+  cl.sync();
+  const uint32_t rank = cl.block_rank();
   {
-    uint32_t c = 0;
-    for (int i = threadIdx.x; i < (int)(kLbBits / 32); i += blockDim.x) c += __popc(lbits[i]);
-    c = warp_sum(c);
-    if (lane == 0 && c) atomicAdd(&s_lbc, c);
+    uint32_t c = 0, dc = 0;
+    const uint32_t *lb[kStatsCluster], *ba[kStatsCluster], *bb[kStatsCluster];
+#pragma unroll
+    for (int k = 0; k < kStatsCluster; k++) {
+      lb[k] = cl.map_shared_rank(lbits, k);
+      ba[k] = cl.map_shared_rank(bitsA, k);
+      bb[k] = cl.map_shared_rank(bitsB, k);
+    }
+    constexpr uint32_t kLbPart = kLbBits / 32 / kStatsCluster, kBitPart = 512 / kStatsCluster;
+    for (uint32_t i = rank * kLbPart + threadIdx.x; i < (rank + 1) * kLbPart; i += blockDim.x)
+      c += __popc(lb[0][i] | lb[1][i] | lb[2][i] | lb[3][i]);
+    for (uint32_t i = rank * kBitPart + threadIdx.x; i < (rank + 1) * kBitPart; i += blockDim.x) {
+      const uint32_t x = ba[0][i] | ba[1][i] | ba[2][i] | ba[3][i], y = bb[0][i] | bb[1][i] | bb[2][i] | bb[3][i];
+      dc += __popc(x);
+      winbits[win * kWinWords + i] = x;
+      winbits[win * kWinWords + 512 + i] = y;
+    }
+    static_assert(kStatsCluster == 4, "four shares are joined");
+    c = __reduce_add_sync(0xffffffffu, c);
+    dc = __reduce_add_sync(0xffffffffu, dc);
+    if (lane == 0 && c) atomicAdd(cl.map_shared_rank(&s_lbc, 0), c);
+    if (lane == 0 && dc) atomicAdd(cl.map_shared_rank(&s_dc, 0), dc);
   }
-  __syncthreads();
-  if (threadIdx.x == 0) winbits[(uint64_t)blockIdx.x * kWinWords + 1024] = s_lbc;
-  if (warp == 0 && wlen) {
-    uint32_t dc = 0;
-    for (int i = lane; i < 512; i += 32) dc += __popc(bitsA[i]);
-    dc = warp_sum(dc);
-    uint32_t tr = 0;
-    if (lane < kStatsWarps && s_cnt[lane]) {
-      tr = s_neq[lane];
-      if (lane > 0 && s_first[lane] != s_last[lane - 1]) tr++;
+  uint32_t tr = 0;
+  if (rank == 0 && warp == 0) {  // a lane per sub-block of the window
+    const int k = lane / kStatsWarps, w = lane % kStatsWarps;
+    if (cl.map_shared_rank(s_cnt, k)[w]) {
+      tr = cl.map_shared_rank(s_neq, k)[w];
+      const uint64_t f = cl.map_shared_rank(s_first, k)[w];
+      if (lane > 0 && f != (w ? cl.map_shared_rank(s_last, k)[w - 1]
+                              : cl.map_shared_rank(s_last, k - 1)[kStatsWarps - 1]))
+        tr++;
     }
-    tr = warp_sum(tr);
-    if (lane == 0) {
+    tr = __reduce_add_sync(0xffffffffu, tr);
+  }
+  cl.sync();  // the counts are in, and no CTA's shared memory is read any more
+  if (rank == 0 && threadIdx.x == 0) {
+    winbits[win * kWinWords + 1024] = s_lbc;
+    if (wlen) {
       uint32_t consec = wlen - tr;
-      grow[blockIdx.x] = (dc < 2048 || (uint64_t)consec * 2 > wlen) ? 1 : 0;
-    }
-    for (int i = lane; i < 512; i += 32) {
-      winbits[(uint64_t)blockIdx.x * kWinWords + i] = bitsA[i];
-      winbits[(uint64_t)blockIdx.x * kWinWords + 512 + i] = bitsB[i];
+      grow[win] = (s_dc < 2048 || (uint64_t)consec * 2 > wlen) ? 1 : 0;
     }
   }
 }
@@ -3542,7 +3671,7 @@ void launch_plan(const uint8_t* grow, uint64_t n, uint64_t fixed_bs, FrameDesc* 
 
 uint64_t sub_stats_items(uint64_t n, uint64_t fixed_bs) {
   if (fixed_bs) return ((n + fixed_bs - 1) / fixed_bs) * ((fixed_bs + kSub - 1) / kSub);
-  return ((n + kBaseQuantum - 1) / kBaseQuantum) * (uint64_t)kStatsWarps;
+  return ((n + kBaseQuantum - 1) / kBaseQuantum) * (uint64_t)(kBaseQuantum / kSub);
 }
 uint64_t sub_stats_bytes() { return sizeof(SubStats); }
 uint64_t fm_stats_bytes() { return sizeof(FmStat); }
@@ -3550,10 +3679,11 @@ uint64_t fm_stats_bytes() { return sizeof(FmStat); }
 void launch_sub_stats(const uint64_t* lane, uint64_t n, uint64_t fixed_bs, int dtype, int level, void* ss, void* fms,
                       uint64_t* smp16, uint8_t* grow, uint32_t* winbits, cudaStream_t st) {
   uint64_t items = sub_stats_items(n, fixed_bs);
-  unsigned g = (unsigned)((items + kStatsWarps - 1) / kStatsWarps);
-  if (!g) return;
+  if (!items) return;
+  const uint64_t per = kStatsWarps * kStatsCluster;
+  const unsigned g = (unsigned)((items + per - 1) / per * kStatsCluster);
   if (dtype_float(dtype)) {
-    k_sub_stats<true><<<g, kStatsWarps * 32, 0, st>>>(lane, n, fixed_bs, dtype, level, (SubStats*)ss, (FmStat*)fms,
+    k_sub_stats<true><<<g, kStatsWarps * 32, 0, st>>>(lane, n, fixed_bs, items, dtype, level, (SubStats*)ss, (FmStat*)fms,
                                                        smp16, grow, winbits);
     if (level >= 1) {
       k_alp_stats<<<(unsigned)((items + kAlpWarps - 1) / kAlpWarps), kAlpWarps * 32, 0, st>>>(lane, n, fixed_bs, items,
@@ -3561,7 +3691,7 @@ void launch_sub_stats(const uint64_t* lane, uint64_t n, uint64_t fixed_bs, int d
       count_launches(1);
     }
   } else
-    k_sub_stats<false><<<g, kStatsWarps * 32, 0, st>>>(lane, n, fixed_bs, dtype, level, (SubStats*)ss,
+    k_sub_stats<false><<<g, kStatsWarps * 32, 0, st>>>(lane, n, fixed_bs, items, dtype, level, (SubStats*)ss,
                                                         (FmStat*)fms, nullptr, grow, winbits);
   count_launches(1);
 }
