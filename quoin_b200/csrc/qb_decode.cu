@@ -170,7 +170,7 @@ __global__ void __launch_bounds__(kWalkWarps * 32) k_walk_frames(const uint8_t* 
         if (!scratch) { e = E_UNSUPPORTED; break; }
         uint32_t* offs = reinterpret_cast<uint32_t*>(scratch + d.value_off);  // nexc <= n of them
         uint64_t prev = ~0ull;  // the position before the group's first (~0: none)
-        e = warp_exc_walk(p, plen, &pos, nexc, [&](bool act, uint64_t x, uint64_t q, uint64_t v) {
+        e = warp_exc_walk<true>(p, plen, &pos, nexc, [&](bool act, uint64_t x, uint64_t q, uint64_t v) {
           if (act) offs[x] = (uint32_t)q;
           uint64_t before = __shfl_up_sync(0xffffffffu, v, 1);
           if (l == 0) before = prev;
@@ -1691,10 +1691,11 @@ __global__ void __launch_bounds__(kDecThreads) k_decode_frames(const uint8_t* __
                                                               DecodeOut O, uint64_t* __restrict__ scratch,
                                                               unsigned long long* __restrict__ err,
                                                               const uint32_t* __restrict__ list,
-                                                              uint8_t* __restrict__ ent, BatchView bv) {
+                                                              uint8_t* __restrict__ ent, const DpLaneOut* dyn,
+                                                              BatchView bv) {
   extern __shared__ __align__(16) uint8_t smem_raw[];
   DecSmem& S = *reinterpret_cast<DecSmem*>(smem_raw);
-  if ((int)blockIdx.x >= nf) return;
+  if ((int)blockIdx.x >= (dyn ? (int)dyn->nlist : nf)) return;
   int f = list ? (int)list[blockIdx.x] : (int)blockIdx.x;
   if (bv.cols) {  // a batch: the frame's column decides the output
     const BatchCol& C = bv.cols[bv.frame_col[f]];
@@ -1702,6 +1703,7 @@ __global__ void __launch_bounds__(kDecThreads) k_decode_frames(const uint8_t* __
     dtype = C.dtype;
     scratch = C.scratch;
   }
+  if (O.d_nvalid) O.nvalid = *O.d_nvalid;
   const FrameAux& A = aux[f];
   if (A.err) return;
   FrameDesc d = frames[f];
@@ -1964,9 +1966,11 @@ __global__ void __launch_bounds__(kDecThreads) k_dict_values(const uint8_t* __re
                                                             const FrameDesc* __restrict__ frames,
                                                             const FrameAux* __restrict__ aux,
                                                             uint64_t* __restrict__ scratch,
-                                                            const uint32_t* __restrict__ list, BatchView bv) {
+                                                            const uint32_t* __restrict__ list, const DpLaneOut* dyn,
+                                                            BatchView bv) {
   extern __shared__ __align__(16) uint8_t smem_raw[];
   DecSmem& S = *reinterpret_cast<DecSmem*>(smem_raw);
+  if (dyn && blockIdx.x >= dyn->nlist) return;
   int f = (int)list[blockIdx.x];
   FrameDesc d = frames[f];
   if (d.mode != M_DICT) return;
@@ -2451,12 +2455,12 @@ __global__ void __launch_bounds__(kItemWarps * 32, 6) k_prepass(const uint8_t* _
                                                            const FrameAux* __restrict__ aux,
                                                            const ItemRef* __restrict__ items, uint32_t nitems,
                                                            PreRec* __restrict__ pre, uint64_t* __restrict__ scratch,
-                                                           BatchView bv) {
+                                                           const DpLaneOut* dyn, BatchView bv) {
   __shared__ __align__(16) uint32_t rle_stage[kItemWarps][kSub];  // XORZ: the round's byte buffer
   static_assert(kSub * 4 >= kXorzBufWords * 8, "the XORZ buffer fits a warp's stage");
   uint32_t g = blockIdx.x * kItemWarps + (threadIdx.x >> 5);
   int l = threadIdx.x & 31;
-  if (g >= nitems) return;
+  if (g >= (dyn ? dyn->npre : nitems)) return;
   ItemRef it = items[g];
   const FrameAux& A = aux[it.frame];
   if (A.err) return;
@@ -2597,12 +2601,13 @@ __global__ void __launch_bounds__(kItemWarps * 32, QB_ITEM_MIN_BLOCKS) k_decode_
                                                                 const uint2* __restrict__ frame_pre,
                                                                 const PreRec* __restrict__ pre, DecodeOut O,
                                                                 const uint64_t* __restrict__ scratch,
-                                                                unsigned long long* __restrict__ err, BatchView bv) {
+                                                                unsigned long long* __restrict__ err,
+                                                                const DpLaneOut* dyn, BatchView bv) {
   __shared__ __align__(16) uint64_t stage_all[kItemWarps][kItemStage];
   __shared__ __align__(16) uint64_t xbuf_all[kItemWarps][kXorzBufWords];  // XORZ rounds' bytes
   int warp = threadIdx.x >> 5, l = threadIdx.x & 31;
   uint32_t g = blockIdx.x * kItemWarps + warp;
-  if (g >= nitems) return;
+  if (g >= (dyn ? dyn->nmain : nitems)) return;
   ItemRef it = items[g];
   const FrameAux& A = aux[it.frame];
   if (A.err) return;
@@ -2613,6 +2618,7 @@ __global__ void __launch_bounds__(kItemWarps * 32, QB_ITEM_MIN_BLOCKS) k_decode_
     dtype = C.dtype;
     scratch = C.scratch;
   }
+  if (O.d_nvalid) O.nvalid = *O.d_nvalid;
   const uint8_t* p = stream + d.payload_off;
   uint64_t n = d.n;
   uint64_t* stg = stage_all[warp];
@@ -2973,7 +2979,7 @@ void launch_decode_frames(const uint8_t* stream, const FrameDesc* frames, int nf
                                                                                err, bv);
   set_decode_frames_smem();
   k_decode_frames<<<nf, kDecThreads, sizeof(DecSmem), st>>>(stream, frames, nf, dtype, A, out, scratch, err, nullptr,
-                                                            nullptr, bv);
+                                                            nullptr, nullptr, bv);
   count_launches(2);
 }
 
@@ -2989,13 +2995,13 @@ void launch_decode_items(const uint8_t* stream, const FrameDesc* frames, int nf,
   int launches = 1;
   if (plan.nlist) {
     set_decode_frames_smem();
-    k_dict_values<<<plan.nlist, kDecThreads, sizeof(DecSmem), st>>>(stream, frames, A, scratch, plan.list, bv);
+    k_dict_values<<<plan.nlist, kDecThreads, sizeof(DecSmem), st>>>(stream, frames, A, scratch, plan.list, plan.dyn, bv);
     launches++;
   }
   if (plan.npre) {
     k_prepass<<<(plan.npre + kItemWarps - 1) / kItemWarps, kItemWarps * 32, 0, st>>>(stream, frames, A,
                                                                                    plan.pre_items, plan.npre, P,
-                                                                                   scratch, bv);
+                                                                                   scratch, plan.dyn, bv);
     launches++;
   }
   if (plan.need_scan) {
@@ -3005,12 +3011,12 @@ void launch_decode_items(const uint8_t* stream, const FrameDesc* frames, int nf,
   }
   if (plan.nmain) {
     k_decode_items<<<(plan.nmain + kItemWarps - 1) / kItemWarps, kItemWarps * 32, 0, st>>>(
-        stream, frames, dtype, A, plan.main_items, plan.nmain, plan.frame_pre, P, out, scratch, err, bv);
+        stream, frames, dtype, A, plan.main_items, plan.nmain, plan.frame_pre, P, out, scratch, err, plan.dyn, bv);
     launches++;
   }
   if (plan.nlist) {
     k_decode_frames<<<plan.nlist, kDecThreads, sizeof(DecSmem), st>>>(stream, frames, (int)plan.nlist, dtype, A, out,
-                                                                       scratch, err, plan.list, plan.ent, bv);
+                                                                       scratch, err, plan.list, plan.ent, plan.dyn, bv);
     launches++;
   }
   count_launches(launches);

@@ -171,11 +171,94 @@ __device__ void dp_parse_head(const uint8_t* __restrict__ s, uint64_t len, DpHea
   } while (false);
 }
 
-__global__ void k_dp_head(const uint8_t* __restrict__ s, uint64_t len, DpHead* __restrict__ out) {
+// A plain column of a few frames has them walked right here, one header
+// latency each (0.5 us): the scan for candidates, its three-launch scan, the
+// compaction and the chain's resolution cost 45 us whatever the column's size
+// (1M prices in 32 frames: 216 us through them, 161 us so).
+// A first frame that promises more frames than the list holds stops the walk
+// at once.  The values past the lane's count (unknown while a bitmap is
+// unread) and all errors are left to k_dp_plan_small, which hands the stream
+// to the host reader.
+__global__ void k_dp_head(const uint8_t* __restrict__ s, uint64_t len, DpHead* __restrict__ out,
+                          DpCand* __restrict__ chain) {
   if (threadIdx.x || blockIdx.x) return;
   DpHead H;
   dp_parse_head(s, len, H);
+  if (H.kind == 0 && !H.decimal && H.n) {
+    const DpLane& L = H.lanes[0];
+    const uint64_t end = L.base + L.len;
+    uint64_t pos = L.fstart, counted = 0, modes = 0;
+    uint32_t nf = 0;
+    while (counted < H.n && pos + 9 <= end) {
+      const uint32_t mode = s[pos], n = ld_u32(s + pos + 1), plen = ld_u32(s + pos + 5);
+      if (nf == kDpChainMax || (nf == 0 && n && H.n / n > 2 * kDpChainMax)) {
+        nf = 0;
+        break;
+      }
+      if (mode > 63 || n == 0 || n > (uint32_t)kMaxBlock || plen > end - pos - 9 || plen >= (1u << 24)) break;
+      DpCand c;
+      c.pos = pos;
+      c.n = n;
+      c.plen_mode = plen << 8 | mode;
+      chain[nf++] = c;
+      modes |= 1ull << mode;
+      pos += 9ull + plen;
+      counted += n;
+    }
+    H.chain = nf;
+    H.chain_modes = modes;
+  }
   *out = H;
+}
+
+// The bitmap of a short column: k_dp_bitmap, the rank scan, k_select_table and
+// the copy of the caller's bytes by one CTA.
+__global__ void __launch_bounds__(1024) k_dp_bitmap_small(const uint8_t* __restrict__ s, const DpHead* __restrict__ H,
+                                                          uint64_t n, uint32_t* __restrict__ bm32,
+                                                          uint64_t* __restrict__ rank, uint64_t* __restrict__ sel,
+                                                          uint64_t* __restrict__ nvalid,
+                                                          uint8_t* __restrict__ valid_out) {
+  __shared__ uint64_t s_warp[33];
+  const uint8_t* src = s + H->vblob_off;
+  const uint64_t nb = (n + 7) / 8;
+  const uint32_t nw = (uint32_t)((n + 31) / 32);
+  uint32_t bits[kSmallPer];
+  uint64_t sum = 0;
+  const uint32_t per = (nw + 1023) / 1024;  // words a thread
+#pragma unroll
+  for (uint32_t k = 0; k < kSmallPer; k++) {
+    const uint32_t w = threadIdx.x * per + k;
+    bits[k] = 0;
+    if (k < per && w < nw) {
+      const uint64_t b0 = 4ull * w;
+      if (b0 + 4 <= nb) bits[k] = ld_u32(src + b0);
+      else
+        for (uint64_t q = 0; b0 + q < nb; q++) bits[k] |= (uint32_t)src[b0 + q] << (8 * q);
+      const uint64_t rem = n - 32ull * w;
+      if (rem < 32) bits[k] &= (1u << rem) - 1u;
+      if (valid_out)
+        for (uint64_t q = 0; q < 4 && b0 + q < nb; q++) valid_out[b0 + q] = (uint8_t)(bits[k] >> (8 * q));
+    }
+    if (k < per && w < nw) bm32[w] = bits[k];
+    sum += __popc(bits[k]);
+  }
+  if (threadIdx.x == 0) bm32[nw] = 0;
+  uint64_t total, r = block_excl_scan<ScanSum>(sum, s_warp, &total);
+  if (threadIdx.x == 0) *nvalid = total;
+#pragma unroll
+  for (uint32_t k = 0; k < kSmallPer; k++) {
+    const uint32_t w = threadIdx.x * per + k;
+    if (k >= per || w >= nw) break;
+    rank[w] = r;
+    const uint32_t c = __popc(bits[k]);
+    const uint64_t m = (r + 511) / 512 * 512;
+    if (m < r + c) {
+      uint32_t x = bits[k];
+      for (uint64_t q = m - r; q; q--) x &= x - 1u;
+      sel[m / 512] = 32ull * w + (uint64_t)(__ffs(x) - 1);
+    }
+    r += c;
+  }
 }
 
 // Bitmap words of the RAW blob (bits past n cleared) and each word's
@@ -568,7 +651,7 @@ __device__ bool dp_alprd_tags(const uint8_t* p, uint64_t plen, uint64_t* nexc, u
   if (plen < 2 || p[1] > 8) return false;
   uint64_t pos = 2 + 8ull * p[1], clen = 0;
   if (pos > plen || rd_varint(p, plen, &pos, nexc) != E_OK) return false;
-  if (warp_exc_walk(p, plen, &pos, *nexc, [](bool, uint64_t, uint64_t, uint64_t) { return true; })) return false;
+  if (warp_exc_walk<false>(p, plen, &pos, *nexc, [](bool, uint64_t, uint64_t, uint64_t) { return true; })) return false;
   if (pos >= plen) return false;
   *ctag = p[pos++];
   if (rd_varint(p, plen, &pos, &clen) != E_OK || clen > plen - pos) return false;
@@ -917,12 +1000,123 @@ __global__ void k_dp_expand(const DpLaneOut* __restrict__ out, DpTables T) {
   }
 }
 
+// The tables of a walked chain (k_dp_items, k_dp_layout and k_dp_expand of at
+// most kDpChainMax frames) in one CTA: a warp counts a frame's items, warp 0
+// lays the frames out, all threads list the items.  Table entries of frames
+// that are not kept (all of them when the status is set) are empty frames.
+__global__ void __launch_bounds__(1024) k_dp_plan_small(const uint8_t* __restrict__ s, const DpHead* __restrict__ H,
+                                                        const DpCand* __restrict__ chain,
+                                                        const uint64_t* __restrict__ nvalid, DpTables T,
+                                                        DpLaneOut* __restrict__ out, unsigned long long* __restrict__ err) {
+  __shared__ FrameItems s_it[kDpChainMax];
+  __shared__ uint32_t s_main[kDpChainMax + 1], s_pre[kDpChainMax + 1], s_kept;
+  const int l = threadIdx.x & 31, warp = threadIdx.x >> 5;
+  const uint32_t F = H->chain, plog2 = H->lanes[0].plog2;
+  const uint64_t n_total = dp_lane_total(H, H->lanes[0], nvalid);
+  for (uint32_t f = warp; f < F; f += 32) {
+    const DpCand c = chain[f];
+    FrameItems it = dp_frame_items(s + c.pos + 9, c.n, c.plen_mode >> 8, c.plen_mode & 0xFF, plog2);
+    if (l == 0) s_it[f] = it;
+  }
+  __syncthreads();
+  if (warp == 0) {
+    static_assert(kDpChainMax <= 64, "two frames a lane");
+    uint64_t voff = 0;
+    uint32_t mo = 0, po = 0, lo = 0, kept = 0;
+    bool scan = false, dict = false, ent = false, bad = false, done = n_total == 0;
+    for (uint32_t f0 = 0; f0 < F; f0 += 32) {
+      const uint32_t f = f0 + l;
+      const bool in = f < F;
+      const DpCand c = in ? chain[f] : DpCand{0, 0, 0};
+      const FrameItems it = in ? s_it[f] : FrameItems{0, 0, false, false, false, 0};
+      const uint64_t vin = warp_incl_scan((uint64_t)c.n), v0 = voff + vin - c.n;
+      const bool keep = in && v0 < n_total;
+      const uint32_t nm = keep ? it.nmain : 0, np = keep ? it.npre : 0;
+      const bool li = keep && it.list;
+      const uint32_t im = warp_incl_scan(nm), ip = warp_incl_scan(np), lm = __ballot_sync(0xffffffffu, li);
+      if (in) {
+        FrameDesc d;
+        d.payload_off = c.pos + 9;
+        d.value_off = v0;
+        d.n = c.n;
+        d.plen = c.plen_mode >> 8;
+        d.mode = c.plen_mode & 0xFF;
+        d.aux = 0;
+        T.frames[f] = d;
+        s_main[f] = mo + im - nm;
+        s_pre[f] = po + ip - np;
+        T.frame_pre[f] = make_uint2(po + ip - np, np);
+        if (li) T.list[lo + __popc(lm & ((1u << l) - 1u))] = f;
+      }
+      kept += __popc(__ballot_sync(0xffffffffu, keep));
+      scan = __any_sync(0xffffffffu, keep && it.scan) || scan;
+      dict = __any_sync(0xffffffffu, keep && it.dict) || dict;
+      ent = __any_sync(0xffffffffu, keep && it.ent != 0) || ent;
+      done = __any_sync(0xffffffffu, keep && v0 + c.n == n_total) || done;
+      bad = __any_sync(0xffffffffu, keep && v0 + c.n > n_total) || bad;
+      // the modes that the parallel reader leaves out (PRED) or does not know
+      bad = __any_sync(0xffffffffu, keep && !(kCandModes >> (c.plen_mode & 0xFF) & 1)) || bad;
+      voff += __shfl_sync(0xffffffffu, vin, 31);
+      mo += __shfl_sync(0xffffffffu, im, 31);
+      po += __shfl_sync(0xffffffffu, ip, 31);
+      lo += __popc(lm);
+    }
+    if (l == 0) {
+      DpLaneOut R;
+      memset(&R, 0, sizeof(R));
+      R.status = H->kind || bad || !done || n_total == ~0ull ? 1u : ent || n_total == 0 ? 2u : 0u;
+      if (R.status) {
+        kept = mo = po = lo = 0;
+      }
+      R.nframes = kept;
+      R.nmain = mo;
+      R.npre = po;
+      R.nlist = lo;
+      R.need_scan = scan;
+      R.any_dict = dict;
+      *out = R;
+      *err = ~0ull;
+      s_kept = kept;
+      s_main[kept] = mo;
+      s_pre[kept] = po;
+    }
+  }
+  __syncthreads();
+  const uint32_t kept = s_kept;
+  for (uint32_t f = kept + threadIdx.x; f < F; f += blockDim.x) {
+    FrameDesc d;
+    d.payload_off = 0;
+    d.value_off = 0;
+    d.n = d.plen = 0;
+    d.mode = M_RAW;
+    d.aux = 0;
+    T.frames[f] = d;
+    T.frame_pre[f] = make_uint2(0, 0);
+  }
+  for (uint32_t f = warp; f < kept; f += 32) {
+    for (uint32_t k = s_main[f] + l; k < s_main[f + 1]; k += 32) T.main_items[k] = ItemRef{f, k - s_main[f]};
+    for (uint32_t k = s_pre[f] + l; k < s_pre[f + 1]; k += 32) T.pre_items[k] = ItemRef{f, k - s_pre[f]};
+  }
+}
+
 std::atomic<unsigned long long> g_chain_attr{0};
 
 }  // namespace
 
-void launch_dp_head(const uint8_t* s, uint64_t len, DpHead* H, cudaStream_t st) {
-  k_dp_head<<<1, 32, 0, st>>>(s, len, H);
+void launch_dp_head(const uint8_t* s, uint64_t len, DpHead* H, DpCand* chain, cudaStream_t st) {
+  k_dp_head<<<1, 32, 0, st>>>(s, len, H, chain);
+  count_launches(1);
+}
+
+void launch_dp_bitmap_small(const uint8_t* s, const DpHead* H, uint64_t n, uint32_t* bm32, uint64_t* rank,
+                            uint64_t* sel, uint64_t* nvalid, uint8_t* valid_out, cudaStream_t st) {
+  k_dp_bitmap_small<<<1, 1024, 0, st>>>(s, H, n, bm32, rank, sel, nvalid, valid_out);
+  count_launches(1);
+}
+
+void launch_dp_plan_small(const uint8_t* s, const DpHead* H, const DpCand* chain, const uint64_t* nvalid,
+                          const DpTables& T, DpLaneOut* out, unsigned long long* err, cudaStream_t st) {
+  k_dp_plan_small<<<1, 1024, 0, st>>>(s, H, chain, nvalid, T, out, err);
   count_launches(1);
 }
 

@@ -1891,10 +1891,11 @@ __device__ inline uint32_t sub_range(uint64_t item, uint64_t n, uint64_t fixed_b
 constexpr int kAlpWarps = 8;
 constexpr uint16_t kAlpEfKnown = 0x8000;  // SubStats::pad16 holds e | f << 8 of a sub-block that passed
 __global__ void __launch_bounds__(kAlpWarps * 32) k_alp_stats(const uint64_t* __restrict__ v, uint64_t n,
-                                                              uint64_t fixed_bs, uint64_t items,
+                                                              const uint64_t* d_n, uint64_t fixed_bs, uint64_t items,
                                                               SubStats* __restrict__ ss) {
   __shared__ uint64_t smp[kAlpWarps][32];
   __shared__ double pexp[19], pfrac[19];
+  if (d_n) n = *d_n;
   if (threadIdx.x < 19) {
     pexp[threadIdx.x] = kExp10[threadIdx.x];
     pfrac[threadIdx.x] = kFrac10[threadIdx.x];
@@ -2080,8 +2081,8 @@ __device__ __noinline__ void stats_partial(const uint64_t* __restrict__ sv, uint
 
 template <bool FLOATS>
 __global__ void __cluster_dims__(kStatsCluster, 1, 1) __launch_bounds__(kStatsWarps * 32, FLOATS ? 3 : 5) k_sub_stats(
-    const uint64_t* __restrict__ v, uint64_t n, uint64_t fixed_bs, uint64_t items, int dtype, int level,
-    SubStats* __restrict__ ss, FmStat* __restrict__ fms, uint64_t* __restrict__ smp16, uint8_t* __restrict__ grow,
+    const uint64_t* __restrict__ v, uint64_t n, const uint64_t* d_n, uint64_t fixed_bs, uint64_t items, int dtype,
+    int level, SubStats* __restrict__ ss, FmStat* __restrict__ fms, uint64_t* __restrict__ smp16, uint8_t* __restrict__ grow,
     uint32_t* __restrict__ winbits) {
   __shared__ uint32_t bitsA[512], bitsB[512];
   __shared__ uint32_t lbits[kLbBits / 32];  // dictionary cardinality lower bound (the CTA's share of the window)
@@ -2089,6 +2090,7 @@ __global__ void __cluster_dims__(kStatsCluster, 1, 1) __launch_bounds__(kStatsWa
   __shared__ uint64_t s_first[kStatsWarps], s_last[kStatsWarps];
   __shared__ uint32_t s_neq[kStatsWarps], s_cnt[kStatsWarps];
   int lane = threadIdx.x & 31, warp = threadIdx.x >> 5;
+  if (d_n) n = *d_n;
   const bool do_float = FLOATS && level >= 1;
   uint64_t item = (uint64_t)blockIdx.x * kStatsWarps + warp;
   const uint64_t win = blockIdx.x / kStatsCluster;
@@ -3533,8 +3535,10 @@ __global__ void __launch_bounds__(kEncThreads, 2) k_emit(const uint64_t* __restr
 // (adaptive) each window's block.
 constexpr int kPlanThreads = 1024;
 __global__ void __launch_bounds__(kPlanThreads)
-    k_plan(const uint8_t* __restrict__ grow, uint64_t n, uint64_t fixed_bs, FrameDesc* frames, uint32_t* nb,
-           uint32_t* __restrict__ w2b) {
+    k_plan(const uint8_t* __restrict__ grow, uint64_t n, const uint64_t* d_n, uint64_t fixed_bs, FrameDesc* frames,
+           uint32_t* nb, uint32_t* __restrict__ w2b) {
+  const uint64_t bound = n;
+  if (d_n) n = *d_n;
   if (fixed_bs) {
     uint64_t nblk = (n + fixed_bs - 1) / fixed_bs;
     for (uint64_t i = (uint64_t)blockIdx.x * blockDim.x + threadIdx.x; i < nblk; i += (uint64_t)gridDim.x * blockDim.x) {
@@ -3562,6 +3566,29 @@ __global__ void __launch_bounds__(kPlanThreads)
   __shared__ uint32_t s_state, s_count;
   int t = threadIdx.x, lane = t & 31, warp = t >> 5;
   uint64_t nwin = (n + kBaseQuantum - 1) / kBaseQuantum;
+  if (nwin <= 32) {  // a short column: one warp, a lane per window, no barrier
+    if (warp) return;
+    const uint32_t gm = __ballot_sync(0xffffffffu, lane < nwin && grow[lane]);
+    uint32_t starts = 0;
+    for (uint32_t w = 0; w < nwin; w += gm >> w & 1u ? 4 : 1) starts |= 1u << w;
+    if (lane < nwin) {
+      const uint32_t b = __popc(starts & ((2u << lane) - 1u)) - 1;
+      w2b[lane] = b;
+      if (starts >> lane & 1u) {
+        FrameDesc f;
+        f.value_off = lane * (uint64_t)kBaseQuantum;
+        f.n = (uint32_t)(qmin(f.value_off + (gm >> lane & 1u ? kMaxBlock : kBaseQuantum), n) - f.value_off);
+        f.payload_off = 0;
+        f.plen = 0;
+        f.mode = 0;
+        f.aux = 0;
+        frames[b] = f;
+      }
+    }
+    for (uint64_t w = nwin + lane; w * kBaseQuantum < bound; w += 32) w2b[w] = kEmpty32;  // no block
+    if (lane == 0) *nb = __popc(starts);
+    return;
+  }
   if (t == 0) {
     s_state = 0;
     s_count = 0;
@@ -3639,6 +3666,7 @@ __global__ void __launch_bounds__(kPlanThreads)
     __syncthreads();
   }
   if (t == 0) *nb = s_count;
+  for (uint64_t w = nwin + t; w * kBaseQuantum < bound; w += kPlanThreads) w2b[w] = kEmpty32;  // no block
 }
 
 __global__ void k_frame_sizes(const FrameDesc* __restrict__ frames, const uint32_t* __restrict__ nbp, uint32_t maxb,
@@ -3660,12 +3688,12 @@ __global__ void k_frame_apply(FrameDesc* frames, const uint32_t* __restrict__ nb
 // ---------------------------------------------------------------------------
 static size_t enc_smem_bytes() { return sizeof(EncSmem); }
 
-void launch_plan(const uint8_t* grow, uint64_t n, uint64_t fixed_bs, FrameDesc* frames, uint32_t* nb, uint32_t* w2b,
-                 cudaStream_t st) {
+void launch_plan(const uint8_t* grow, uint64_t n, const uint64_t* d_n, uint64_t fixed_bs, FrameDesc* frames,
+                 uint32_t* nb, uint32_t* w2b, cudaStream_t st) {
   unsigned g = 1;
   if (fixed_bs) g = (unsigned)qmin(((n + fixed_bs - 1) / fixed_bs + kPlanThreads - 1) / kPlanThreads, 4096);
   if (g == 0) g = 1;
-  k_plan<<<g, kPlanThreads, 0, st>>>(grow, n, fixed_bs, frames, nb, w2b);
+  k_plan<<<g, kPlanThreads, 0, st>>>(grow, n, d_n, fixed_bs, frames, nb, w2b);
   count_launches(1);
 }
 
@@ -3676,22 +3704,22 @@ uint64_t sub_stats_items(uint64_t n, uint64_t fixed_bs) {
 uint64_t sub_stats_bytes() { return sizeof(SubStats); }
 uint64_t fm_stats_bytes() { return sizeof(FmStat); }
 
-void launch_sub_stats(const uint64_t* lane, uint64_t n, uint64_t fixed_bs, int dtype, int level, void* ss, void* fms,
-                      uint64_t* smp16, uint8_t* grow, uint32_t* winbits, cudaStream_t st) {
+void launch_sub_stats(const uint64_t* lane, uint64_t n, const uint64_t* d_n, uint64_t fixed_bs, int dtype, int level,
+                      void* ss, void* fms, uint64_t* smp16, uint8_t* grow, uint32_t* winbits, cudaStream_t st) {
   uint64_t items = sub_stats_items(n, fixed_bs);
   if (!items) return;
   const uint64_t per = kStatsWarps * kStatsCluster;
   const unsigned g = (unsigned)((items + per - 1) / per * kStatsCluster);
   if (dtype_float(dtype)) {
-    k_sub_stats<true><<<g, kStatsWarps * 32, 0, st>>>(lane, n, fixed_bs, items, dtype, level, (SubStats*)ss, (FmStat*)fms,
+    k_sub_stats<true><<<g, kStatsWarps * 32, 0, st>>>(lane, n, d_n, fixed_bs, items, dtype, level, (SubStats*)ss, (FmStat*)fms,
                                                        smp16, grow, winbits);
     if (level >= 1) {
-      k_alp_stats<<<(unsigned)((items + kAlpWarps - 1) / kAlpWarps), kAlpWarps * 32, 0, st>>>(lane, n, fixed_bs, items,
+      k_alp_stats<<<(unsigned)((items + kAlpWarps - 1) / kAlpWarps), kAlpWarps * 32, 0, st>>>(lane, n, d_n, fixed_bs, items,
                                                                                             (SubStats*)ss);
       count_launches(1);
     }
   } else
-    k_sub_stats<false><<<g, kStatsWarps * 32, 0, st>>>(lane, n, fixed_bs, items, dtype, level, (SubStats*)ss,
+    k_sub_stats<false><<<g, kStatsWarps * 32, 0, st>>>(lane, n, d_n, fixed_bs, items, dtype, level, (SubStats*)ss,
                                                         (FmStat*)fms, nullptr, grow, winbits);
   count_launches(1);
 }

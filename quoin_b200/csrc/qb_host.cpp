@@ -313,6 +313,12 @@ struct LaneJob {
   uint64_t block_size;  // 0 = adaptive, else clamped to [1, 131072]
   uint8_t plog2;
   bool vb_raw = false;  // the bitmap's transition count proves the RAW validity blob
+  // A short nullable column: its bitmap and values, and where the device keeps
+  // its valid count (n_valid is then a bound); the header, the validity blob and
+  // the lane are written without waiting for the count.
+  const uint64_t* d_n = nullptr;
+  const uint8_t* d_bm_in = nullptr;
+  const void* d_values = nullptr;
   uint64_t* d_nest = nullptr;  // a decimal's limb lane: its place in the container (device; moves past the stream)
 };
 
@@ -360,6 +366,10 @@ int encode_lane(QuoinCtx* c, cudaStream_t st, const LaneJob& j, uint8_t* d_dst, 
     nest.pos = j.d_nest;
     nest.out = d_dst;
     nest.cap = dst_cap;
+  } else if (j.d_n) {
+    launch_begin_small(j.d_bm_in, j.logical_n, c->p<uint64_t>(S_RANK), d_misc + 8, d_dst, h, d_misc, st);
+    TimedRegion tr(T_LOWER, st);
+    launch_lower(j.d_values, j.dtype, j.d_bm_in, c->p<uint64_t>(S_RANK), j.logical_n, c->p<uint64_t>(S_LANE), st);
   } else {
     launch_put_header(d_dst, h, d_misc, st);
   }
@@ -419,9 +429,9 @@ int encode_lane(QuoinCtx* c, cudaStream_t st, const LaneJob& j, uint8_t* d_dst, 
   uint32_t* nb = c->p<uint32_t>(S_NB);
   {
     TimedRegion tr(T_PLAN, st);
-    launch_sub_stats(j.lane, n, bs, j.dtype, level, c->p<void>(S_SUBST), fl ? c->p<void>(S_FMST) : nullptr,
+    launch_sub_stats(j.lane, n, j.d_n, bs, j.dtype, level, c->p<void>(S_SUBST), fl ? c->p<void>(S_FMST) : nullptr,
                      fl ? c->p<uint64_t>(S_SMP16) : nullptr, c->p<uint8_t>(S_GROW), c->p<uint32_t>(S_WINBITS), st);
-    launch_plan(c->p<uint8_t>(S_GROW), n, bs, fr, nb, c->p<uint32_t>(S_W2B), st);
+    launch_plan(c->p<uint8_t>(S_GROW), n, j.d_n, bs, fr, nb, c->p<uint32_t>(S_W2B), st);
   }
   {
     TimedRegion tr(T_COMPETE, st);
@@ -638,6 +648,18 @@ int compress_column_device(QuoinCtx* c, cudaStream_t st, int wire, uint64_t n, c
   const uint8_t* d_bm = nullptr;
   bool vb_raw = false;
   const uint64_t* lane = nullptr;
+  // A short nullable column whose validity blob fits the destination whatever
+  // the bitmap (else the longer way decides what is too small).
+  if (d_validity && n && (n + 31) / 32 <= kSmallWords && dst_cap >= 16 + 10 + 1 + (n + 7) / 8 + 16) {
+    CK(c->ensure(S_RANK, (n + 31) / 32 * 8 + 64));
+    CK(c->ensure(S_MISC, 64 * 8));
+    CK(c->ensure(S_LANE, n * 8 + 64));
+    LaneJob j{c->p<uint64_t>(S_LANE), n, wire, n, nullptr, level, bs, plog2};
+    j.d_n = c->p<uint64_t>(S_MISC) + 8;
+    j.d_bm_in = d_validity;
+    j.d_values = d_values;
+    return encode_lane(c, st, j, d_dst, dst_cap, out_len);
+  }
   rc = lower_column(c, st, wire, n, d_values, d_validity, &lane, &n_valid, &d_bm, &vb_raw);
   if (rc) return rc;
   LaneJob j{lane, n_valid, wire, n, d_bm, level, bs, plog2, vb_raw};
@@ -674,7 +696,7 @@ int probe_windows_device(QuoinCtx* c, cudaStream_t st, int wire, uint64_t n, con
   }
   {
     TimedRegion tr(T_PLAN, st);
-    launch_sub_stats(lane, nv, 0, wire, QUOIN_LEVEL_FAST, c->p<void>(S_SUBST), fl ? c->p<void>(S_FMST) : nullptr,
+    launch_sub_stats(lane, nv, nullptr, 0, wire, QUOIN_LEVEL_FAST, c->p<void>(S_SUBST), fl ? c->p<void>(S_FMST) : nullptr,
                      fl ? c->p<uint64_t>(S_SMP16) : nullptr, c->p<uint8_t>(S_GROW), c->p<uint32_t>(S_WINBITS), st);
   }
   CK(cudaMemcpyAsync(grow_out, c->p<uint8_t>(S_GROW), nwin, cudaMemcpyDeviceToHost, st));
@@ -1041,6 +1063,7 @@ struct QuoinDecodeIndex {
   uint64_t* d_items = nullptr;  // item tables of every lane (layout_items)
   uint64_t items_bytes = 0;
   uint64_t max_pre = 0;
+  uint64_t src_len = 0;  // a host-buffer decode's stream length (its device copy is S_SRC)
 };
 
 namespace {
@@ -1320,6 +1343,7 @@ int begin_decode(QuoinCtx* c, const uint8_t* src, uint64_t len, QuoinDecodeIndex
   CK(c->ensure(S_SRC, len + 64));
   if (len) CK(cudaMemcpyAsync(c->p<uint8_t>(S_SRC), src, len, cudaMemcpyHostToDevice, st));
   int k = parse_stream(src, len, X);
+  X.src_len = len;
   if (k) {
     cudaStreamSynchronize(st);
     return kind_to_code(k);
@@ -1327,11 +1351,34 @@ int begin_decode(QuoinCtx* c, const uint8_t* src, uint64_t len, QuoinDecodeIndex
   return QUOIN_OK;
 }
 
+constexpr int kChainNo = -1000, kChainHost = -1001;  // decode_chain
+int decode_device(QuoinCtx* c, cudaStream_t st, const uint8_t* d_src, uint64_t len, void* d_out,
+                  uint64_t out_cap_bytes, uint8_t* d_valid_out, int32_t* wire_out, uint64_t* n_out,
+                  bool general = true);
+
 // Second half: uploads the index, decodes, copies the values (and the
 // validity bitmap) out.  Every return waits for the stream's work.
 int finish_decode(QuoinCtx* c, QuoinDecodeIndex* X, void* values_out, uint8_t* validity_out) {
   cudaStream_t st = c->stream;
   uint64_t nf = total_frames(*X);
+  // A short column's tables are made on the device from its copy of the stream
+  // (decode_chain): sending the host's took five copies, five launches for the
+  // ranks and a wait.
+  if (!X->decimal && X->n && nf && nf <= kDpChainMax && X->src_len <= (1u << 20)) {
+    const uint64_t bytes = X->n * native_width(X->wire);
+    CK(c->ensure(S_OUTVALS, bytes + 64));
+    int32_t wire = 0;
+    uint64_t n = 0;
+    int rc = decode_device(c, st, c->p<uint8_t>(S_SRC), X->src_len, c->p<void>(S_OUTVALS), bytes, nullptr, &wire, &n,
+                           false);
+    if (rc == QUOIN_OK) {
+      CK(cudaMemcpyAsync(values_out, c->p<void>(S_OUTVALS), bytes, cudaMemcpyDeviceToHost, st));
+      CK(cudaStreamSynchronize(st));
+      if (validity_out && X->has_validity) memcpy(validity_out, X->bitmap.data(), X->bitmap.size());
+      return QUOIN_OK;
+    }
+    if (rc != kChainNo) return rc;
+  }
   CK(c->ensure(S_DFRAMES, (nf + 1) * sizeof(FrameDesc)));
   CK(c->ensure(S_DBM, X->bitmap.size() + 16));
   CK(c->ensure(S_DRANK, ((X->n + 31) / 32 + 1) * 8));
@@ -1374,8 +1421,15 @@ struct DpMisc {  // the reader's small results, read back in one copy
   uint64_t nruns;  // runs of an RLE validity blob
   uint64_t ctl[4][2];  // per lane: chain resolved, chain frames
 };
-constexpr uint64_t kDpHeadOff = 0, kDpMiscOff = 512;
-static_assert(sizeof(DpHead) <= kDpMiscOff && sizeof(DpMisc) <= 512, "reader results fit their slot");
+struct DpSmall {  // a short column's results, read back in one copy
+  unsigned long long err;
+  DpLaneOut out;
+  uint64_t nvalid;
+};
+constexpr uint64_t kDpHeadOff = 0, kDpMiscOff = 512, kDpSmallOff = 1024, kDpChainOff = 1280;
+constexpr uint64_t kDpMiscBytes = kDpChainOff + kDpChainMax * sizeof(DpCand);
+static_assert(sizeof(DpHead) <= kDpMiscOff && sizeof(DpMisc) <= 512 && sizeof(DpSmall) <= 256,
+              "reader results fit their slot");
 
 // Decodes of device streams read by the device reader, and those the host
 // reader took (with the reason of the last: 1 header, 2 a lane's chain, 3 a
@@ -1420,24 +1474,117 @@ int decode_device_via_host(QuoinCtx* c, cudaStream_t st, const uint8_t* d_src, u
                         c->p<uint64_t>(S_DSEL), dvmin, c->p<uint64_t>(S_DITEMS), d_src, d_out, d_valid_out);
 }
 
+// A short column whose frames the head kernel walked: its bitmap and tables in
+// one launch each, and the block decoder launched for as many items as the
+// column can have, so that nothing is waited for until the result.  kChainNo: a
+// column for the general way (all null, entropy-coded parts); kChainHost: for
+// the host reader.
+int decode_chain(QuoinCtx* c, cudaStream_t st, const uint8_t* d_src, uint64_t len, const DpHead& H, void* d_out,
+                 uint8_t* d_valid_out) {
+  auto has = [&](int m) { return (H.chain_modes >> m & 1) != 0; };
+  for (int m : {0, 4, 7, 11, 20, 25, 29, 45})  // always entropy-coded, or not a frame this reader takes
+    if (has(m)) return kChainNo;
+  const uint64_t n = H.n, nw = (n + 31) / 32;
+  const uint32_t nf = H.chain;
+  uint8_t* misc = c->p<uint8_t>(S_DPMISC);
+  DpHead* dH = reinterpret_cast<DpHead*>(misc + kDpHeadOff);
+  DpSmall* dS = reinterpret_cast<DpSmall*>(misc + kDpSmallOff);
+  const DpCand* chain = reinterpret_cast<const DpCand*>(misc + kDpChainOff);
+  const bool need_scan = has(51) || has(3) || has(53), listed = has(19) || has(52);
+  const uint64_t nmax = n / 512 + 2 * nf + (has(3) ? len / kXorzItemBytes : 0) + 1;
+  CK(c->ensure(S_DFRAMES, (nf + 1) * sizeof(FrameDesc)));
+  CK(c->ensure(S_DITEMS, (2 * nmax + 2 * kDpChainMax + 2) * 8));
+  CK(c->ensure(S_DAUX, decode_aux_bytes((int)nf)));
+  if (need_scan) CK(c->ensure(S_PRE, (nmax + 1) * prepass_rec_bytes()));
+  uint64_t* scr = nullptr;
+  if (listed || has(53)) {
+    CK(c->ensure(S_DSCR, n * 8 + 64));
+    scr = c->p<uint64_t>(S_DSCR);
+  }
+  bool bytes_out = false;  // the caller's bitmap is written with the words
+  if (H.has_validity) {
+    TimedRegion tr(T_READ, st);
+    CK(c->ensure(S_DBM, (nw + 2) * 4 + 16));
+    CK(c->ensure(S_DRANK, (nw + 1) * 8));
+    CK(c->ensure(S_DSEL, (n / 512 + 2) * 8));
+    if (H.vtag == 0 && nw <= kSmallWords) {
+      launch_dp_bitmap_small(d_src, dH, n, c->p<uint32_t>(S_DBM), c->p<uint64_t>(S_DRANK), c->p<uint64_t>(S_DSEL),
+                             &dS->nvalid, d_valid_out, st);
+      bytes_out = true;
+    } else {
+      CK(c->ensure(S_TILE, (scan_tile_count(nw) + 16) * 8));
+      if (H.vtag == 0) {
+        launch_dp_bitmap(d_src, dH, n, c->p<uint8_t>(S_DBM), c->p<uint64_t>(S_DRANK), st);
+      } else {
+        CK(c->ensure(S_DPRUNS, (H.vblob_len + 3) * 8));
+        uint64_t* ends = c->p<uint64_t>(S_DPRUNS);
+        launch_dp_bitmap_rle(d_src, dH, n, ends + 1, ends, c->p<uint8_t>(S_DBM), c->p<uint64_t>(S_DRANK), st);
+      }
+      launch_scan_sum(c->p<uint64_t>(S_DRANK), c->p<uint64_t>(S_DRANK), nw, c->p<uint64_t>(S_TILE), &dS->nvalid, st);
+      launch_select_table(c->p<uint8_t>(S_DBM), n, c->p<uint64_t>(S_DRANK), n, c->p<uint64_t>(S_DSEL), st);
+    }
+  }
+  uint64_t* ditems = c->p<uint64_t>(S_DITEMS);
+  DpTables T;
+  T.frames = c->p<FrameDesc>(S_DFRAMES);
+  T.main_items = reinterpret_cast<ItemRef*>(ditems);
+  T.pre_items = reinterpret_cast<ItemRef*>(ditems + nmax);
+  T.frame_pre = reinterpret_cast<uint2*>(ditems + 2 * nmax);
+  T.list = reinterpret_cast<uint32_t*>(ditems + 2 * nmax + kDpChainMax);
+  T.main_off = nullptr;
+  {
+    TimedRegion tr(T_READ, st);
+    launch_dp_plan_small(d_src, dH, chain, &dS->nvalid, T, &dS->out, &dS->err, st);
+  }
+  ItemPlan P;
+  P.main_items = T.main_items;
+  P.nmain = (uint32_t)nmax;
+  P.pre_items = T.pre_items;
+  P.npre = need_scan ? (uint32_t)nmax : 0;
+  P.frame_pre = T.frame_pre;
+  P.list = T.list;
+  P.nlist = listed ? nf : 0;
+  P.need_scan = need_scan;
+  P.ent = nullptr;
+  P.dyn = &dS->out;
+  DecodeOut O{d_out, (int)H.wire, H.has_validity ? c->p<uint32_t>(S_DBM) : nullptr, c->p<uint64_t>(S_DRANK),
+              c->p<uint64_t>(S_DSEL), n, n};
+  O.plog2 = H.lanes[0].plog2;
+  if (H.has_validity) O.d_nvalid = &dS->nvalid;
+  {
+    TimedRegion tr(T_DECODE, st);
+    launch_decode_items(d_src, T.frames, (int)nf, (int)H.wire, O, P, c->p<void>(S_PRE), scr, c->p<void>(S_DAUX),
+                        &dS->err, st);
+  }
+  if (d_valid_out && H.has_validity && !bytes_out)
+    CK(cudaMemcpyAsync(d_valid_out, c->p<uint8_t>(S_DBM), (n + 7) / 8, cudaMemcpyDeviceToDevice, st));
+  DpSmall R;
+  CK(read_small(c, st, &R, dS, sizeof(R)));
+  resolve_timing();
+  if (R.out.status) return R.out.status == 2 ? kChainNo : kChainHost;
+  if (R.err != ~0ull) return kind_to_code((int)(R.err & 0xFF));
+  return QUOIN_OK;
+}
+
 // Reference decoder.rs:43-118 (+ decimal.rs:100-168, lib.rs:462-508) for a
 // stream in device memory: header, validity and frame table are read by the
 // device reader, then the block decoder runs as for an indexed decode.  Three
 // host synchronisations: the header (output sizes), the frame tables (launch
-// sizes), the final status.
+// sizes), the final status; two for a short column (decode_chain), and with
+// `general` false nothing but that way is tried (kChainNo otherwise).
 int decode_device(QuoinCtx* c, cudaStream_t st, const uint8_t* d_src, uint64_t len, void* d_out,
-                  uint64_t out_cap_bytes, uint8_t* d_valid_out, int32_t* wire_out, uint64_t* n_out) {
-  CK(c->ensure(S_DPMISC, 1024));
+                  uint64_t out_cap_bytes, uint8_t* d_valid_out, int32_t* wire_out, uint64_t* n_out, bool general) {
+  CK(c->ensure(S_DPMISC, kDpMiscBytes));
   uint8_t* misc = c->p<uint8_t>(S_DPMISC);
   DpHead* dH = reinterpret_cast<DpHead*>(misc + kDpHeadOff);
   DpMisc* dM = reinterpret_cast<DpMisc*>(misc + kDpMiscOff);
-  CK(cudaMemsetAsync(dM, 0, sizeof(DpMisc), st));  // the valid count stays 0 without a bitmap
   {
     TimedRegion tr(T_READ, st);
-    launch_dp_head(d_src, len, dH, st);
+    launch_dp_head(d_src, len, dH, reinterpret_cast<DpCand*>(misc + kDpChainOff), st);
   }
   DpHead H;
   CK(read_small(c, st, &H, dH, sizeof(H)));
+  if (H.kind && !general) return kChainNo;
   if (H.kind)
     return decode_device_via_host(c, st, d_src, len, d_out, out_cap_bytes, d_valid_out, wire_out, n_out, 1);
   *wire_out = (int32_t)H.wire;
@@ -1446,6 +1593,20 @@ int decode_device(QuoinCtx* c, cudaStream_t st, const uint8_t* d_src, uint64_t l
   if (H.n * (uint64_t)w > out_cap_bytes) return QUOIN_ERR_BUFFER_TOO_SMALL;
   const uint64_t n = H.n;
   const uint64_t nw = (n + 31) / 32;
+  if (H.chain && ((uintptr_t)d_out % w) == 0) {
+    int rc = decode_chain(c, st, d_src, len, H, d_out, d_valid_out);
+    if (!general) return rc == kChainHost ? kChainNo : rc;
+    if (rc == kChainHost)
+      return decode_device_via_host(c, st, d_src, len, d_out, out_cap_bytes, d_valid_out, wire_out, n_out, 2);
+    if (rc != kChainNo) {
+      g_last_ncand.store(H.chain);
+      g_last_attempts.store(1);
+      g_reads_device.fetch_add(1);
+      return rc;
+    }
+  }
+  if (!general) return kChainNo;
+  CK(cudaMemsetAsync(dM, 0, sizeof(DpMisc), st));  // the valid count stays 0 without a bitmap
   // validity: bitmap, word ranks, valid count, select table
   if (H.has_validity && n) {
     TimedRegion tr(T_READ, st);

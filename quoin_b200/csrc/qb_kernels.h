@@ -10,6 +10,10 @@ struct QuoinCtx;
 
 namespace qb {
 
+// A column of at most kSmallWords bitmap words has them handled by one CTA of
+// 1,024 threads.
+constexpr uint32_t kSmallPer = 8, kSmallWords = 1024 * kSmallPer;
+
 // ---- decoder (qb_decode.cu) ----
 // Payload bytes of one XORZ warp item (the readers cut XORZ frames into
 // items of this many bytes; other modes into items of 512 values).
@@ -46,6 +50,7 @@ struct DecodeOut {
   uint64_t n;       // logical values (positions)
   uint64_t nvalid;  // lane values
   uint32_t plog2 = 16;  // the stream header's predictor_log2 (FCM / DFCM table size)
+  const uint64_t* d_nvalid = nullptr;  // the lane's value count on the device, in place of nvalid
 };
 void launch_decode_frames(const uint8_t* stream, const FrameDesc* frames, int nf, int dtype, const DecodeOut& out,
                           uint64_t* scratch, void* aux, unsigned long long* err, cudaStream_t st);
@@ -71,6 +76,7 @@ struct BatchView {
 struct ItemRef {
   uint32_t frame, local;
 };
+struct DpLaneOut;
 struct ItemPlan {
   const ItemRef* pre_items;
   uint32_t npre;
@@ -81,6 +87,7 @@ struct ItemPlan {
   uint32_t nlist;
   bool need_scan;
   uint8_t* ent;  // entropy areas of the listed frames (FrameDesc::aux), or null
+  const DpLaneOut* dyn = nullptr;  // the item and list counts on the device (those above are then bounds)
 };
 uint64_t prepass_rec_bytes();
 void launch_decode_items(const uint8_t* stream, const FrameDesc* frames, int nf, int dtype, const DecodeOut& out,
@@ -103,8 +110,13 @@ struct DpHead {
   uint64_t vblob_off, vblob_len;  // the validity blob's bytes after its tag
   uint32_t vtag, pad2;            // 0 RAW (ceil(n/8) bitmap bytes), 1 RLE (varint runs)
   uint64_t vmin[4];
+  // A plain column of at most kDpChainMax frames: their count (0: not walked)
+  // and the set of their modes (bit per id).
+  uint64_t chain_modes;
+  uint32_t chain, pad3;
   DpLane lanes[4];
 };
+constexpr uint32_t kDpChainMax = 48;
 // A frame-header candidate (pos = header offset; plen < 2^24).
 struct DpCand {
   uint64_t pos;
@@ -134,7 +146,17 @@ struct DpTables {
   ItemRef* pre_items;
 };
 constexpr uint64_t kDpChainSmem = 200 * 1024;  // successor tables in shared memory up to 25,598 candidates
-void launch_dp_head(const uint8_t* s, uint64_t len, DpHead* H, cudaStream_t st);
+// The header, and the frames of a short column in `chain` (kDpChainMax).
+void launch_dp_head(const uint8_t* s, uint64_t len, DpHead* H, DpCand* chain, cudaStream_t st);
+// A short column after its head is known: the validity bitmap of at most
+// kSmallWords words (words, ranks, select table, valid count, the caller's
+// bytes) in one launch, and the frame and item tables of the walked chain in
+// another (*out's status: 0, 1 the host reader parses the stream, 2 a frame
+// has an entropy-coded part; *err is set to "none").
+void launch_dp_bitmap_small(const uint8_t* s, const DpHead* H, uint64_t n, uint32_t* bm32, uint64_t* rank,
+                            uint64_t* sel, uint64_t* nvalid, uint8_t* valid_out, cudaStream_t st);
+void launch_dp_plan_small(const uint8_t* s, const DpHead* H, const DpCand* chain, const uint64_t* nvalid,
+                          const DpTables& T, DpLaneOut* out, unsigned long long* err, cudaStream_t st);
 // The validity bitmap of an n-value stream as 32-bit words (ceil(n/32) + 1
 // written, the last zero) and each word's popcount in cnt: from a RAW blob,
 // or from an RLE blob (validity.rs:92-119; `ends` holds vblob_len entries).
@@ -257,11 +279,13 @@ constexpr uint64_t kWinWords = 1028;
 uint64_t sub_stats_items(uint64_t n, uint64_t fixed_bs);
 uint64_t sub_stats_bytes();
 uint64_t fm_stats_bytes();
-void launch_sub_stats(const uint64_t* lane, uint64_t n, uint64_t fixed_bs, int dtype, int level, void* ss, void* fms,
-                      uint64_t* smp16, uint8_t* grow, uint32_t* winbits, cudaStream_t st);
+// d_n (optional, here and below): the value count on the device, n then being
+// a bound.
+void launch_sub_stats(const uint64_t* lane, uint64_t n, const uint64_t* d_n, uint64_t fixed_bs, int dtype, int level,
+                      void* ss, void* fms, uint64_t* smp16, uint8_t* grow, uint32_t* winbits, cudaStream_t st);
 // w2b (adaptive): the block of each window.
-void launch_plan(const uint8_t* grow, uint64_t n, uint64_t fixed_bs, FrameDesc* frames, uint32_t* nb, uint32_t* w2b,
-                 cudaStream_t st);
+void launch_plan(const uint8_t* grow, uint64_t n, const uint64_t* d_n, uint64_t fixed_bs, FrameDesc* frames,
+                 uint32_t* nb, uint32_t* w2b, cudaStream_t st);
 // Competition part 2: one CTA per planned block; writes mode / plen / aux.
 // With `ent` (max_blocks records of ent_rec_bytes()) the Balanced in-pool
 // candidates run too (rANS-coded parts, BYTE_TRANSPOSE) and their choices
@@ -329,9 +353,13 @@ void launch_bitmap_transitions(const uint8_t* bm, uint64_t n, unsigned long long
 // transitions counted by one CTA (rank = exclusive word ranks, *total = the
 // valid count, *trans = 0/1 transitions); frame offsets of at most
 // kSmallWords blocks by one CTA.
-constexpr uint32_t kSmallPer = 8, kSmallWords = 1024 * kSmallPer;
 void launch_valid_small(const uint8_t* bm, uint64_t n, uint64_t* rank, uint64_t* total, unsigned long long* trans,
                         cudaStream_t st);
+// A short nullable column's stream up to its first frame: the ranks and valid
+// count as above, then the header at dst (hdr, its validity flag set when the
+// bitmap has a null) and the validity blob; *d_base = their length.
+void launch_begin_small(const uint8_t* bm, uint64_t n, uint64_t* rank, uint64_t* total, uint8_t* dst, Bytes16 hdr,
+                        uint64_t* d_base, cudaStream_t st);
 // The stream a call on context c runs on: `stream` when given, else the
 // context's own (the default context when c is null).
 cudaStream_t ctx_stream(struct ::QuoinCtx* c, void* stream);

@@ -20,8 +20,9 @@ __device__ inline uint64_t lower_one(const uint8_t* base, uint64_t i, int dtype)
 __device__ inline uint32_t bm_word_at(const uint8_t* bm, uint64_t w, uint64_t n) {
   uint64_t nbytes = (n + 7) / 8;
   uint32_t bits = 0;
-  for (int k = 0; k < 4; k++)
-    if (w * 4 + k < nbytes) bits |= (uint32_t)bm[w * 4 + k] << (8 * k);
+  if (w * 4 + 4 <= nbytes) bits = ld_u32(bm + w * 4);
+  else
+    for (int k = 0; w * 4 + k < nbytes; k++) bits |= (uint32_t)bm[w * 4 + k] << (8 * k);
   uint64_t rem = n - w * 32;
   if (rem < 32) bits &= (1u << rem) - 1u;
   return bits;
@@ -255,20 +256,11 @@ void launch_decimal_split(const uint8_t* values, int nlimbs, const uint8_t* bm, 
 // Validity blob: the smaller of [1] ++ LEB128 alternating run lengths
 // (starting with a null run) or [0] ++ the raw bitmap bytes.
 // ---------------------------------------------------------------------------
-__device__ inline uint32_t bm_word(const uint8_t* bm, uint64_t w, uint64_t n) {
-  uint64_t nbytes = (n + 7) / 8;
-  uint32_t bits = 0;
-  for (int k = 0; k < 4; k++)
-    if (w * 4 + k < nbytes) bits |= (uint32_t)bm[w * 4 + k] << (8 * k);
-  uint64_t rem = n - w * 32;
-  if (rem < 32) bits &= (1u << rem) - 1u;
-  return bits;
-}
 // Transition mask of word w: bit j set when bit (32w + j) differs from its
 // predecessor (the bit before position 0 is taken as 0, i.e. a null).
 __device__ inline uint32_t trans_mask(const uint8_t* bm, uint64_t w, uint64_t n) {
-  uint32_t b = bm_word(bm, w, n);
-  uint32_t prev = w ? (bm_word(bm, w - 1, n) >> 31) : 0u;
+  uint32_t b = bm_word_at(bm, w, n);
+  uint32_t prev = w ? (bm_word_at(bm, w - 1, n) >> 31) : 0u;
   uint32_t t = b ^ ((b << 1) | prev);
   uint64_t rem = n - w * 32;
   if (rem < 32) t &= (1u << rem) - 1u;
@@ -359,51 +351,74 @@ __global__ void k_bitmap_transitions(const uint8_t* __restrict__ bm, uint64_t n,
   }
 }
 // A short column's bitmap (at most kSmallWords 32-bit words) in one CTA of
-// 1,024 threads: every word's exclusive valid rank, the valid count and the
-// 0/1 transition count -- k_word_popcount, the rank scan and
+// 1,024 threads: every word's exclusive valid rank, the valid count (returned)
+// and the 0/1 transition count (optional) -- k_word_popcount, the rank scan and
 // k_bitmap_transitions in one launch, since short columns pay per launch.
-__global__ void __launch_bounds__(1024) k_valid_small(const uint8_t* __restrict__ bm, uint64_t n,
-                                                      uint64_t* __restrict__ rank, uint64_t* __restrict__ total,
-                                                      unsigned long long* __restrict__ trans) {
+struct SmallWords {
+  uint32_t w[kSmallPer];   // the thread's consecutive words
+  uint32_t tm[kSmallPer];  // their transition masks (trans_mask)
+  uint32_t first, per;     // the first of them, words a thread
+};
+__device__ inline SmallWords small_words(const uint8_t* __restrict__ bm, uint64_t n) {
+  SmallWords s;
+  const uint32_t nw = (uint32_t)((n + 31) / 32);
+  s.per = (nw + 1023) / 1024;
+  s.first = threadIdx.x * s.per;
+  uint32_t prev = s.first && s.first <= nw ? bm_word_at(bm, s.first - 1, n) >> 31 : 0u;
+#pragma unroll
+  for (uint32_t k = 0; k < kSmallPer; k++) s.w[k] = k < s.per && s.first + k < nw ? bm_word_at(bm, s.first + k, n) : 0u;
+#pragma unroll
+  for (uint32_t k = 0; k < kSmallPer; k++) {
+    s.tm[k] = 0;
+    if (k < s.per && s.first + k < nw) {
+      uint32_t t = s.w[k] ^ ((s.w[k] << 1) | prev);
+      const uint64_t rem = n - 32ull * (s.first + k);
+      if (rem < 32) t &= (1u << rem) - 1u;
+      s.tm[k] = t;
+    }
+    prev = s.w[k] >> 31;
+  }
+  return s;
+}
+// Ranks, the valid count (returned) and the number of transitions.
+__device__ uint64_t valid_small(const SmallWords& S, uint64_t n, uint64_t* __restrict__ rank, uint32_t* trans) {
   __shared__ uint64_t wsum[32];
-  __shared__ uint32_t wtr[32];
+  __shared__ uint32_t wtr[32], s_tr;
   uint32_t nw = (uint32_t)((n + 31) / 32), t = threadIdx.x, l = t & 31, warp = t >> 5;
-  uint32_t c[kSmallPer];
   uint32_t s = 0, tr = 0;
 #pragma unroll
   for (uint32_t k = 0; k < kSmallPer; k++) {
-    uint32_t w = t * kSmallPer + k;
-    c[k] = w < nw ? (uint32_t)__popc(bm_word_at(bm, w, n)) : 0u;
-    s += c[k];
-    if (w < nw) tr += __popc(trans_mask(bm, w, n));
+    s += __popc(S.w[k]);
+    tr += __popc(S.tm[k]);
   }
-  uint64_t inc = s;
-  for (int o = 1; o < 32; o <<= 1) {
-    uint64_t u = __shfl_up_sync(0xffffffffu, inc, o);
-    if ((int)l >= o) inc += u;
-  }
-  tr = warp_sum(tr);
+  const uint64_t inc = warp_incl_scan(s);
+  tr = __reduce_add_sync(0xffffffffu, tr);
   if (l == 31) wsum[warp] = inc;
   if (l == 0) wtr[warp] = tr;
   __syncthreads();
   if (warp == 0) {
-    uint64_t x = wsum[l];
-    for (int o = 1; o < 32; o <<= 1) {
-      uint64_t u = __shfl_up_sync(0xffffffffu, x, o);
-      if ((int)l >= o) x += u;
-    }
-    wsum[l] = x;  // inclusive over warps
-    uint32_t y = warp_sum(wtr[l]);
-    if (l == 31) *total = x;
-    if (l == 0) *trans = y;
+    wsum[l] = warp_incl_scan(wsum[l]);  // inclusive over warps
+    uint32_t y = __reduce_add_sync(0xffffffffu, wtr[l]);
+    if (l == 0) s_tr = y;
   }
   __syncthreads();
   uint64_t run = (warp ? wsum[warp - 1] : 0ull) + inc - s;
 #pragma unroll
   for (uint32_t k = 0; k < kSmallPer; k++) {
-    uint32_t w = t * kSmallPer + k;
-    if (w < nw) rank[w] = run;
-    run += c[k];
+    if (k < S.per && S.first + k < nw) rank[S.first + k] = run;
+    run += __popc(S.w[k]);
+  }
+  *trans = s_tr;
+  return wsum[31];
+}
+__global__ void __launch_bounds__(1024) k_valid_small(const uint8_t* __restrict__ bm, uint64_t n,
+                                                      uint64_t* __restrict__ rank, uint64_t* __restrict__ total,
+                                                      unsigned long long* __restrict__ trans) {
+  uint32_t tr;
+  const uint64_t nv = valid_small(small_words(bm, n), n, rank, &tr);
+  if (threadIdx.x == 0) {
+    *total = nv;
+    *trans = tr;
   }
 }
 
@@ -480,16 +495,23 @@ uint64_t validity_tmp_words(uint64_t n) {
 // The validity blob of a short column (at most kSmallWords words) in one CTA
 // of 1,024 threads: the three passes above (last transitions + max scan, run
 // bytes + sum scan, write) with block scans in place of the grid scans.
-__global__ void __launch_bounds__(1024) k_vb_small(const uint8_t* __restrict__ bm, uint64_t n,
-                                                   uint8_t* __restrict__ out, uint64_t* __restrict__ blob_len) {
+// place(blob length) gives the blob's destination.
+template <class P>
+__device__ void vb_small(const SmallWords& S, const uint8_t* __restrict__ bm, uint64_t n, bool raw, P place) {
   __shared__ uint64_t wa[32], wb[32];
-  uint32_t nw = (uint32_t)((n + 31) / 32), t = threadIdx.x, l = t & 31, warp = t >> 5;
-  uint32_t tm[kSmallPer];
+  if (raw) {  // proven by the transitions
+    uint8_t* out = place(1 + (n + 7) / 8);
+    if (threadIdx.x == 0) out[0] = 0;
+#pragma unroll 4
+    for (uint64_t i = threadIdx.x; i < (n + 7) / 8; i += 1024) out[1 + i] = bm[i];
+    return;
+  }
+  uint32_t t = threadIdx.x, l = t & 31, warp = t >> 5;
+  const uint32_t* tm = S.tm;
   uint64_t mx = 0;
 #pragma unroll
   for (uint32_t k = 0; k < kSmallPer; k++) {
-    uint32_t w = t * kSmallPer + k;
-    tm[k] = w < nw ? trans_mask(bm, w, n) : 0u;
+    uint32_t w = S.first + k;
     if (tm[k]) mx = (uint64_t)w * 32 + (31 - __clz(tm[k]));  // words ascend: the thread's last transition
   }
   // exclusive max scan of the threads' last transitions (positions ascend, 0 = none yet)
@@ -518,7 +540,7 @@ __global__ void __launch_bounds__(1024) k_vb_small(const uint8_t* __restrict__ b
 #pragma unroll
   for (uint32_t k = 0; k < kSmallPer; k++) {
     uint32_t tt = tm[k];
-    uint32_t w = t * kSmallPer + k;
+    uint32_t w = S.first + k;
     while (tt) {
       uint64_t p = (uint64_t)w * 32 + (__ffs(tt) - 1);
       tt &= tt - 1;
@@ -545,10 +567,8 @@ __global__ void __launch_bounds__(1024) k_vb_small(const uint8_t* __restrict__ b
   uint64_t run_bytes = wb[31], raw_len = (n + 7) / 8;
   uint64_t rle_len = run_bytes + varint_len(n - t_last);
   bool rle = rle_len < raw_len;
-  if (t == 0) {
-    out[0] = rle ? 1 : 0;
-    *blob_len = 1 + (rle ? rle_len : raw_len);
-  }
+  uint8_t* out = place(1 + (rle ? rle_len : raw_len));
+  if (t == 0) out[0] = rle ? 1 : 0;
   if (!rle) {
     for (uint64_t i = t; i < raw_len; i += blockDim.x) out[1 + i] = bm[i];
     return;
@@ -558,7 +578,7 @@ __global__ void __launch_bounds__(1024) k_vb_small(const uint8_t* __restrict__ b
 #pragma unroll
   for (uint32_t k = 0; k < kSmallPer; k++) {
     uint32_t tt = tm[k];
-    uint32_t w = t * kSmallPer + k;
+    uint32_t w = S.first + k;
     while (tt) {
       uint64_t p = (uint64_t)w * 32 + (__ffs(tt) - 1);
       tt &= tt - 1;
@@ -579,6 +599,45 @@ __global__ void __launch_bounds__(1024) k_vb_small(const uint8_t* __restrict__ b
       out[q++] = v ? (b | 0x80) : b;
     } while (v);
   }
+}
+__global__ void __launch_bounds__(1024) k_vb_small(const uint8_t* __restrict__ bm, uint64_t n,
+                                                   uint8_t* __restrict__ out, uint64_t* __restrict__ blob_len) {
+  vb_small(small_words(bm, n), bm, n, false, [&](uint64_t len) {
+    if (threadIdx.x == 0) *blob_len = len;
+    return out;
+  });
+}
+// A short nullable column's stream up to its first frame, without the host: a
+// call that waited for the valid count before it could go on paid 25 us of the
+// 96 that a 65,537-value page took; with this kernel and the one-warp plan the
+// page takes 72.
+__global__ void __launch_bounds__(1024) k_begin_small(const uint8_t* __restrict__ bm, uint64_t n,
+                                                      uint64_t* __restrict__ rank, uint64_t* __restrict__ total,
+                                                      uint8_t* dst, Bytes16 hdr, uint64_t* __restrict__ d_base) {
+  const SmallWords S = small_words(bm, n);
+  uint32_t trans;
+  const uint64_t nv = valid_small(S, n, rank, &trans);
+  const int t = threadIdx.x;
+  if (t < 16) dst[t] = t == 5 ? (nv < n ? 1 : 0) : hdr.b[t];
+  if (t == 0) {
+    *total = nv;
+    if (nv == n) *d_base = 16;
+  }
+  if (nv == n) return;  // all valid: no bitmap in the stream
+  vb_small(S, bm, n, trans + 1ull >= (n + 7) / 8, [&](uint64_t len) {
+    const uint32_t vl = varint_len(len);
+    if (t == 0) {
+      uint64_t v = len;
+      for (uint32_t k = 0; k < vl; k++, v >>= 7) dst[16 + k] = (uint8_t)((v & 0x7f) | (k + 1 < vl ? 0x80u : 0u));
+      *d_base = 16 + vl + len;
+    }
+    return dst + 16 + vl;
+  });
+}
+void launch_begin_small(const uint8_t* bm, uint64_t n, uint64_t* rank, uint64_t* total, uint8_t* dst, Bytes16 hdr,
+                        uint64_t* d_base, cudaStream_t st) {
+  k_begin_small<<<1, 1024, 0, st>>>(bm, n, rank, total, dst, hdr, d_base);
+  count_launches(1);
 }
 
 void launch_validity_blob(const uint8_t* bm, uint64_t n, uint64_t* tmp, uint64_t* tile_tmp, uint8_t* out,

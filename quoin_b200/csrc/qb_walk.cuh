@@ -110,9 +110,10 @@ __device__ inline uint32_t warp_alp_walk(const uint8_t* p, uint64_t plen, uint64
 // ALP-RD exception list (reference codecs/alp_rd.rs:230-245): nexc records of
 // a varint position and 8 bytes from *pos.  rec(active, x, q, v) is called by
 // the whole warp for groups of up to 32 consecutive records, the active lanes
-// first: record x starts at q and has position v; it returns false for a
-// position out of range (E_CORRUPT).  On success *pos is the list's end.
-template <class R>
+// first: record x starts at q and has position v (0 without VALUES, for a
+// caller that only looks for the end); it returns false for a position out of
+// range (E_CORRUPT).  On success *pos is the list's end.
+template <bool VALUES, class R>
 __device__ inline uint32_t warp_exc_walk(const uint8_t* p, uint64_t plen, uint64_t* pos, uint64_t nexc, R rec) {
   constexpr uint32_t kPer = 4;
   const uint32_t l = threadIdx.x & 31;
@@ -135,7 +136,7 @@ __device__ inline uint32_t warp_exc_walk(const uint8_t* p, uint64_t plen, uint64
           const uint64_t high = w & 0x8080808080808080ull & (~0ull >> (64 - 8 * len));
           ok[j] = ok[j] && high == (0x0080808080808080ull & (len == 1 ? 0ull : (~0ull >> (64 - 8 * (len - 1)))));
 #pragma unroll
-          for (uint32_t b = 0; b < 8; b++)
+          for (uint32_t b = 0; VALUES && b < 8; b++)
             if (b < len) v[j] |= ((w >> (8 * b)) & 0x7Full) << (7 * b);
         } else if (ok[j]) {
           uint64_t t = q;
