@@ -320,8 +320,10 @@ int quoin_b200_timing_read(double *ms_out, uint64_t *calls_out, int n);
  * length and mixed dtype).  A batch holds `workers` contexts (1..64) on the
  * current device; a batch call hands its columns, longest first, to one host
  * worker per context, so short columns' launch and synchronisation latencies
- * overlap.  Every column's stream is byte-identical to the single-column
- * call's.  One batch call at a time per batch. */
+ * overlap; columns of up to 2^20 values are compressed in groups that share
+ * their launches (about 45 bytes of device memory per value of a group, kept
+ * by its context).  Every column's stream is byte-identical to the
+ * single-column call's.  One batch call at a time per batch. */
 typedef struct QuoinBatch QuoinBatch;
 QuoinBatch *quoin_b200_batch_create(int workers);
 void quoin_b200_batch_free(QuoinBatch *batch);

@@ -1890,9 +1890,9 @@ __device__ inline uint32_t sub_range(uint64_t item, uint64_t n, uint64_t fixed_b
 // (e, f) search reads them at a different index in every lane.
 constexpr int kAlpWarps = 8;
 constexpr uint16_t kAlpEfKnown = 0x8000;  // SubStats::pad16 holds e | f << 8 of a sub-block that passed
-__global__ void __launch_bounds__(kAlpWarps * 32) k_alp_stats(const uint64_t* __restrict__ v, uint64_t n,
-                                                              const uint64_t* d_n, uint64_t fixed_bs, uint64_t items,
-                                                              SubStats* __restrict__ ss) {
+__device__ __forceinline__ void alp_stats(const uint32_t cta, const uint64_t* __restrict__ v, uint64_t n,
+                                          const uint64_t* d_n, uint64_t fixed_bs, uint64_t items,
+                                          SubStats* __restrict__ ss) {
   __shared__ uint64_t smp[kAlpWarps][32];
   __shared__ double pexp[19], pfrac[19];
   if (d_n) n = *d_n;
@@ -1902,7 +1902,7 @@ __global__ void __launch_bounds__(kAlpWarps * 32) k_alp_stats(const uint64_t* __
   }
   __syncthreads();
   int lane = threadIdx.x & 31, warp = threadIdx.x >> 5;
-  uint64_t item = (uint64_t)blockIdx.x * kAlpWarps + warp;
+  uint64_t item = (uint64_t)cta * kAlpWarps + warp;
   if (item >= items) return;
   uint64_t s;
   uint32_t cnt = sub_range(item, n, fixed_bs, &s);
@@ -2080,8 +2080,8 @@ __device__ __noinline__ void stats_partial(const uint64_t* __restrict__ sv, uint
 }
 
 template <bool FLOATS>
-__global__ void __cluster_dims__(kStatsCluster, 1, 1) __launch_bounds__(kStatsWarps * 32, FLOATS ? 3 : 5) k_sub_stats(
-    const uint64_t* __restrict__ v, uint64_t n, const uint64_t* d_n, uint64_t fixed_bs, uint64_t items, int dtype,
+__device__ __forceinline__ void sub_stats(
+    const uint32_t cta, const uint64_t* __restrict__ v, uint64_t n, const uint64_t* d_n, uint64_t fixed_bs, uint64_t items, int dtype,
     int level, SubStats* __restrict__ ss, FmStat* __restrict__ fms, uint64_t* __restrict__ smp16, uint8_t* __restrict__ grow,
     uint32_t* __restrict__ winbits) {
   __shared__ uint32_t bitsA[512], bitsB[512];
@@ -2092,8 +2092,8 @@ __global__ void __cluster_dims__(kStatsCluster, 1, 1) __launch_bounds__(kStatsWa
   int lane = threadIdx.x & 31, warp = threadIdx.x >> 5;
   if (d_n) n = *d_n;
   const bool do_float = FLOATS && level >= 1;
-  uint64_t item = (uint64_t)blockIdx.x * kStatsWarps + warp;
-  const uint64_t win = blockIdx.x / kStatsCluster;
+  uint64_t item = (uint64_t)cta * kStatsWarps + warp;
+  const uint64_t win = cta / kStatsCluster;
   uint64_t s = 0;
   uint32_t cnt = item < items ? sub_range(item, n, fixed_bs, &s) : 0u;
   // window probe sampling (adaptive): window-relative stride max(len/4096, 1)
@@ -2491,17 +2491,14 @@ __device__ __noinline__ int sample_winner(EncSmem& S, const uint64_t* v, uint32_
 // FLOAT_MULT, ALP-RD and DICT and the BYTE_TRANSPOSE candidate; the chosen
 // coded parts go to ent[b] for the emission.
 template <bool ENT, bool SAMPLE>
-__global__ void __launch_bounds__(kEncThreads, 2) k_decide(const uint64_t* __restrict__ lane, FrameDesc* frames,
-                                                        const uint32_t* __restrict__ nbp, uint64_t fixed_bs,
-                                                        int dtype, int level, const SubStats* __restrict__ ss,
-                                                        const FmStat* __restrict__ fms,
-                                                        const uint64_t* __restrict__ smp16,
-                                                        const uint32_t* __restrict__ winbits,
-                                                        uint8_t* __restrict__ scratch, EntRec* __restrict__ ent,
-                                                        RdRec* __restrict__ rdr, BlkRec* __restrict__ blk) {
+__device__ __forceinline__ void decide(const uint32_t b, const uint64_t* __restrict__ lane, FrameDesc* frames,
+                                       const uint32_t* __restrict__ nbp, uint64_t fixed_bs, int dtype, int level,
+                                       const SubStats* __restrict__ ss, const FmStat* __restrict__ fms,
+                                       const uint64_t* __restrict__ smp16, const uint32_t* __restrict__ winbits,
+                                       uint8_t* __restrict__ scratch, EntRec* __restrict__ ent,
+                                       RdRec* __restrict__ rdr, BlkRec* __restrict__ blk) {
   extern __shared__ __align__(16) uint8_t smem_raw[];
   EncSmem& S = *reinterpret_cast<EncSmem*>(smem_raw);
-  uint32_t b = blockIdx.x;
   if (b >= *nbp) return;
   FrameDesc fd = frames[b];
   const uint64_t* v = lane + fd.value_off;
@@ -3400,19 +3397,16 @@ __device__ __noinline__ void emit_rle(EncSmem& S, const uint64_t* v, uint32_t n,
 // w2b: the block of each window (adaptive plan); split: CTAs per window.
 constexpr uint32_t kWinSubs = kBaseQuantum / kSub;
 template <bool ENT>
-__global__ void __launch_bounds__(kEncThreads, 2) k_emit(const uint64_t* __restrict__ lane,
-                                                      const FrameDesc* __restrict__ frames,
-                                                      const uint32_t* __restrict__ nbp,
-                                                      const uint32_t* __restrict__ w2b, uint32_t split,
-                                                      uint64_t fixed_bs, int dtype,
-                                                      const SubStats* __restrict__ ss,
-                                                      const FmStat* __restrict__ fms,
-                                                      const RdRec* __restrict__ rdr, const BlkRec* __restrict__ blk,
-                                                      uint8_t* __restrict__ scratch, uint8_t* __restrict__ outbuf,
-                                                      uint64_t out_cap, const EntRec* __restrict__ ent) {
+__device__ __forceinline__ void emit_unit(const uint32_t cta, const uint64_t* __restrict__ lane,
+                                          const FrameDesc* __restrict__ frames, const uint32_t* __restrict__ nbp,
+                                          const uint32_t* __restrict__ w2b, uint32_t split, uint64_t fixed_bs,
+                                          int dtype, const SubStats* __restrict__ ss, const FmStat* __restrict__ fms,
+                                          const RdRec* __restrict__ rdr, const BlkRec* __restrict__ blk,
+                                          uint8_t* __restrict__ scratch, uint8_t* __restrict__ outbuf,
+                                          uint64_t out_cap, const EntRec* __restrict__ ent) {
   extern __shared__ __align__(16) uint8_t smem_raw[];
   EncSmem& S = *reinterpret_cast<EncSmem*>(smem_raw);
-  const uint32_t unit = blockIdx.x / split, part = blockIdx.x % split;
+  const uint32_t unit = cta / split, part = cta % split;
   uint32_t b, win;  // the block, and the unit's window within it
   if (fixed_bs) {
     const uint32_t per = (uint32_t)((fixed_bs + kBaseQuantum - 1) / kBaseQuantum);
@@ -3534,14 +3528,14 @@ __global__ void __launch_bounds__(kEncThreads, 2) k_emit(const uint64_t* __restr
 // Block plan (reference encoder.rs:154-178): fills frames[].value_off / .n and
 // (adaptive) each window's block.
 constexpr int kPlanThreads = 1024;
-__global__ void __launch_bounds__(kPlanThreads)
-    k_plan(const uint8_t* __restrict__ grow, uint64_t n, const uint64_t* d_n, uint64_t fixed_bs, FrameDesc* frames,
-           uint32_t* nb, uint32_t* __restrict__ w2b) {
+__device__ __forceinline__ void plan_blocks(const uint32_t cta, const uint32_t ctas, const uint8_t* __restrict__ grow,
+                                            uint64_t n, const uint64_t* d_n, uint64_t fixed_bs, FrameDesc* frames,
+                                            uint32_t* nb, uint32_t* __restrict__ w2b) {
   const uint64_t bound = n;
   if (d_n) n = *d_n;
   if (fixed_bs) {
     uint64_t nblk = (n + fixed_bs - 1) / fixed_bs;
-    for (uint64_t i = (uint64_t)blockIdx.x * blockDim.x + threadIdx.x; i < nblk; i += (uint64_t)gridDim.x * blockDim.x) {
+    for (uint64_t i = (uint64_t)cta * blockDim.x + threadIdx.x; i < nblk; i += (uint64_t)ctas * blockDim.x) {
       FrameDesc f;
       f.value_off = i * fixed_bs;
       f.n = (uint32_t)qmin(fixed_bs, n - f.value_off);
@@ -3551,7 +3545,7 @@ __global__ void __launch_bounds__(kPlanThreads)
       f.aux = 0;
       frames[i] = f;
     }
-    if (blockIdx.x == 0 && threadIdx.x == 0) *nb = (uint32_t)nblk;
+    if (cta == 0 && threadIdx.x == 0) *nb = (uint32_t)nblk;
     return;
   }
   // Adaptive: the block starts form a chain over the 32768-value windows
@@ -3560,7 +3554,7 @@ __global__ void __launch_bounds__(kPlanThreads)
   // block), and window w maps it by f_w(s) = s ? s - 1 : (grow[w] ? 3 : 0).
   // The maps compose (4 entries of 2 bits), so one CTA scans them in chunks
   // of 4096 windows, then compacts the starts into the frame table.
-  if (blockIdx.x) return;
+  if (cta) return;
   constexpr int kPer = 4, kWarps = kPlanThreads / 32;
   __shared__ uint32_t s_wmap[kWarps], s_wcnt[kWarps];
   __shared__ uint32_t s_state, s_count;
@@ -3684,6 +3678,94 @@ __global__ void k_frame_apply(FrameDesc* frames, const uint32_t* __restrict__ nb
 }
 
 // ---------------------------------------------------------------------------
+// The kernels: of one lane (the arguments are the launch's), and of a group of
+// lanes, where map[CTA] names the lane and the CTA's place among the lane's.
+// A group's launch takes as long as its longest lane or as their sum needs on
+// the whole chip: 192 columns of 1,024 to 1,048,576 values in 2,183 launches
+// and 256 waits took 5.6 ms, in 50 launches and 5 waits 1.2 ms.
+// ---------------------------------------------------------------------------
+__global__ void __launch_bounds__(kAlpWarps * 32) k_alp_stats(const uint64_t* __restrict__ v, uint64_t n,
+                                                              const uint64_t* d_n, uint64_t fixed_bs, uint64_t items,
+                                                              SubStats* __restrict__ ss) {
+  alp_stats(blockIdx.x, v, n, d_n, fixed_bs, items, ss);
+}
+template <bool FLOATS>
+__global__ void __cluster_dims__(kStatsCluster, 1, 1) __launch_bounds__(kStatsWarps * 32, FLOATS ? 3 : 5) k_sub_stats(
+    const uint64_t* __restrict__ v, uint64_t n, const uint64_t* d_n, uint64_t fixed_bs, uint64_t items, int dtype,
+    int level, SubStats* __restrict__ ss, FmStat* __restrict__ fms, uint64_t* __restrict__ smp16, uint8_t* __restrict__ grow,
+    uint32_t* __restrict__ winbits) {
+  sub_stats<FLOATS>(blockIdx.x, v, n, d_n, fixed_bs, items, dtype, level, ss, fms, smp16, grow, winbits);
+}
+template <bool ENT, bool SAMPLE>
+__global__ void __launch_bounds__(kEncThreads, 2) k_decide(const uint64_t* __restrict__ lane, FrameDesc* frames,
+                                                        const uint32_t* __restrict__ nbp, uint64_t fixed_bs,
+                                                        int dtype, int level, const SubStats* __restrict__ ss,
+                                                        const FmStat* __restrict__ fms,
+                                                        const uint64_t* __restrict__ smp16,
+                                                        const uint32_t* __restrict__ winbits,
+                                                        uint8_t* __restrict__ scratch, EntRec* __restrict__ ent,
+                                                        RdRec* __restrict__ rdr, BlkRec* __restrict__ blk) {
+  decide<ENT, SAMPLE>(blockIdx.x, lane, frames, nbp, fixed_bs, dtype, level, ss, fms, smp16, winbits, scratch, ent, rdr,
+                      blk);
+}
+template <bool ENT>
+__global__ void __launch_bounds__(kEncThreads, 2) k_emit(const uint64_t* __restrict__ lane,
+                                                      const FrameDesc* __restrict__ frames,
+                                                      const uint32_t* __restrict__ nbp,
+                                                      const uint32_t* __restrict__ w2b, uint32_t split,
+                                                      uint64_t fixed_bs, int dtype,
+                                                      const SubStats* __restrict__ ss,
+                                                      const FmStat* __restrict__ fms,
+                                                      const RdRec* __restrict__ rdr, const BlkRec* __restrict__ blk,
+                                                      uint8_t* __restrict__ scratch, uint8_t* __restrict__ outbuf,
+                                                      uint64_t out_cap, const EntRec* __restrict__ ent) {
+  emit_unit<ENT>(blockIdx.x, lane, frames, nbp, w2b, split, fixed_bs, dtype, ss, fms, rdr, blk, scratch, outbuf,
+                 out_cap, ent);
+}
+__global__ void __launch_bounds__(kPlanThreads)
+    k_plan(const uint8_t* __restrict__ grow, uint64_t n, const uint64_t* d_n, uint64_t fixed_bs, FrameDesc* frames,
+           uint32_t* nb, uint32_t* __restrict__ w2b) {
+  plan_blocks(blockIdx.x, gridDim.x, grow, n, d_n, fixed_bs, frames, nb, w2b);
+}
+
+__global__ void __launch_bounds__(kAlpWarps * 32) k_group_alp(const EncLane* __restrict__ lanes,
+                                                              const uint32_t* __restrict__ map) {
+  const uint32_t m = map[blockIdx.x];
+  const EncLane& L = lanes[m >> 16];
+  alp_stats(m & 0xFFFF, L.v, L.n, L.d_n, L.fixed_bs, L.items, (SubStats*)L.ss);
+}
+template <bool FLOATS>
+__global__ void __cluster_dims__(kStatsCluster, 1, 1) __launch_bounds__(kStatsWarps * 32, FLOATS ? 3 : 5)
+    k_group_stats(const EncLane* __restrict__ lanes, const uint32_t* __restrict__ map, int level) {
+  const uint32_t m = map[blockIdx.x];
+  const EncLane& L = lanes[m >> 16];
+  sub_stats<FLOATS>(m & 0xFFFF, L.v, L.n, L.d_n, L.fixed_bs, L.items, L.dtype, level, (SubStats*)L.ss, (FmStat*)L.fms,
+                    L.smp16, L.grow, L.winbits);
+}
+template <bool ENT, bool SAMPLE>
+__global__ void __launch_bounds__(kEncThreads, 2)
+    k_group_decide(const EncLane* __restrict__ lanes, const uint32_t* __restrict__ map, int level) {
+  const uint32_t m = map[blockIdx.x];
+  const EncLane& L = lanes[m >> 16];
+  decide<ENT, SAMPLE>(m & 0xFFFF, L.v, L.frames, L.nb, L.fixed_bs, L.dtype, level, (const SubStats*)L.ss,
+                      (const FmStat*)L.fms, L.smp16, L.winbits, L.scratch, (EntRec*)L.ent, (RdRec*)L.rdr,
+                      (BlkRec*)L.blk);
+}
+template <bool ENT>
+__global__ void __launch_bounds__(kEncThreads, 2)
+    k_group_emit(const EncLane* __restrict__ lanes, const uint32_t* __restrict__ map) {
+  const uint32_t m = map[blockIdx.x];
+  const EncLane& L = lanes[m >> 16];
+  emit_unit<ENT>(m & 0xFFFF, L.v, L.frames, L.nb, L.w2b, 1, L.fixed_bs, L.dtype, (const SubStats*)L.ss,
+                 (const FmStat*)L.fms, (const RdRec*)L.rdr, (const BlkRec*)L.blk, L.scratch, L.out, L.out_cap,
+                 (const EntRec*)L.ent);
+}
+__global__ void __launch_bounds__(kPlanThreads) k_group_plan(const EncLane* __restrict__ lanes) {
+  const EncLane& L = lanes[blockIdx.x];
+  plan_blocks(0, 1, L.grow, L.n, L.d_n, L.fixed_bs, L.frames, L.nb, L.w2b);
+}
+
+// ---------------------------------------------------------------------------
 // Host launchers
 // ---------------------------------------------------------------------------
 static size_t enc_smem_bytes() { return sizeof(EncSmem); }
@@ -3724,19 +3806,30 @@ void launch_sub_stats(const uint64_t* lane, uint64_t n, const uint64_t* d_n, uin
   count_launches(1);
 }
 
+static int enc_smem_ready() {
+  const int sm = (int)enc_smem_bytes();
+  static std::atomic<unsigned long long> smem_set{0};
+  once_per_device(smem_set, [sm] {
+    auto set = [sm](auto* kernel) { cudaFuncSetAttribute(kernel, cudaFuncAttributeMaxDynamicSharedMemorySize, sm); };
+    set(k_decide<false, false>);
+    set(k_decide<true, false>);
+    set(k_decide<false, true>);
+    set(k_emit<false>);
+    set(k_emit<true>);
+    set(k_group_decide<false, false>);
+    set(k_group_decide<true, false>);
+    set(k_group_decide<false, true>);
+    set(k_group_emit<false>);
+    set(k_group_emit<true>);
+  });
+  return sm;
+}
+
 void launch_decide(const uint64_t* lane, FrameDesc* frames, const uint32_t* nb, uint32_t max_blocks, uint64_t fixed_bs,
                    int dtype, int level, const void* ss, const void* fms, const uint64_t* smp16,
                    const uint32_t* winbits, uint8_t* scratch, void* ent, void* rdr, void* blk, bool sample,
                    cudaStream_t st) {
-  int sm = (int)enc_smem_bytes();
-  static std::atomic<unsigned long long> smem_set{0};
-  once_per_device(smem_set, [sm] {
-    cudaFuncSetAttribute(k_decide<false, false>, cudaFuncAttributeMaxDynamicSharedMemorySize, sm);
-    cudaFuncSetAttribute(k_decide<true, false>, cudaFuncAttributeMaxDynamicSharedMemorySize, sm);
-    cudaFuncSetAttribute(k_decide<false, true>, cudaFuncAttributeMaxDynamicSharedMemorySize, sm);
-    cudaFuncSetAttribute(k_emit<false>, cudaFuncAttributeMaxDynamicSharedMemorySize, sm);
-    cudaFuncSetAttribute(k_emit<true>, cudaFuncAttributeMaxDynamicSharedMemorySize, sm);
-  });
+  const int sm = enc_smem_ready();
   if (max_blocks) {
     if (ent)
       k_decide<true, false><<<max_blocks, kEncThreads, sm, st>>>(lane, frames, nb, fixed_bs, dtype, level,
@@ -3754,6 +3847,10 @@ void launch_decide(const uint64_t* lane, FrameDesc* frames, const uint32_t* nb, 
   count_launches(max_blocks ? 1 : 0);
 }
 
+static uint64_t emit_units(uint64_t n, uint64_t fixed_bs, uint64_t max_blocks) {
+  return fixed_bs ? max_blocks * ((fixed_bs + kBaseQuantum - 1) / kBaseQuantum) : (n + kBaseQuantum - 1) / kBaseQuantum;
+}
+
 // Two CTAs per window while the windows alone leave places free (two CTAs of
 // an SM's registers): 1,048,576 prices' 32 windows emit on 64 SMs.
 void launch_emit(const uint64_t* lane, const FrameDesc* frames, const uint32_t* nb, uint32_t max_blocks,
@@ -3761,8 +3858,7 @@ void launch_emit(const uint64_t* lane, const FrameDesc* frames, const uint32_t* 
                  const void* rdr, const void* blk, uint8_t* scratch, uint8_t* out, uint64_t out_cap, const void* ent,
                  cudaStream_t st) {
   if (max_blocks) {
-    const uint64_t units = fixed_bs ? max_blocks * ((fixed_bs + kBaseQuantum - 1) / kBaseQuantum)
-                                    : (n + kBaseQuantum - 1) / kBaseQuantum;
+    const uint64_t units = emit_units(n, fixed_bs, max_blocks);
     const uint32_t split = units < 2 * 148 && !ent ? 2 : 1;
     const unsigned g = (unsigned)(units * split);
     if (ent)
@@ -3804,6 +3900,7 @@ __device__ inline void nest_write(const NestedLane& nest, uint64_t pos, uint64_t
   if (at <= nest.cap) {
     put_varint(nest.out + pos, 16 + total);
     for (int i = 0; i < 16; i++) nest.out[at - 16 + i] = nest.hdr.b[i];
+    for (int i = 0; nest.d_n && i < 8; i++) nest.out[at - 8 + i] = (uint8_t)(*nest.d_n >> (8 * i));
   }
   *nest.pos = at + total;
 }
@@ -3816,9 +3913,9 @@ __global__ void k_nest_base(NestedLane nest, const uint64_t* __restrict__ total,
 
 // At most kSmallWords frames in one CTA of 1,024 threads: k_frame_sizes, the
 // exclusive scan and k_frame_apply in one launch.
-__global__ void __launch_bounds__(1024) k_frame_offsets_small(FrameDesc* frames, const uint32_t* __restrict__ nbp,
-                                                              uint64_t* __restrict__ base_p,
-                                                              uint64_t* __restrict__ total, NestedLane nest) {
+__device__ __forceinline__ void frame_offsets_small(FrameDesc* frames, const uint32_t* __restrict__ nbp,
+                                                    uint64_t* __restrict__ base_p, uint64_t* __restrict__ total,
+                                                    const NestedLane& nest) {
   __shared__ uint64_t wsum[32];
   uint32_t nb = *nbp, t = threadIdx.x, l = t & 31, warp = t >> 5;
   uint64_t base = nest.pos ? *nest.pos : *base_p;
@@ -3858,6 +3955,50 @@ __global__ void __launch_bounds__(1024) k_frame_offsets_small(FrameDesc* frames,
     if (i < nb) frames[i].payload_off = base + run + 9;
     run += v[k];
   }
+}
+
+__global__ void __launch_bounds__(1024) k_frame_offsets_small(FrameDesc* frames, const uint32_t* __restrict__ nbp,
+                                                              uint64_t* __restrict__ base_p,
+                                                              uint64_t* __restrict__ total, NestedLane nest) {
+  frame_offsets_small(frames, nbp, base_p, total, nest);
+}
+// A column's lanes one after another: a limb's stream begins where the one
+// before it ends.
+__global__ void __launch_bounds__(1024) k_group_offsets(const EncLane* __restrict__ lanes,
+                                                        const EncCol* __restrict__ cols) {
+  const EncCol& C = cols[blockIdx.x];
+  for (int k = 0; k < max(C.nl, 1); k++) {
+    const EncLane& L = lanes[C.lane0 + k];
+    frame_offsets_small(L.frames, L.nb, C.res, C.nl ? C.vmin + 4 : C.res + 1, L.nest);
+    __syncthreads();
+  }
+}
+
+// All lanes of a group of columns whose lanes launch_begin_cols has written.
+void launch_encode_group(const EncGroup& G, int level, bool ent, bool sample, cudaStream_t st) {
+  const int sm = enc_smem_ready();
+  if (G.nfstats) k_group_stats<true><<<G.nfstats, kStatsWarps * 32, 0, st>>>(G.lanes, G.fstats, level);
+  if (G.nistats) k_group_stats<false><<<G.nistats, kStatsWarps * 32, 0, st>>>(G.lanes, G.istats, level);
+  if (G.nalp && level >= 1) k_group_alp<<<G.nalp, kAlpWarps * 32, 0, st>>>(G.lanes, G.alp);
+  k_group_plan<<<G.nlanes, kPlanThreads, 0, st>>>(G.lanes);
+  if (ent) k_group_decide<true, false><<<G.nblocks, kEncThreads, sm, st>>>(G.lanes, G.blocks, level);
+  else if (sample) k_group_decide<false, true><<<G.nblocks, kEncThreads, sm, st>>>(G.lanes, G.blocks, level);
+  else k_group_decide<false, false><<<G.nblocks, kEncThreads, sm, st>>>(G.lanes, G.blocks, level);
+  k_group_offsets<<<G.ncols, 1024, 0, st>>>(G.lanes, G.cols);
+  if (ent) k_group_emit<true><<<G.nunits, kEncThreads, sm, st>>>(G.lanes, G.units);
+  else k_group_emit<false><<<G.nunits, kEncThreads, sm, st>>>(G.lanes, G.units);
+  count_launches(4 + (G.nfstats != 0) + (G.nistats != 0) + (G.nalp && level >= 1));
+}
+// CTAs of a lane in the group's launches, as map entries of lane `lane`.
+static void map_ctas(std::vector<uint32_t>& map, uint32_t lane, uint64_t ctas) {
+  for (uint64_t k = 0; k < ctas; k++) map.push_back(lane << 16 | (uint32_t)k);
+}
+void map_lane(EncMaps& M, uint32_t lane, uint64_t n, uint64_t fixed_bs, int dtype, uint64_t max_blocks) {
+  const uint64_t items = sub_stats_items(n, fixed_bs), per = kStatsWarps * kStatsCluster;
+  map_ctas(dtype_float(dtype) ? M.fstats : M.istats, lane, (items + per - 1) / per * kStatsCluster);
+  if (dtype_float(dtype)) map_ctas(M.alp, lane, (items + kAlpWarps - 1) / kAlpWarps);
+  map_ctas(M.blocks, lane, max_blocks);
+  map_ctas(M.units, lane, emit_units(n, fixed_bs, max_blocks));
 }
 
 void launch_frame_offsets(FrameDesc* frames, const uint32_t* nb, uint32_t max_blocks, uint64_t* base,

@@ -2045,6 +2045,173 @@ int decode_queue(QuoinCtx* c, cudaStream_t st, QuoinB200DeviceDecodeJob* jobs, s
   return first;
 }
 
+// ---------------------------------------------------------------------------
+// Several columns of a batch call in shared launches.
+// ---------------------------------------------------------------------------
+// A column that a group can take: short enough for the tables' 16-bit places
+// and for one CTA's share of the offsets, with room for whatever validity blob
+// it has (else the longer way decides what is too small).
+constexpr uint64_t kGroupColumn = 1 << 20;
+constexpr int kGroupNoRoom = 1;  // no device memory for the group's arena: its columns go one by one
+
+bool group_takes(const QuoinB200CompressJob& J, uint64_t bs) {
+  if (J.wire_dtype < 0 || J.wire_dtype > 7 || !J.d_values || !J.d_dst || J.n == 0 || J.n > kGroupColumn) return false;
+  if (bs && max_blocks_for(J.n, bs) > kSmallWords) return false;
+  const bool dec = J.wire_dtype == WT_DEC128 || J.wire_dtype == WT_DEC256;
+  const uint64_t head = dec ? 19 + (J.wire_dtype == WT_DEC128 ? 16 : 32) : 16;
+  return J.dst_cap >= head + (J.d_validity ? 10 + 1 + (J.n + 7) / 8 + 16 : 0);
+}
+
+// compress_column_device of the k jobs `idx` names, without a wait until their
+// lengths are read.
+int compress_group(QuoinCtx* c, cudaStream_t st, QuoinB200CompressJob* jobs, const size_t* idx, size_t k,
+                   const QuoinConfig* cfg) {
+  int lv;
+  uint64_t bs;
+  uint8_t plog2;
+  int rc = check_level(cfg, &lv, &bs, &plog2);
+  if (rc) return rc;
+  const uint64_t bound_bs = bs;
+  if (bs > kMaxBlockValues) bs = kMaxBlockValues;
+  const int level = lv & 0xFF;
+  const bool sample = (lv & kSelectSample) != 0;
+  std::vector<EncCol> cols(k);
+  std::vector<EncLane> lanes;
+  bool decimals = false;
+  uint64_t o_res = 0;
+  // The columns and lanes with their pieces of the arena at `base`; returns
+  // the arena's size (with no base: only that).
+  auto lay = [&](uint8_t* base) {
+    BumpAlloc ba;
+    auto bytes = [&](uint64_t n) { return base + ba.take(n); };
+    auto words = [&](uint64_t n) { return reinterpret_cast<uint64_t*>(bytes(n * 8)); };
+    lanes.clear();
+    o_res = ba.take(k * 3 * 8);
+    for (size_t i = 0; i < k; i++) {
+      const QuoinB200CompressJob& J = jobs[idx[i]];
+      const int wire = J.wire_dtype;
+      const uint64_t n = J.n;
+      EncCol C = {};
+      C.values = static_cast<const uint8_t*>(J.d_values);
+      C.bm = J.d_validity;
+      C.n = n;
+      C.res = reinterpret_cast<uint64_t*>(base + o_res) + 3 * i;
+      C.dst = J.d_dst;
+      C.dtype = wire;
+      C.nl = wire == WT_DEC128 ? 2 : wire == WT_DEC256 ? 4 : 0;
+      C.lane0 = (int)lanes.size();
+      C.stride = n;
+      if (C.bm) C.rank = words((n + 31) / 32);
+      memcpy(C.hdr, "FCR1", 4);
+      C.hdr[4] = 2;
+      C.hdr[5] = C.nl ? 2 : 0;  // and 1 with nulls
+      C.hdr[6] = C.nl ? 0 : plog2;
+      C.hdr[7] = (uint8_t)wire;
+      for (int b = 0; b < 8; b++) C.hdr[8 + b] = (uint8_t)(n >> (8 * b));
+      if (C.nl) {
+        decimals = true;
+        C.hdr[16] = (uint8_t)J.scale;
+        C.hdr[17] = J.precision;
+        C.hdr[18] = (uint8_t)C.nl;
+        C.vmin = words(5);
+        C.parts = words(enc_col_part_words());
+      }
+      // no copy where the values are the lane
+      const bool direct = !C.nl && !C.bm && lane_bytes_h(wire) == 8 && ((uintptr_t)J.d_values & 7) == 0;
+      const int nlanes = C.nl ? C.nl : 1, dtype = C.nl ? WT_U64 : wire;
+      if (!direct) C.lane = words(nlanes * n + 8);
+      cols[i] = C;
+      const bool fl = dtype == WT_F64 || dtype == WT_F32;
+      const uint64_t maxb = max_blocks_for(n, bs), nwin = (n + kBaseQuantumH - 1) / kBaseQuantumH;
+      for (int q = 0; q < nlanes; q++) {
+        EncLane L = {};
+        L.v = direct ? static_cast<const uint64_t*>(J.d_values) : C.lane + q * n;
+        L.n = n;
+        L.d_n = C.bm ? C.res + 2 : nullptr;
+        L.fixed_bs = bs;
+        L.items = sub_stats_items(n, bs);
+        L.dtype = dtype;
+        L.ss = bytes((L.items + 1) * sub_stats_bytes());
+        if (fl) {
+          L.fms = bytes((L.items + 1) * fm_stats_bytes());
+          L.smp16 = words(n / 16 + 2);
+        }
+        L.rdr = bytes((L.items + 1) * rd_rec_bytes());
+        L.blk = bytes(maxb * blk_rec_bytes());
+        if (level >= 2) L.ent = bytes(maxb * ent_rec_bytes());
+        L.grow = bytes(nwin + 16);
+        L.winbits = reinterpret_cast<uint32_t*>(bytes((nwin + 1) * kWinWords * 4));
+        L.nb = reinterpret_cast<uint32_t*>(bytes(64));
+        L.w2b = reinterpret_cast<uint32_t*>(bytes(nwin * 4 + 16));
+        L.frames = reinterpret_cast<FrameDesc*>(bytes(maxb * sizeof(FrameDesc)));
+        L.scratch = bytes(n * kEncScratchPerValue + 256);
+        L.out = J.d_dst;
+        L.out_cap = J.dst_cap;
+        if (C.nl) {
+          L.nest.pos = C.res;
+          L.nest.out = J.d_dst;
+          L.nest.cap = J.dst_cap;
+          L.nest.d_n = L.d_n;
+          memcpy(L.nest.hdr.b, C.hdr, 16);
+          L.nest.hdr.b[5] = 0;
+          L.nest.hdr.b[6] = plog2;
+          L.nest.hdr.b[7] = WT_U64;
+        }
+        lanes.push_back(L);
+      }
+    }
+    return ba.off;
+  };
+  if (c->ensure(S_BSCR, lay(nullptr)) != cudaSuccess) return kGroupNoRoom;
+  uint8_t* base = c->p<uint8_t>(S_BSCR);
+  lay(base);
+  EncMaps M;
+  for (size_t q = 0; q < lanes.size(); q++)
+    map_lane(M, (uint32_t)q, lanes[q].n, bs, lanes[q].dtype, max_blocks_for(lanes[q].n, bs));
+  // the tables, one copy
+  EncGroup G = {};
+  BumpAlloc tb;
+  const uint64_t t_cols = tb.take(k * sizeof(EncCol)), t_lanes = tb.take(lanes.size() * sizeof(EncLane));
+  const std::vector<uint32_t>* maps[5] = {&M.fstats, &M.istats, &M.alp, &M.blocks, &M.units};
+  uint64_t t_maps[5];
+  for (int m = 0; m < 5; m++) t_maps[m] = tb.take(maps[m]->size() * 4);
+  std::vector<uint8_t> tables(tb.off);
+  memcpy(tables.data() + t_cols, cols.data(), k * sizeof(EncCol));
+  memcpy(tables.data() + t_lanes, lanes.data(), lanes.size() * sizeof(EncLane));
+  for (int m = 0; m < 5; m++)
+    if (!maps[m]->empty()) memcpy(tables.data() + t_maps[m], maps[m]->data(), maps[m]->size() * 4);
+  CK(c->ensure(S_BHOST, tb.off));
+  uint8_t* dt = c->p<uint8_t>(S_BHOST);
+  CK(cudaMemcpyAsync(dt, tables.data(), tb.off, cudaMemcpyHostToDevice, st));
+  G.cols = reinterpret_cast<EncCol*>(dt + t_cols);
+  G.lanes = reinterpret_cast<EncLane*>(dt + t_lanes);
+  G.ncols = (unsigned)k;
+  G.nlanes = (unsigned)lanes.size();
+  const uint32_t** mp[5] = {&G.fstats, &G.istats, &G.alp, &G.blocks, &G.units};
+  unsigned* mn[5] = {&G.nfstats, &G.nistats, &G.nalp, &G.nblocks, &G.nunits};
+  for (int m = 0; m < 5; m++) {
+    *mp[m] = reinterpret_cast<uint32_t*>(dt + t_maps[m]);
+    *mn[m] = (unsigned)maps[m]->size();
+  }
+  launch_begin_cols(G.cols, (int)k, decimals, st);
+  launch_encode_group(G, level, level >= 2, sample, st);
+  std::vector<uint64_t> res(3 * k);
+  CK(cudaMemcpyAsync(res.data(), base + o_res, k * 24, cudaMemcpyDeviceToHost, st));
+  CK(cudaGetLastError());
+  CK(cudaStreamSynchronize(st));
+  for (size_t i = 0; i < k; i++) {
+    QuoinB200CompressJob& J = jobs[idx[i]];
+    const uint64_t total = res[3 * i] + res[3 * i + 1];
+    J.out_len = total;
+    J.status = QUOIN_OK;
+    if (total > J.dst_cap) {
+      J.status = QUOIN_ERR_BUFFER_TOO_SMALL;
+      if (cols[i].nl) J.out_len = column_bound(J.wire_dtype, J.n, res[3 * i + 2] < J.n, bound_bs);
+    }
+  }
+  return QUOIN_OK;
+}
+
 // Host-buffer compress of a typed column (wire dtype, native little-endian values).
 int compress_host(QuoinCtx* c, int wire, uint64_t n, const void* values, const uint8_t* validity, int8_t scale,
                   uint8_t precision, const QuoinConfig* cfg, uint8_t* dst, size_t dst_cap, size_t* out_len) {
@@ -2080,6 +2247,31 @@ const QuoinConfig kFastCfg = {QUOIN_LEVEL_FAST, 0, 16};
 // ===========================================================================
 // C ABI
 // ===========================================================================
+// The batch calls' side of the groups (qb_batch.cpp).
+bool qb::batch_group_takes(const QuoinB200CompressJob& job, const QuoinConfig* cfg) {
+  int level;
+  uint64_t bs;
+  uint8_t plog2;
+  return check_level(cfg, &level, &bs, &plog2) == QUOIN_OK && group_takes(job, bs);
+}
+bool qb::batch_compress_group(QuoinCtx* c, QuoinB200CompressJob* jobs, const size_t* idx, size_t k,
+                              const QuoinConfig* cfg) {
+  std::lock_guard<std::mutex> l(c->mu);
+  DeviceScope ds(c->device);
+  int rc = QUOIN_ERR_PANIC;
+  try {
+    rc = compress_group(c, c->stream, jobs, idx, k, cfg);
+  } catch (...) {
+  }
+  if (rc == kGroupNoRoom) return false;
+  if (rc != QUOIN_OK)
+    for (size_t i = 0; i < k; i++) {
+      jobs[idx[i]].out_len = 0;
+      jobs[idx[i]].status = rc;
+    }
+  return true;
+}
+
 extern "C" {
 
 const char* quoin_version(void) { return "quoin-b200 0.1.0 (sm_100a)"; }

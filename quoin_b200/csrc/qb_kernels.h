@@ -4,9 +4,10 @@
 #include <cstdint>
 #include <cuda_runtime.h>
 
-#include "qb_layout.h"
+#include <vector>
 
-struct QuoinCtx;
+#include "../../include/quoin.h"
+#include "qb_layout.h"
 
 namespace qb {
 
@@ -309,6 +310,7 @@ struct NestedLane {
   uint64_t* pos = nullptr;
   uint8_t* out = nullptr;
   uint64_t cap = 0;
+  const uint64_t* d_n = nullptr;  // the header's value count, when only the device knows it
   Bytes16 hdr;
 };
 // `base` (device) holds the byte offset at which the first frame starts (for a
@@ -324,6 +326,57 @@ void launch_emit(const uint64_t* lane, const FrameDesc* frames, const uint32_t* 
                  const uint32_t* w2b, uint64_t n, uint64_t fixed_bs, int dtype, const void* ss, const void* fms,
                  const void* rdr, const void* blk, uint8_t* scratch, uint8_t* out, uint64_t out_cap, const void* ent,
                  cudaStream_t st);
+
+// ---- a group of columns of one batch call (qb_lower.cu, qb_encode.cu) ----
+struct EncCol {
+  const uint8_t* values;
+  const uint8_t* bm;  // null: no nulls
+  uint64_t n;
+  uint64_t* rank;
+  uint64_t* lane;    // its lane (a decimal's limbs, `stride` apart); null: the values are the lane
+  uint64_t* res;     // [0] stream bytes before the frames (a decimal's whole length), [1] frames, [2] valid values
+  uint8_t* dst;
+  uint64_t* vmin;    // a decimal's minimum (4 words and one of scratch)
+  uint64_t* parts;   // enc_col_part_words()
+  uint64_t stride;
+  int32_t dtype, nl;  // nl: a decimal's limbs, else 0
+  int32_t lane0;      // the first of its lanes in EncGroup::lanes
+  uint8_t hdr[20];
+};
+struct EncLane {
+  const uint64_t* v;
+  uint64_t n;  // a bound when d_n gives the count
+  const uint64_t* d_n;
+  uint64_t fixed_bs, items;
+  int32_t dtype;
+  void *ss, *fms, *rdr, *blk, *ent;
+  uint64_t* smp16;
+  uint8_t* grow;
+  uint32_t *winbits, *nb, *w2b;
+  FrameDesc* frames;
+  uint8_t *scratch, *out;
+  uint64_t out_cap;
+  NestedLane nest;
+};
+struct EncMaps {  // host: a launch's CTAs, lane << 16 | the CTA's place among the lane's
+  std::vector<uint32_t> fstats, istats, alp, blocks, units;
+};
+// A lane of at most kSmallWords blocks and 2^20 values: no place exceeds 16 bits.
+void map_lane(EncMaps& M, uint32_t lane, uint64_t n, uint64_t fixed_bs, int dtype, uint64_t max_blocks);
+struct EncGroup {  // EncMaps on the device
+  const EncLane* lanes;
+  const EncCol* cols;
+  const uint32_t *fstats, *istats, *alp, *blocks, *units;
+  unsigned nlanes, ncols, nfstats, nistats, nalp, nblocks, nunits;
+};
+// Whether a column may be in a group; and a group's columns `idx` of `jobs`,
+// false when there was no device memory for all of them at once.
+bool batch_group_takes(const QuoinB200CompressJob& job, const QuoinConfig* cfg);
+bool batch_compress_group(QuoinCtx* c, QuoinB200CompressJob* jobs, const size_t* idx, size_t k,
+                          const QuoinConfig* cfg);
+uint64_t enc_col_part_words();
+void launch_begin_cols(const EncCol* cols, int ncols, bool decimals, cudaStream_t st);
+void launch_encode_group(const EncGroup& G, int level, bool ent, bool sample, cudaStream_t st);
 
 // ---- lowering / validity (qb_lower.cu) ----
 // Lower n native values (dtype width) to the u64 lane, keeping only positions

@@ -31,8 +31,9 @@ __device__ inline uint32_t bm_word_at(const uint8_t* bm, uint64_t w, uint64_t n)
 // A warp lowers 8 bitmap words (256 positions) per step: lanes 0-7 fetch the
 // words and their ranks, every lane loads its 8 values up front, then each
 // valid value goes to lane[rank].
-__global__ void k_lower(const uint8_t* __restrict__ values, int dtype, const uint8_t* __restrict__ bm,
-                        const uint64_t* __restrict__ word_rank, uint64_t n, uint64_t* __restrict__ lane) {
+__device__ __forceinline__ void lower_words(const uint8_t* __restrict__ values, int dtype,
+                                            const uint8_t* __restrict__ bm, const uint64_t* __restrict__ word_rank,
+                                            uint64_t n, uint64_t* __restrict__ lane) {
   uint64_t nw = (n + 31) / 32;
   int l = threadIdx.x & 31;
   uint32_t below = (1u << l) - 1u;
@@ -61,6 +62,11 @@ __global__ void k_lower(const uint8_t* __restrict__ values, int dtype, const uin
       else if ((bits >> l) & 1u) lane[rank + __popc(bits & below)] = vals[q];
     }
   }
+}
+
+__global__ void k_lower(const uint8_t* __restrict__ values, int dtype, const uint8_t* __restrict__ bm,
+                        const uint64_t* __restrict__ word_rank, uint64_t n, uint64_t* __restrict__ lane) {
+  lower_words(values, dtype, bm, word_rank, n, lane);
 }
 
 static unsigned grid_for_words(uint64_t n) {
@@ -131,9 +137,8 @@ __device__ Limbs<NL> block_min(Limbs<NL> m, Limbs<NL>* s_v) {
 // 10,000,019 Decimal128 values; reading them takes 25 us at the copy rate.
 constexpr int kVminParts = 148 * 6;
 template <int NL>
-__global__ void __launch_bounds__(256) k_decimal_vmin_partial(const uint64_t* __restrict__ values,
-                                                              const uint8_t* __restrict__ bm, uint64_t n,
-                                                              uint64_t* __restrict__ tmp) {
+__device__ __forceinline__ void vmin_partial(const uint64_t* __restrict__ values, const uint8_t* __restrict__ bm,
+                                             uint64_t n, uint64_t* __restrict__ tmp) {
   __shared__ Limbs<NL> s_v[32];
   Limbs<NL> best = most_positive<NL>();
   const uint64_t step = (uint64_t)gridDim.x * blockDim.x;
@@ -158,8 +163,14 @@ __global__ void __launch_bounds__(256) k_decimal_vmin_partial(const uint64_t* __
     for (int k = 0; k < NL; k++) tmp[blockIdx.x * NL + k] = best.l[k];
 }
 template <int NL>
-__global__ void __launch_bounds__(1024) k_decimal_vmin_final(const uint64_t* __restrict__ tmp, int nparts, bool any,
-                                                             uint64_t* __restrict__ vmin) {
+__global__ void __launch_bounds__(256) k_decimal_vmin_partial(const uint64_t* __restrict__ values,
+                                                              const uint8_t* __restrict__ bm, uint64_t n,
+                                                              uint64_t* __restrict__ tmp) {
+  vmin_partial<NL>(values, bm, n, tmp);
+}
+template <int NL>
+__device__ __forceinline__ void vmin_final(const uint64_t* __restrict__ tmp, int nparts, bool any,
+                                           uint64_t* __restrict__ vmin) {
   __shared__ Limbs<NL> s_v[32];
   Limbs<NL> m = most_positive<NL>();
   for (int b = threadIdx.x; b < nparts; b += blockDim.x) {
@@ -176,6 +187,11 @@ __global__ void __launch_bounds__(1024) k_decimal_vmin_final(const uint64_t* __r
       if (k == (int)threadIdx.x && any) v = m.l[k];
     vmin[threadIdx.x] = v;
   }
+}
+template <int NL>
+__global__ void __launch_bounds__(1024) k_decimal_vmin_final(const uint64_t* __restrict__ tmp, int nparts, bool any,
+                                                             uint64_t* __restrict__ vmin) {
+  vmin_final<NL>(tmp, nparts, any, vmin);
 }
 
 uint64_t decimal_vmin_tmp_words() { return 4ull * kVminParts; }
@@ -211,9 +227,10 @@ void launch_put_decimal_header(uint8_t* dst, const Bytes19& head, int nl, const 
 }
 
 // limbs[k * stride + j] = limb k of (v_i - vmin) for the j-th valid value i.
-__global__ void k_decimal_split(const uint8_t* __restrict__ values, int nl, const uint8_t* __restrict__ bm,
-                                const uint64_t* __restrict__ word_rank, uint64_t n, const uint64_t* __restrict__ vmin,
-                                uint64_t* __restrict__ limbs, uint64_t stride) {
+__device__ __forceinline__ void split_words(const uint8_t* __restrict__ values, int nl, const uint8_t* __restrict__ bm,
+                                            const uint64_t* __restrict__ word_rank, uint64_t n,
+                                            const uint64_t* __restrict__ vmin, uint64_t* __restrict__ limbs,
+                                            uint64_t stride) {
   uint64_t nw = (n + 31) / 32, nbytes = (n + 7) / 8;
   int l = threadIdx.x & 31;
   uint64_t warp = ((uint64_t)blockIdx.x * blockDim.x + threadIdx.x) >> 5;
@@ -244,6 +261,12 @@ __global__ void k_decimal_split(const uint8_t* __restrict__ values, int nl, cons
       borrow = b1 | b2;
     }
   }
+}
+
+__global__ void k_decimal_split(const uint8_t* __restrict__ values, int nl, const uint8_t* __restrict__ bm,
+                                const uint64_t* __restrict__ word_rank, uint64_t n, const uint64_t* __restrict__ vmin,
+                                uint64_t* __restrict__ limbs, uint64_t stride) {
+  split_words(values, nl, bm, word_rank, n, vmin, limbs, stride);
 }
 
 void launch_decimal_split(const uint8_t* values, int nlimbs, const uint8_t* bm, const uint64_t* word_rank,
@@ -350,7 +373,8 @@ __global__ void k_bitmap_transitions(const uint8_t* __restrict__ bm, uint64_t n,
     if (t) atomicAdd(count, t);
   }
 }
-// A short column's bitmap (at most kSmallWords 32-bit words) in one CTA of
+// A short column's bitmap (at most kSmallWords 32-bit words, or such a stretch
+// of a longer one from word w0 on) in one CTA of
 // 1,024 threads: every word's exclusive valid rank, the valid count (returned)
 // and the 0/1 transition count (optional) -- k_word_popcount, the rank scan and
 // k_bitmap_transitions in one launch, since short columns pay per launch.
@@ -359,11 +383,14 @@ struct SmallWords {
   uint32_t tm[kSmallPer];  // their transition masks (trans_mask)
   uint32_t first, per;     // the first of them, words a thread
 };
-__device__ inline SmallWords small_words(const uint8_t* __restrict__ bm, uint64_t n) {
+__device__ inline uint32_t small_end(uint64_t n, uint32_t w0) {
+  return (uint32_t)qmin((n + 31) / 32, (uint64_t)w0 + kSmallWords);
+}
+__device__ inline SmallWords small_words(const uint8_t* __restrict__ bm, uint64_t n, uint32_t w0 = 0) {
   SmallWords s;
-  const uint32_t nw = (uint32_t)((n + 31) / 32);
-  s.per = (nw + 1023) / 1024;
-  s.first = threadIdx.x * s.per;
+  const uint32_t nw = small_end(n, w0);
+  s.per = (nw - w0 + 1023) / 1024;
+  s.first = w0 + threadIdx.x * s.per;
   uint32_t prev = s.first && s.first <= nw ? bm_word_at(bm, s.first - 1, n) >> 31 : 0u;
 #pragma unroll
   for (uint32_t k = 0; k < kSmallPer; k++) s.w[k] = k < s.per && s.first + k < nw ? bm_word_at(bm, s.first + k, n) : 0u;
@@ -380,11 +407,13 @@ __device__ inline SmallWords small_words(const uint8_t* __restrict__ bm, uint64_
   }
   return s;
 }
-// Ranks, the valid count (returned) and the number of transitions.
-__device__ uint64_t valid_small(const SmallWords& S, uint64_t n, uint64_t* __restrict__ rank, uint32_t* trans) {
+// Ranks (from rank0 on), the valid count with rank0 (returned) and the number
+// of transitions.
+__device__ uint64_t valid_small(const SmallWords& S, uint64_t n, uint64_t* __restrict__ rank, uint32_t* trans,
+                                uint32_t w0 = 0, uint64_t rank0 = 0) {
   __shared__ uint64_t wsum[32];
   __shared__ uint32_t wtr[32], s_tr;
-  uint32_t nw = (uint32_t)((n + 31) / 32), t = threadIdx.x, l = t & 31, warp = t >> 5;
+  uint32_t nw = small_end(n, w0), t = threadIdx.x, l = t & 31, warp = t >> 5;
   uint32_t s = 0, tr = 0;
 #pragma unroll
   for (uint32_t k = 0; k < kSmallPer; k++) {
@@ -402,14 +431,14 @@ __device__ uint64_t valid_small(const SmallWords& S, uint64_t n, uint64_t* __res
     if (l == 0) s_tr = y;
   }
   __syncthreads();
-  uint64_t run = (warp ? wsum[warp - 1] : 0ull) + inc - s;
+  uint64_t run = rank0 + (warp ? wsum[warp - 1] : 0ull) + inc - s;
 #pragma unroll
   for (uint32_t k = 0; k < kSmallPer; k++) {
     if (k < S.per && S.first + k < nw) rank[S.first + k] = run;
     run += __popc(S.w[k]);
   }
   *trans = s_tr;
-  return wsum[31];
+  return rank0 + wsum[31];
 }
 __global__ void __launch_bounds__(1024) k_valid_small(const uint8_t* __restrict__ bm, uint64_t n,
                                                       uint64_t* __restrict__ rank, uint64_t* __restrict__ total,
@@ -492,27 +521,24 @@ uint64_t validity_tmp_words(uint64_t n) {
   return 3 * nw + scan_tiles(nw) + 8;
 }
 
-// The validity blob of a short column (at most kSmallWords words) in one CTA
-// of 1,024 threads: the three passes above (last transitions + max scan, run
-// bytes + sum scan, write) with block scans in place of the grid scans.
-// place(blob length) gives the blob's destination.
-template <class P>
-__device__ void vb_small(const SmallWords& S, const uint8_t* __restrict__ bm, uint64_t n, bool raw, P place) {
+// The validity blob of a short column in one CTA of 1,024 threads: the three
+// passes above (last transitions + max scan, run bytes + sum scan, write) with
+// block scans in place of the grid scans.  place(blob length) gives the blob's
+// destination.  A longer bitmap goes stretch by stretch, first for the blob's
+// size and then to write it.
+struct VbRuns {
+  uint64_t last, bytes;  // the last transition so far and the bytes of the runs that end at one
+};
+// This stretch's runs: in *r the totals, *prev and the result are the last
+// transition and the run bytes before this thread's words.
+__device__ uint64_t vb_scan(const SmallWords& S, VbRuns* r, uint64_t* prev0) {
   __shared__ uint64_t wa[32], wb[32];
-  if (raw) {  // proven by the transitions
-    uint8_t* out = place(1 + (n + 7) / 8);
-    if (threadIdx.x == 0) out[0] = 0;
-#pragma unroll 4
-    for (uint64_t i = threadIdx.x; i < (n + 7) / 8; i += 1024) out[1 + i] = bm[i];
-    return;
-  }
   uint32_t t = threadIdx.x, l = t & 31, warp = t >> 5;
-  const uint32_t* tm = S.tm;
   uint64_t mx = 0;
 #pragma unroll
   for (uint32_t k = 0; k < kSmallPer; k++) {
     uint32_t w = S.first + k;
-    if (tm[k]) mx = (uint64_t)w * 32 + (31 - __clz(tm[k]));  // words ascend: the thread's last transition
+    if (S.tm[k]) mx = (uint64_t)w * 32 + (31 - __clz(S.tm[k]));  // words ascend: the thread's last transition
   }
   // exclusive max scan of the threads' last transitions (positions ascend, 0 = none yet)
   uint64_t inc = mx;
@@ -533,13 +559,14 @@ __device__ void vb_small(const SmallWords& S, const uint8_t* __restrict__ bm, ui
     wa[l] = x;
   }
   __syncthreads();
-  uint64_t before = warp ? wa[warp - 1] : 0ull;
-  uint64_t prev0 = ex > before ? ex : before, t_last = wa[31];
+  const uint64_t before = warp ? wa[warp - 1] : 0ull;
+  *prev0 = qmax(r->last, qmax(ex, before));
+  r->last = qmax(r->last, wa[31]);
   // bytes of the runs that end at this thread's transitions, then their offsets
-  uint64_t prev = prev0, s = 0;
+  uint64_t prev = *prev0, s = 0;
 #pragma unroll
   for (uint32_t k = 0; k < kSmallPer; k++) {
-    uint32_t tt = tm[k];
+    uint32_t tt = S.tm[k];
     uint32_t w = S.first + k;
     while (tt) {
       uint64_t p = (uint64_t)w * 32 + (__ffs(tt) - 1);
@@ -548,56 +575,91 @@ __device__ void vb_small(const SmallWords& S, const uint8_t* __restrict__ bm, ui
       prev = p;
     }
   }
-  uint64_t inc2 = s;
-  for (int o = 1; o < 32; o <<= 1) {
-    uint64_t u = __shfl_up_sync(0xffffffffu, inc2, o);
-    if ((int)l >= o) inc2 += u;
-  }
+  const uint64_t inc2 = warp_incl_scan(s);
   if (l == 31) wb[warp] = inc2;
   __syncthreads();
-  if (warp == 0) {
-    uint64_t x = wb[l];
-    for (int o = 1; o < 32; o <<= 1) {
-      uint64_t u = __shfl_up_sync(0xffffffffu, x, o);
-      if ((int)l >= o) x += u;
-    }
-    wb[l] = x;
-  }
+  if (warp == 0) wb[l] = warp_incl_scan(wb[l]);
   __syncthreads();
-  uint64_t run_bytes = wb[31], raw_len = (n + 7) / 8;
-  uint64_t rle_len = run_bytes + varint_len(n - t_last);
-  bool rle = rle_len < raw_len;
-  uint8_t* out = place(1 + (rle ? rle_len : raw_len));
-  if (t == 0) out[0] = rle ? 1 : 0;
-  if (!rle) {
-    for (uint64_t i = t; i < raw_len; i += blockDim.x) out[1 + i] = bm[i];
-    return;
-  }
-  uint64_t pos = 1 + (warp ? wb[warp - 1] : 0ull) + inc2 - s;
-  prev = prev0;
+  const uint64_t at = r->bytes + (warp ? wb[warp - 1] : 0ull) + inc2 - s;
+  r->bytes += wb[31];
+  return at;
+}
+__device__ inline uint64_t vb_leb(uint8_t* out, uint64_t pos, uint64_t v) {
+  do {
+    uint8_t b = (uint8_t)(v & 0x7f);
+    v >>= 7;
+    out[pos++] = v ? (b | 0x80) : b;
+  } while (v);
+  return pos;
+}
+__device__ inline void vb_put(const SmallWords& S, uint64_t prev, uint64_t pos, uint8_t* out) {
 #pragma unroll
   for (uint32_t k = 0; k < kSmallPer; k++) {
-    uint32_t tt = tm[k];
+    uint32_t tt = S.tm[k];
     uint32_t w = S.first + k;
     while (tt) {
       uint64_t p = (uint64_t)w * 32 + (__ffs(tt) - 1);
       tt &= tt - 1;
-      uint64_t v = p - prev;
-      do {
-        uint8_t b = (uint8_t)(v & 0x7f);
-        v >>= 7;
-        out[pos++] = v ? (b | 0x80) : b;
-      } while (v);
+      pos = vb_leb(out, pos, p - prev);
       prev = p;
     }
   }
-  if (t == 0) {
-    uint64_t v = n - t_last, q = 1 + run_bytes;
-    do {
-      uint8_t b = (uint8_t)(v & 0x7f);
-      v >>= 7;
-      out[q++] = v ? (b | 0x80) : b;
-    } while (v);
+}
+__device__ inline void vb_raw(const uint8_t* __restrict__ bm, uint64_t n, uint8_t* out) {
+  if (threadIdx.x == 0) out[0] = 0;
+#pragma unroll 4
+  for (uint64_t i = threadIdx.x; i < (n + 7) / 8; i += 1024) out[1 + i] = bm[i];
+}
+template <class P>
+__device__ void vb_small(const SmallWords& S, const uint8_t* __restrict__ bm, uint64_t n, bool raw, P place) {
+  const uint64_t raw_len = (n + 7) / 8;
+  if (raw) {  // proven by the transitions
+    vb_raw(bm, n, place(1 + raw_len));
+    return;
+  }
+  VbRuns r = {0, 0};
+  uint64_t prev;
+  uint64_t at = vb_scan(S, &r, &prev);
+  const uint64_t rle_len = r.bytes + varint_len(n - r.last);
+  const bool rle = rle_len < raw_len;
+  uint8_t* out = place(1 + (rle ? rle_len : raw_len));
+  if (!rle) {
+    vb_raw(bm, n, out);
+    return;
+  }
+  if (threadIdx.x == 0) {
+    out[0] = 1;
+    vb_leb(out, 1 + r.bytes, n - r.last);
+  }
+  vb_put(S, prev, 1 + at, out);
+}
+template <class P>
+__device__ void vb_long(const uint8_t* __restrict__ bm, uint64_t n, bool raw, P place) {
+  const uint32_t nw = (uint32_t)((n + 31) / 32);
+  const uint64_t raw_len = (n + 7) / 8;
+  VbRuns r = {0, 0};
+  uint64_t prev;
+  for (uint32_t w0 = 0; !raw && w0 < nw; w0 += kSmallWords) {
+    vb_scan(small_words(bm, n, w0), &r, &prev);
+    __syncthreads();
+  }
+  const uint64_t rle_len = r.bytes + varint_len(n - r.last);
+  const bool rle = !raw && rle_len < raw_len;
+  uint8_t* out = place(1 + (rle ? rle_len : raw_len));
+  if (!rle) {
+    vb_raw(bm, n, out);
+    return;
+  }
+  if (threadIdx.x == 0) {
+    out[0] = 1;
+    vb_leb(out, 1 + r.bytes, n - r.last);
+  }
+  r = {0, 0};
+  for (uint32_t w0 = 0; w0 < nw; w0 += kSmallWords) {
+    const SmallWords S = small_words(bm, n, w0);
+    const uint64_t at = vb_scan(S, &r, &prev);
+    vb_put(S, prev, 1 + at, out);
+    __syncthreads();
   }
 }
 __global__ void __launch_bounds__(1024) k_vb_small(const uint8_t* __restrict__ bm, uint64_t n,
@@ -638,6 +700,74 @@ void launch_begin_small(const uint8_t* bm, uint64_t n, uint64_t* rank, uint64_t*
                         uint64_t* d_base, cudaStream_t st) {
   k_begin_small<<<1, 1024, 0, st>>>(bm, n, rank, total, dst, hdr, d_base);
   count_launches(1);
+}
+
+// ---------------------------------------------------------------------------
+// A group of columns of one batch call (EncCol): what the kernels above do for
+// a column, for all of them in one launch each.  One column's launches of 2-8 us
+// and its wait for the valid count were most of what a short column cost.
+// ---------------------------------------------------------------------------
+// CTAs a column: 192 columns of up to 1,048,576 values take 1,282 us with 32
+// (a long column's lowering then is 128 dependent steps), 1,211 with 64 and
+// 1,207 with 128 (more CTAs that find nothing to do).
+constexpr int kColParts = 64;
+__global__ void __launch_bounds__(256) k_cols_vmin(const EncCol* __restrict__ cols) {
+  const EncCol& C = cols[blockIdx.y];
+  const uint64_t* v = reinterpret_cast<const uint64_t*>(C.values);
+  if (C.nl == 2) vmin_partial<2>(v, C.bm, C.n, C.parts);
+  else if (C.nl == 4) vmin_partial<4>(v, C.bm, C.n, C.parts);
+}
+__global__ void __launch_bounds__(1024) k_cols_begin(const EncCol* __restrict__ cols) {
+  const EncCol& C = cols[blockIdx.x];
+  const int t = threadIdx.x, nl = C.nl;
+  const uint64_t n = C.n;
+  const uint32_t nw = (uint32_t)((n + 31) / 32);
+  uint64_t nv = n, trans = 0;
+  for (uint32_t w0 = 0; C.bm && w0 < nw; w0 += kSmallWords) {
+    uint32_t tr;
+    if (w0 == 0) nv = 0;
+    nv = valid_small(small_words(C.bm, n, w0), n, C.rank, &tr, w0, nv);
+    trans += tr;
+    __syncthreads();
+  }
+  const uint64_t head = nl ? 19 + 8ull * nl : 16;
+  uint8_t* dst = C.dst;
+  if (t < (nl ? 19 : 16)) dst[t] = t == 5 ? C.hdr[5] | (nv < n ? 1 : 0) : C.hdr[t];
+  if (nl) {
+    if (nl == 2) vmin_final<2>(C.parts, kColParts, nv != 0, C.vmin);
+    else vmin_final<4>(C.parts, kColParts, nv != 0, C.vmin);
+    __syncthreads();
+    if (t < 8 * nl) dst[19 + t] = (uint8_t)(C.vmin[t >> 3] >> (8 * (t & 7)));
+  }
+  if (t == 0) {
+    C.res[0] = head;
+    C.res[1] = 0;
+    C.res[2] = nv;
+  }
+  if (nv == n) return;  // all valid: no bitmap in the stream
+  auto place = [&](uint64_t len) {
+    const uint32_t vl = varint_len(len);
+    if (t == 0) {
+      vb_leb(dst, head, len);
+      C.res[0] = head + vl + len;
+    }
+    return dst + head + vl;
+  };
+  const bool raw = trans + 1 >= (n + 7) / 8;
+  if (nw <= kSmallWords) vb_small(small_words(C.bm, n), C.bm, n, raw, place);
+  else vb_long(C.bm, n, raw, place);
+}
+__global__ void __launch_bounds__(256) k_cols_lower(const EncCol* __restrict__ cols) {
+  const EncCol& C = cols[blockIdx.y];
+  if (C.nl) split_words(C.values, C.nl, C.bm, C.rank, C.n, C.vmin, C.lane, C.stride);
+  else if (C.lane) lower_words(C.values, C.dtype, C.bm, C.rank, C.n, C.lane);
+}
+uint64_t enc_col_part_words() { return 4ull * kColParts; }
+void launch_begin_cols(const EncCol* cols, int ncols, bool decimals, cudaStream_t st) {
+  if (decimals) k_cols_vmin<<<dim3(kColParts, ncols), 256, 0, st>>>(cols);
+  k_cols_begin<<<ncols, 1024, 0, st>>>(cols);
+  k_cols_lower<<<dim3(kColParts, ncols), 256, 0, st>>>(cols);
+  count_launches(decimals ? 3 : 2);
 }
 
 void launch_validity_blob(const uint8_t* bm, uint64_t n, uint64_t* tmp, uint64_t* tile_tmp, uint8_t* out,
