@@ -2920,9 +2920,10 @@ __global__ void k_finalize(const uint64_t* __restrict__ lane, const uint8_t* __r
 
 // Decimal recombine (reference decimal.rs:218-246, 379-408): value = vmin +
 // (limb0 | limb1 << 64 | ...) with carries, scattered through the bitmap.
-__global__ void k_decimal_combine(const uint64_t* __restrict__ limbs, uint64_t limb_stride, int nlimbs,
-                                  const uint64_t* __restrict__ vmin, const uint8_t* __restrict__ bm,
-                                  const uint64_t* __restrict__ word_rank, uint64_t n, uint8_t* __restrict__ out) {
+__device__ __forceinline__ void combine_words(const uint64_t* __restrict__ limbs, uint64_t limb_stride, int nlimbs,
+                                              const uint64_t* __restrict__ vmin, const uint8_t* __restrict__ bm,
+                                              const uint64_t* __restrict__ word_rank, uint64_t n,
+                                              uint8_t* __restrict__ out) {
   uint64_t nw = (n + 31) / 32, nbytes = (n + 7) / 8;
   int l = threadIdx.x & 31;
   uint64_t warp = ((uint64_t)blockIdx.x * blockDim.x + threadIdx.x) >> 5;
@@ -2955,6 +2956,18 @@ __global__ void k_decimal_combine(const uint64_t* __restrict__ limbs, uint64_t l
       o[k] = r;
     }
   }
+}
+
+__global__ void k_decimal_combine(const uint64_t* __restrict__ limbs, uint64_t limb_stride, int nlimbs,
+                                  const uint64_t* __restrict__ vmin, const uint8_t* __restrict__ bm,
+                                  const uint64_t* __restrict__ word_rank, uint64_t n, uint8_t* __restrict__ out) {
+  combine_words(limbs, limb_stride, nlimbs, vmin, bm, word_rank, n, out);
+}
+// All decimal columns of a batch, a row of CTAs each: 24 columns of up to
+// 1,048,576 values as 24 launches took 114 us and their gaps.
+__global__ void __launch_bounds__(256) k_cols_combine(const CombineCol* __restrict__ cols) {
+  const CombineCol& C = cols[blockIdx.y];
+  combine_words(C.limbs, C.stride, C.nl, C.vmin, C.bm, C.rank, C.n, C.out);
 }
 
 // ---------------------------------------------------------------------------
@@ -3047,6 +3060,12 @@ void launch_finalize(const uint64_t* lane, const uint8_t* bm, const uint64_t* wo
   unsigned g = (unsigned)qmin((nw + 7) / 8, 148ull * 32);
   if (g == 0) g = 1;
   k_finalize<<<g, 256, 0, st>>>(lane, bm, word_rank, n, dtype, out);
+  count_launches(1);
+}
+
+void launch_cols_combine(const CombineCol* cols, int ncols, uint64_t n_max, cudaStream_t st) {
+  const unsigned g = (unsigned)qmin((n_max + 2047) / 2048, 256);  // 8 words a warp
+  k_cols_combine<<<dim3(g ? g : 1, ncols), 256, 0, st>>>(cols);
   count_launches(1);
 }
 

@@ -586,6 +586,7 @@ __global__ void __launch_bounds__(kDpThreads) k_dp_cand_scan(const uint8_t* __re
                                                              const DpHead* __restrict__ H, int lane,
                                                              uint64_t* __restrict__ cnt, DpCand* __restrict__ slots) {
   __shared__ uint64_t s_warp[33];
+  if (blockIdx.x == 0 && threadIdx.x == 0) cnt[gridDim.x] = 0;  // the scan's last entry
   if (H->kind) {  // uniform over the CTA
     if (threadIdx.x == 0) cnt[blockIdx.x] = 0;
     return;
@@ -1148,7 +1149,7 @@ void launch_dp_candidates(const uint8_t* s, uint64_t buf_len, const DpHead* H, i
   // exclusive scan cnt[j + 1] - cnt[j] is chunk j's count
   uint64_t nchunks = dp_chunks(lane_frames_bytes);
   if (nchunks) k_dp_cand_scan<<<(unsigned)nchunks, kDpThreads, 0, st>>>(s, buf_len, H, lane, cnt, slots);
-  cudaMemsetAsync(cnt + nchunks, 0, 8, st);
+  else cudaMemsetAsync(cnt, 0, 8, st);
   launch_scan_sum(cnt, cnt, nchunks + 1, tile_tmp, d_ncand, st);
   if (nchunks)
     k_dp_cand_compact<<<(unsigned)nchunks, kDpThreads, 0, st>>>(s, buf_len, H, lane, cnt, slots, cap, cand);

@@ -4021,6 +4021,6 @@ void launch_frame_offsets(FrameDesc* frames, const uint32_t* nb, uint32_t max_bl
   scan_exclusive_u64(sizes_tmp, sizes_tmp, max_blocks, tile_tmp, total, st);
   if (nest.pos) k_nest_base<<<1, 32, 0, st>>>(nest, total, base);
   k_frame_apply<<<g, 256, 0, st>>>(frames, nb, sizes_tmp, base);
-  count_launches(nest.pos ? 6 : 5);
+  count_launches((nest.pos ? 3 : 2) + scan_launches(max_blocks));
 }
 }  // namespace qb

@@ -4,6 +4,7 @@
 // the C ABI of include/quoin.h (capi/src/lib.rs, capi/src/typed.rs).
 #include <cuda_runtime.h>
 
+#include <algorithm>
 #include <atomic>
 #include <cstddef>
 #include <cstdint>
@@ -1767,6 +1768,8 @@ struct BumpAlloc {  // carves 256-byte aligned pieces out of one buffer
   }
 };
 
+constexpr size_t kCombineCols = 4096;  // decimal columns of one launch
+
 int decode_queue(QuoinCtx* c, cudaStream_t st, QuoinB200DeviceDecodeJob* jobs, size_t nj) {
   for (size_t i = 0; i < nj; i++) {
     jobs[i].wire = 0;
@@ -1993,16 +1996,24 @@ int decode_queue(QuoinCtx* c, cudaStream_t st, QuoinB200DeviceDecodeJob* jobs, s
         }
         {  // decimal containers: vmin + the limbs, through the container's bitmap
           TimedRegion tr(T_FINALIZE, st);
+          std::vector<CombineCol> dec;
+          uint64_t n_max = 0;
           for (size_t t = 0; t < take.size(); t++) {
             const DpHead& h = H[take[t]];
-            if (!h.decimal || !col_ok[t]) continue;
-            int k0 = col_lane0[t];
+            if (!h.decimal || !col_ok[t] || h.n == 0) continue;
+            const int k0 = col_lane0[t];
             const bool bm = h.has_validity != 0;
-            launch_decimal_combine(limb_base + limb_off[k0], h.n, (int)h.nl,
-                                   reinterpret_cast<const uint64_t*>(bb + o_vmin) + 4 * t,
-                                   bm ? reinterpret_cast<const uint8_t*>(B.bm32 + lanes[k0].word0) : nullptr,
-                                   bm ? B.ranks + lanes[k0].word0 : nullptr, h.n,
-                                   static_cast<uint8_t*>(jobs[take[t]].d_values_out), st);
+            dec.push_back({limb_base + limb_off[k0], reinterpret_cast<const uint64_t*>(bb + o_vmin) + 4 * t,
+                           bm ? B.ranks + lanes[k0].word0 : nullptr,
+                           bm ? reinterpret_cast<const uint8_t*>(B.bm32 + lanes[k0].word0) : nullptr,
+                           static_cast<uint8_t*>(jobs[take[t]].d_values_out), h.n, h.n, (int64_t)h.nl});
+            n_max = h.n > n_max ? h.n : n_max;
+          }
+          for (size_t t = 0; t < dec.size(); t += kCombineCols) {  // a grid's rows
+            const size_t k = std::min(dec.size() - t, kCombineCols);
+            CK(c->ensure(S_VTMP, kCombineCols * sizeof(CombineCol)));
+            CK(cudaMemcpyAsync(c->p<void>(S_VTMP), dec.data() + t, k * sizeof(CombineCol), cudaMemcpyHostToDevice, st));
+            launch_cols_combine(c->p<CombineCol>(S_VTMP), (int)k, n_max, st);
           }
         }
         unsigned long long herr = 0;

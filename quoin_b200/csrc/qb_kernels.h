@@ -261,6 +261,14 @@ void launch_select_table(const uint8_t* bm, uint64_t n, const uint64_t* word_ran
 void launch_word_popcount(const uint8_t* bm, uint64_t n, uint64_t* cnt, cudaStream_t st);
 void launch_finalize(const uint64_t* lane, const uint8_t* bm, const uint64_t* word_rank, uint64_t n, int dtype,
                      void* out, cudaStream_t st);
+struct CombineCol {  // launch_decimal_combine's arguments of one column
+  const uint64_t *limbs, *vmin, *rank;
+  const uint8_t* bm;
+  uint8_t* out;
+  uint64_t stride, n;
+  int64_t nl;
+};
+void launch_cols_combine(const CombineCol* cols, int ncols, uint64_t n_max, cudaStream_t st);
 void launch_decimal_combine(const uint64_t* limbs, uint64_t limb_stride, int nlimbs, const uint64_t* vmin,
                             const uint8_t* bm, const uint64_t* word_rank, uint64_t n, uint8_t* out, cudaStream_t st);
 

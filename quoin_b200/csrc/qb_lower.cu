@@ -788,13 +788,13 @@ void launch_validity_blob(const uint8_t* bm, uint64_t n, uint64_t* tmp, uint64_t
   k_vb_sizes<<<g, 256, 0, st>>>(bm, n, last, sizes);
   scan_exclusive<ScanSum>(sizes, sizes, nw, tile_tmp, state + 1, st);
   k_vb_write<<<g, 256, 0, st>>>(bm, n, last, sizes, state, out, blob_len);
-  count_launches(9);
+  count_launches(3 + 2 * scan_launches(nw));
 }
 
 void launch_scan_sum(const uint64_t* in, uint64_t* out, uint64_t n, uint64_t* tile_tmp, uint64_t* grand,
                      cudaStream_t st) {
   scan_exclusive<ScanSum>(in, out, n ? n : 1, tile_tmp, grand, st);
-  count_launches(3);
+  count_launches(scan_launches(n));
 }
 
 void launch_write_bytes(uint8_t* dst, const uint8_t* src_dev, uint64_t len, cudaStream_t st) {

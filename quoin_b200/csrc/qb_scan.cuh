@@ -1,5 +1,6 @@
 // Device-wide exclusive scans over u64 (three passes: per-tile totals, a
-// single-CTA scan of the tile totals, per-tile scan with the tile offset).
+// single-CTA scan of the tile totals, per-tile scan with the tile offset; one
+// CTA for short ones).
 // Op is ScanSum (prefix sums: validity ranks, frame and varint offsets) or
 // ScanMax (last-seen position scans for the validity run lengths).
 #pragma once
@@ -99,6 +100,34 @@ __global__ void k_scan_apply(const uint64_t* in, size_t n, const uint64_t* __res
   }
 }
 
+// Up to kScanOne values in one CTA: the three launches above take 6.5 us and
+// three gaps for 3,000 values, this one 5.4 us; for 12,000 values it takes 13.
+constexpr size_t kScanOne = 4096;
+template <class Op>
+__global__ void __launch_bounds__(1024) k_scan_one(const uint64_t* in, uint32_t n, uint64_t* out,
+                                                   uint64_t* __restrict__ grand) {
+  __shared__ uint64_t s_warp[33];
+  uint64_t carry = Op::id();
+  for (uint32_t b = 0; b < n; b += 1024 * kScanItems) {
+    const uint32_t base = b + threadIdx.x * kScanItems;
+    uint64_t v[kScanItems], acc = Op::id(), tot;
+#pragma unroll
+    for (int k = 0; k < kScanItems; k++) {
+      v[k] = base + k < n ? in[base + k] : Op::id();
+      acc = Op::op(acc, v[k]);
+    }
+    uint64_t ex = Op::op(carry, block_excl_scan<Op>(acc, s_warp, &tot));
+#pragma unroll
+    for (int k = 0; k < kScanItems; k++) {
+      if (base + k < n) out[base + k] = ex;
+      ex = Op::op(ex, v[k]);
+    }
+    carry = Op::op(carry, tot);
+  }
+  if (threadIdx.x == 0 && grand) *grand = carry;
+}
+inline int scan_launches(size_t n) { return n <= kScanOne ? 1 : 3; }
+
 inline size_t scan_tiles(size_t n) {
   size_t t = (n + kScanTile - 1) / kScanTile;
   return t ? t : 1;
@@ -109,6 +138,10 @@ inline size_t scan_tiles(size_t n) {
 template <class Op = ScanSum>
 inline void scan_exclusive(const uint64_t* in, uint64_t* out, size_t n, uint64_t* tile_tmp, uint64_t* grand,
                            cudaStream_t st) {
+  if (n <= kScanOne) {
+    k_scan_one<Op><<<1, 1024, 0, st>>>(in, (uint32_t)n, out, grand);
+    return;
+  }
   size_t ntiles = scan_tiles(n);
   k_scan_tile_sums<Op><<<(unsigned)ntiles, kScanThreads, 0, st>>>(in, n, tile_tmp);
   k_scan_sums<Op><<<1, 1024, 0, st>>>(tile_tmp, ntiles, grand);
