@@ -2018,10 +2018,12 @@ static_assert(kItemBytes * kXorzRounds == kXorzItemBytes, "XORZ item size shared
 constexpr int kItemStage = kItemVals + kItemVals / 16;  // u64 staging with one pad per 16
 constexpr int kItemWarps = 8;
 // Resident CTAs per SM the item kernel is compiled for (its register cap):
-// 5 gives 48 registers a thread, and the kernel's 39 KB of shared memory
-// holds five CTAs on an SM.
+// 4 gives 64 registers a thread.  Five (48 registers, as many as the kernel's
+// 39 KB of shared memory allow) spill 2.4 KB over the modes: three columns of
+// 67,108,864 integers decode in 2,363 us with five and 2,286 with four, three
+// float columns of 10,000,019 in 760 and 748.
 #ifndef QB_ITEM_MIN_BLOCKS
-#define QB_ITEM_MIN_BLOCKS 5
+#define QB_ITEM_MIN_BLOCKS 4
 #endif
 
 struct PreRec {
