@@ -1,11 +1,11 @@
 // Block planner, per-block codec competition and winner emission
 // (reference src/encoder.rs:154-469,644-759 and the encode functions of the
-// in-path codecs).  One CTA per block.  The competition never materialises a
+// in-path codecs).  The competition is one CTA per block and never materialises a
 // candidate payload: every candidate's exact byte length is computed in closed
 // form from warp-reduced statistics (sub-block widths, exception counts,
 // distinct/run counts, ALP (e,f) search, ALP-RD cut search), the argmin of
 // `len + penalty` is taken in the reference's candidate order with a strict
-// `<`, and only the winner is written by k_emit.
+// `<`, and only the winner is written, by one or two CTAs per window (k_emit).
 #include <cooperative_groups.h>
 
 #include "qb_common.cuh"
